@@ -1927,15 +1927,23 @@ MOE_TILE_ROWS_OVERRIDE: Optional[int] = None  # measurements only: 0, 1 or 2 pic
 
 def moe_tile_rows(mma: bool, n_pairs: int = 1 << 30, n_experts: int = 1) -> int:
     """Rows of a tile of the routed products: the plain kernels' size, or one of the tensor-core kernels' three - 16
-    rows while an expert gets 12 rows or fewer on average (single tokens), 32 rows up to 32 on average, else 128.
-    (Measured at 16 experts: at 10.7 rows an expert 16-row tiles are 5 to 18 % faster than 32-row ones, at 16 rows
-    an expert - where about half of the experts need a second 16-row tile - 32-row tiles are up to 20 % faster.)"""
+    rows while an expert gets 12 rows or fewer on average (single tokens), 32 rows up to 28 on average, else the 256 of
+    the tcgen05 kernel.  (Measured at 16 experts: at 10.7 rows an expert 16-row tiles are 5 to 18 % faster than 32-row
+    ones, at 16 rows an expert - where about half of the experts need a second 16-row tile - 32-row tiles are up to 20 %
+    faster.  Tiles of 32 rows against the tcgen05 kernel, both
+    products, 16 experts of 2,048 x 2,048: 24 rows an expert 105 / 136 us, 32 rows 151 / 125, 40 rows 184 / 125; of
+    4,096 x 3,584: 12.5 rows 325 / 306, 25 rows 328 / 317.)"""
     if not mma:
         return int(lib().mll_moe_simt_rows())
     if MOE_TILE_ROWS_OVERRIDE is not None:
         return int(lib().mll_moe_mma_rows(ctypes.c_int(MOE_TILE_ROWS_OVERRIDE)))
-    small = 1 if n_pairs <= 12 * n_experts else (2 if n_pairs <= 32 * n_experts else 0)
+    small = 1 if n_pairs <= 12 * n_experts else (2 if n_pairs <= 28 * n_experts else 0)
     return int(lib().mll_moe_mma_rows(ctypes.c_int(small)))
+
+
+def moe_needs_rows(plan: MoePlan) -> bool:
+    """Whether `moe_gate_up` first copies its rows into the experts' order (the tcgen05 kernel's tiles)."""
+    return plan.mma and plan.rows == int(lib().mll_moe_mma_rows(ctypes.c_int(0)))
 
 
 def moe_max_tiles(n_pairs: int, n_experts: int, rows: int) -> int:
@@ -2006,10 +2014,12 @@ def _plan_args(plan: MoePlan):
 EXPERT_SWIGLU, EXPERT_GELU = 0, 1
 
 
-def moe_gate_up(h, w, act, plan: MoePlan, top: int, form: int = EXPERT_SWIGLU, n_experts: Optional[int] = None) -> None:
+def moe_gate_up(h, w, act, plan: MoePlan, top: int, form: int = EXPERT_SWIGLU, n_experts: Optional[int] = None,
+                rows: Optional[torch.Tensor] = None) -> None:
     """act[place] = silu(W_gate,e h[token]) * (W_up,e h[token]); w [E, 2 I, D] holds an expert's gate rows, then
     its up rows; act [pairs, I].  form EXPERT_GELU: act[place] = gelu(W_up,e h[token]) (erf form), w [E, I, D].
-    `n_experts`: the experts that the plan was sorted for, where more are routed to than have matrices."""
+    `n_experts`: the experts that the plan was sorted for, where more are routed to than have matrices.  `rows`: room for
+    the rows in the experts' order ([pairs, D], h's dtype) where `moe_needs_rows(plan)`; made here when not given."""
     _need(h, "moe gate_up h", None, 2)
     _need(w, "moe gate_up w", h.dtype, 3)
     _need(act, "moe gate_up act", h.dtype, 2)
@@ -2020,13 +2030,20 @@ def moe_gate_up(h, w, act, plan: MoePlan, top: int, form: int = EXPERT_SWIGLU, n
     if h.shape[1] != width or tuple(act.shape) != (n_pairs, inter) or (form == EXPERT_SWIGLU and two_inter != 2 * inter):
         raise KernelError(f"moe gate_up: h {tuple(h.shape)}, w {tuple(w.shape)}, act {tuple(act.shape)}")
     fn = lib().mll_moe_gate_up_mma if plan.mma else lib().mll_moe_gate_up
-    args = (_ptr(h), _ptr(w), _ptr(act), *_plan_args(plan))
     tiles = ctypes.c_int(moe_max_tiles(n_pairs, experts, plan.rows))
     if plan.mma:
-        _check(fn(*args, tiles, ctypes.c_int(plan.rows), ctypes.c_int(width), ctypes.c_int(inter), ctypes.c_int(top),
-                  ctypes.c_int(form), _stream()), "moe_gate_up_mma")
+        if moe_needs_rows(plan):
+            if rows is None:
+                rows = torch.empty((n_pairs, width), dtype=h.dtype, device=h.device)
+            _need(rows, "moe gate_up rows", h.dtype, 2)
+            if tuple(rows.shape) != (n_pairs, width):
+                raise KernelError(f"moe gate_up: rows {tuple(rows.shape)} for {n_pairs} pairs of {width}")
+        _check(fn(_ptr(h), _ptr(w), _ptr(act), _ptr(rows), ctypes.c_int(n_pairs), *_plan_args(plan), tiles,
+                  ctypes.c_int(plan.rows), ctypes.c_int(w.shape[0]), ctypes.c_int(width), ctypes.c_int(inter),
+                  ctypes.c_int(top), ctypes.c_int(form), _stream()), "moe_gate_up_mma",
+               kernels=2 if moe_needs_rows(plan) else 1)
     else:
-        _check(fn(*args, dtype_code(h.dtype), tiles, ctypes.c_int(width), ctypes.c_int(inter), ctypes.c_int(top),
+        _check(fn(_ptr(h), _ptr(w), _ptr(act), *_plan_args(plan), dtype_code(h.dtype), tiles, ctypes.c_int(width), ctypes.c_int(inter), ctypes.c_int(top),
                   ctypes.c_int(form), _stream()), "moe_gate_up")
 
 
@@ -2046,8 +2063,8 @@ def moe_down(act, w, y, pair_weight, plan: MoePlan, top: int, n_experts: Optiona
     args = (_ptr(act), _ptr(w), _ptr(y), _ptr(pair_weight), *_plan_args(plan))
     tiles = ctypes.c_int(moe_max_tiles(n_pairs, experts, plan.rows))
     if plan.mma:
-        _check(fn(*args, tiles, ctypes.c_int(plan.rows), ctypes.c_int(inter), ctypes.c_int(width), ctypes.c_int(top),
-                  _stream()), "moe_down_mma")
+        _check(fn(*args, tiles, ctypes.c_int(plan.rows), ctypes.c_int(n_pairs), ctypes.c_int(w.shape[0]),
+                  ctypes.c_int(inter), ctypes.c_int(width), ctypes.c_int(top), _stream()), "moe_down_mma")
     else:
         _check(fn(*args, dtype_code(act.dtype), tiles, ctypes.c_int(inter), ctypes.c_int(width), ctypes.c_int(top),
                   _stream()), "moe_down")

@@ -1,20 +1,15 @@
-// The two products of the routed feed-forward (moe.cu) on tensor cores, bfloat16: tiles of 128 rows of one expert
-// times 128 weight rows, mma.sync m16n8k16 with float32 accumulation, operands through a three-stage cp.async
-// ring (64 columns of k a stage, 108 KB of shared memory: two blocks a multiprocessor keep about 70 KB of weights
-// in flight, which a decode step - every touched expert's weights streamed once - needs to fill the memory pipe).
-// Eight warps as 4 x 2: a warp owns 32 of the tile's rows and 64 of its weight rows.  (Four warps on 64 rows, two blocks
-// a multiprocessor, kept the tensor pipe 43 % busy with an eighth of the warp slots filled.)
-// Steps with few rows per expert (single tokens) take a second instance: tiles of 16 rows - one MMA row tile - and
-// four warps side by side on 64 weight rows, four stages, four such blocks a multiprocessor (256 weight rows, one
-// block a multiprocessor: the same time; two warps on 128 weight rows: a quarter slower).  Such a step streams every touched expert's weights once
-// for a handful of rows, and on the wide tile it was bound by the MMAs spent on empty rows (128-row tiles at batch 64:
-// 2 TB/s from a cold cache).  Between 12 and 32 rows per expert on average a third instance has tiles of 32 rows (two MMA
-// row tiles a warp, otherwise the small one): with 16-row tiles the experts that got 17 rows or more take a second
-// tile each, and a few of those push the grid past the blocks that are resident at once - a second, nearly empty wave.
-//   gate_up  the 128 weight rows are 64 gate rows and the 64 up rows of the same activation columns; a warp's
-//            eight 8-column tiles are four of gate and the same four of up, so silu(gate) * up happens in the
+// The two products of the routed feed-forward (moe.cu) for steps with few rows per expert (single tokens), bfloat16:
+// mma.sync m16n8k16 with float32 accumulation on tiles of 16 rows of one expert - one MMA row tile - times 64 weight rows,
+// four warps side by side, operands through a four-stage cp.async ring (64 columns of k a stage), four such blocks a
+// multiprocessor (256 weight rows, one block a multiprocessor: the same time; two warps on 128 weight rows: a quarter
+// slower).  Such a step streams every touched expert's weights once for a handful of rows: memory bounds it.
+// Between 12 and 32 rows per expert on average a second instance has tiles of 32 rows (two MMA row tiles a warp): with
+// 16-row tiles the experts that got 17 rows or more take a second tile each, and a few of those push the grid past the
+// blocks that are resident at once - a second, nearly empty wave.  Steps with more rows run in moe_tc5.cu.
+//   gate_up  the 64 weight rows are 32 gate rows and the 32 up rows of the same activation columns; a warp's
+//            8-column tiles are half of gate and the same half of up, so silu(gate) * up happens in the
 //            accumulator registers; rows are gathered from the step's tokens by (token, choice) pair.
-//   down     the 128 weight rows are output columns; a row's result is multiplied by its pair's routing weight
+//   down     the 64 weight rows are output columns; a row's result is multiplied by its pair's routing weight
 //            and written as float32 to the pair's row (summed over a token's choices by the combine kernel).
 // Rows past a tile's end and columns past the matrices' edges are zero-filled in shared memory.
 #include "attention_decode.cuh"
@@ -30,7 +25,6 @@ struct MoeMmaShape {
   static constexpr int BM = 16 * MT * WM, BN = 8 * NT * WN, LD = BK + 8, THREADS = 32 * WM * WN;
   static constexpr size_t SMEM = (size_t)STAGES * (BM + BN) * LD * sizeof(__nv_bfloat16);
 };
-using MoeMmaWide = MoeMmaShape<2, 8, 4, 2, 64, 3>;   // 128 rows x 128 weight rows: prompts
 using MoeMmaSmall = MoeMmaShape<1, 2, 1, 4, 64, 4>;  // 16 rows x 64 weight rows: single tokens
 using MoeMmaMedium = MoeMmaShape<2, 2, 1, 4, 64, 4>;  // 32 rows x 64 weight rows: single tokens, 12 to 32 rows an expert
 
@@ -188,41 +182,54 @@ int launch_moe_mma(const MoeProductArgs& a, int max_tiles, cudaStream_t stream) 
 
 template <int KIND>
 int launch_moe_mma_rows(const MoeProductArgs& a, int max_tiles, int tile_rows, cudaStream_t stream) {
-  if (tile_rows == MoeMmaWide::BM) return launch_moe_mma<KIND, 2, 8, 4, 2, 64, 3>(a, max_tiles, stream);
   if (tile_rows == MoeMmaSmall::BM) return launch_moe_mma<KIND, 1, 2, 1, 4, 64, 4>(a, max_tiles, stream);
   if (tile_rows == MoeMmaMedium::BM) return launch_moe_mma<KIND, 2, 2, 1, 4, 64, 4>(a, max_tiles, stream);
-  mll_set_error("moe (mma): tiles of %d rows (known: %d, %d, %d)", tile_rows, MoeMmaSmall::BM, MoeMmaMedium::BM, MoeMmaWide::BM);
+  mll_set_error("moe (mma): tiles of %d rows (known: %d, %d, %d)", tile_rows, MoeMmaSmall::BM, MoeMmaMedium::BM, mll_moe_tc5_rows());
   return -1;
 }
 
 }  // namespace mll
 
-// Rows of a tile: the wide instance (small = 0) or one of the two for steps with few rows per expert (1: 16 rows, 2: 32).
+// Rows of a tile: those of moe_tc5.cu (small = 0) or one of the two here for steps with few rows per expert (1: 16 rows, 2: 32).
 MLL_API int mll_moe_mma_rows(int small) {
-  return small == 1 ? mll::MoeMmaSmall::BM : (small == 2 ? mll::MoeMmaMedium::BM : mll::MoeMmaWide::BM);
+  if (small == 0) return mll_moe_tc5_rows();
+  return small == 1 ? mll::MoeMmaSmall::BM : mll::MoeMmaMedium::BM;
 }
 
 // bfloat16 only; rows of 16-byte words on both sides of both products.
 MLL_API int mll_moe_mma_supported(int width, int inter) { return width > 0 && inter > 0 && width % 8 == 0 && inter % 8 == 0; }
 
-MLL_API int mll_moe_gate_up_mma(const void* h, const void* w, void* act, const int* order, const int* offsets,
+// rows: room for the rows in the experts' order, bfloat16 [n_pairs, width] (tiles of mll_moe_tc5_rows() rows only).
+MLL_API int mll_moe_gate_up_mma(const void* h, const void* w, void* act, void* rows, int n_pairs, const int* order, const int* offsets,
                                 const int* tile_expert, const int* tile_row0, const int* n_tiles, int max_tiles,
-                                int tile_rows, int width, int inter, int top, int form, cudaStream_t stream) {
+                                int tile_rows, int n_experts, int width, int inter, int top, int form,
+                                cudaStream_t stream) {
   MLL_REQUIRE(form == 0 || form == 1, "moe gate_up (mma): unknown expert form %d", form);
   MLL_REQUIRE(mll_moe_mma_supported(width, inter) && max_tiles > 0 && top > 0, "moe gate_up (mma): sizes %d / %d", width, inter);
   MLL_REQUIRE((inter + 31) / 32 <= 65535, "moe gate_up (mma): %d columns are too many for one launch", inter);
   mll::MoeProductArgs a{h, w, act, nullptr, mll::MoePlan{(int*)order, (int*)offsets, (int*)tile_expert, (int*)tile_row0,
                                                          (int*)n_tiles}, width, inter, top};
+  if (tile_rows == mll_moe_tc5_rows()) {
+    MLL_REQUIRE(rows != nullptr && n_pairs > 0 && n_experts > 0, "moe gate_up (tc5): no room for %d rows", n_pairs);
+    MLL_REQUIRE(((uintptr_t)h | (uintptr_t)rows | (uintptr_t)w | (uintptr_t)act) % 16 == 0,
+                "moe gate_up (tc5): operands must be 16-byte aligned");
+    return mll_moe_gate_up_tc5(h, rows, w, act, a.plan, max_tiles, n_pairs, n_experts, width, inter, top, form, stream);
+  }
   if (form == 1) return mll::launch_moe_mma_rows<2>(a, max_tiles, tile_rows, stream);
   return mll::launch_moe_mma_rows<1>(a, max_tiles, tile_rows, stream);
 }
 
 MLL_API int mll_moe_down_mma(const void* act, const void* w, float* y, const float* pair_weight, const int* order,
                              const int* offsets, const int* tile_expert, const int* tile_row0, const int* n_tiles,
-                             int max_tiles, int tile_rows, int inter, int width, int top, cudaStream_t stream) {
+                             int max_tiles, int tile_rows, int n_pairs, int n_experts, int inter, int width, int top,
+                             cudaStream_t stream) {
   MLL_REQUIRE(mll_moe_mma_supported(width, inter) && max_tiles > 0 && top > 0, "moe down (mma): sizes %d / %d", width, inter);
   MLL_REQUIRE((width + 63) / 64 <= 65535, "moe down (mma): %d columns are too many for one launch", width);
   mll::MoeProductArgs a{act, w, y, pair_weight, mll::MoePlan{(int*)order, (int*)offsets, (int*)tile_expert,
                                                              (int*)tile_row0, (int*)n_tiles}, inter, width, top};
+  if (tile_rows == mll_moe_tc5_rows()) {
+    MLL_REQUIRE(((uintptr_t)act | (uintptr_t)w | (uintptr_t)y) % 16 == 0, "moe down (tc5): operands must be 16-byte aligned");
+    return mll_moe_down_tc5(act, w, y, pair_weight, a.plan, max_tiles, n_pairs, n_experts, inter, width, top, stream);
+  }
   return mll::launch_moe_mma_rows<0>(a, max_tiles, tile_rows, stream);
 }

@@ -171,8 +171,9 @@ class RoutedFeedForward(FeedForward):
         plan = self._plan(step, n_pairs, mma)
         K.moe_sort(chosen, plan, self.routed, n_real=self.experts)
         hidden = ws.buffer("moe.act", (n_pairs, self.inter), act)
+        rows = ws.buffer("moe.rows", (n_pairs, D), act) if K.moe_needs_rows(plan) else None
         K.moe_gate_up(h, self.gate_up, hidden, plan, self.top, form=K.EXPERT_GELU if self.gelu else K.EXPERT_SWIGLU,
-                      n_experts=self.routed)
+                      n_experts=self.routed, rows=rows)
         y = ws.buffer("moe.y", (n_pairs, D), torch.float32)
         K.moe_down(hidden, self.down, y, weight, plan, self.top, n_experts=self.routed)
         shared = self.shared.forward(step, h) if self.shared is not None else None
