@@ -14,7 +14,7 @@ import torch
 from ..cache.paged import PAGE  # cache positions per page; the library's MLL_PAGE is checked against it on load
 from .build import KernelBuildError, load_library
 
-ABI_VERSION = 35
+ABI_VERSION = 36
 MAX_TOP_K = 1024
 STATE_RUN = 32  # tokens a run of `state_chunks`
 
@@ -323,6 +323,31 @@ def linear_small(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor],
                                         ctypes.c_int(k), ctypes.c_int(epilogue), ctypes.c_int(ranks),
                                         *_row_norm_args(row_norm, rows, "linear_small"), _ptr(resid), _ptr(next_w),
                                         _ptr(out_sumsq), ctypes.c_int(out_stride), _stream()), "linear_small")
+
+
+def linear_f32_supported(x: torch.Tensor, w: torch.Tensor, epilogue: int = EPI_F32) -> bool:
+    """Whether `linear_f32` takes x . w^T: float32, the few rows of a decode step, rows on 16-byte boundaries."""
+    return (SMALL_LINEAR != "none" and x.dtype == torch.float32 and w.dtype == torch.float32 and x.dim() == 2
+            and x.is_contiguous() and w.is_contiguous() and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
+            and bool(lib().mll_linear_f32_supported(x.shape[0], w.shape[0], w.shape[1], epilogue)))
+
+
+def linear_f32(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor, epilogue: int = EPI_F32,
+               slices: int = 0) -> None:
+    """out = x . w^T (+ bias) in true float32 for at most 16 rows of x [M, K], w [N, K] read once; EPI_SWIGLU and EPI_GEGLU
+    as in `linear_small`, with out float32 [M, N / 2] and no bias.  `slices`: warps that share weight rows, each with a
+    part of K (1, 2, 4 or 8; 0: chosen)."""
+    for t, name in ((x, "x"), (w, "w"), (out, "out")):
+        _need(t, "linear_f32 " + name, torch.float32, 2)
+    (rows, k), n = x.shape, w.shape[0]
+    if w.shape[1] != k or tuple(out.shape) != (rows, n if epilogue == EPI_F32 else n // 2):
+        raise KernelError(f"linear_f32: x {tuple(x.shape)}, w {tuple(w.shape)} and out {tuple(out.shape)} do not fit")
+    if bias is not None:
+        _need(bias, "linear_f32 bias", torch.float32, 1)
+        if bias.shape[0] != n:
+            raise KernelError("linear_f32: bias length differs from the output width")
+    _check(lib().mll_linear_f32(_ptr(x), _ptr(w), _ptr(bias), _ptr(out), ctypes.c_int(rows), ctypes.c_int(n), ctypes.c_int(k),
+                                ctypes.c_int(epilogue), ctypes.c_int(slices), _stream()), "linear_f32")
 
 
 def linear_tma_supported(rows: int, out_features: int, in_features: int, epilogue: int = EPI_BF16) -> bool:

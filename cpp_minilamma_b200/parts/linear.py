@@ -3,8 +3,9 @@
 W is row-major [out, in] as in the reference (src/cuda_matmul.cc:181-186, one
 `cublasSgemm` per call there).  The product runs in the dtype of the weight:
   * bfloat16 weight, bfloat16 x: tensor-core product with float32 accumulation;
-  * float32 weight: a true float32 product (TF32 must be off; it is refused otherwise);
-    bfloat16 activations are widened first and the result narrowed afterwards.
+  * float32 weight: a true float32 product (TF32 must be off; it is refused otherwise), for the few rows of a decode
+    step on a weight-streaming kernel of this package; bfloat16 activations are widened first and the result narrowed
+    afterwards.
 A bias (float32 [N], not in the reference) is added in float32 by the weight-streaming kernels' epilogues, or by a
 kernel behind the library product.
 Large products go to the library GEMM (as the reference's do); small batches of rows go
@@ -74,11 +75,9 @@ class Linear:
                 x = wide
             if out_dtype == torch.float32:
                 out = given if given is not None else ws.buffer(out_name, (rows, self.out_features), torch.float32)
-                torch.mm(x, w.t(), out=out)
-                return self._biased(out)
+                return self._product_f32(step, x, out)
             wide_out = ws.buffer(out_name + ".y32", (rows, self.out_features), torch.float32)
-            torch.mm(x, w.t(), out=wide_out)
-            self._biased(wide_out)
+            self._product_f32(step, x, wide_out)
             out = given if given is not None else ws.buffer(out_name, (rows, self.out_features), out_dtype)
             K.cast(wide_out, out)
             return out
@@ -103,6 +102,13 @@ class Linear:
             torch.mm(x, w.t(), out=out)
         else:  # bfloat16 operands, float32 result (the logits)
             _mm_bf16_to_f32(x, w, out)
+        return self._biased(out)
+
+    def _product_f32(self, step, x: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
+        if x.shape[0] <= step.small_rows and out.is_contiguous() and K.linear_f32_supported(x, self.weight):
+            K.linear_f32(x, self.weight, self.bias, out)
+            return out
+        torch.mm(x, self.weight.t(), out=out)
         return self._biased(out)
 
     def _biased(self, out: torch.Tensor) -> torch.Tensor:
