@@ -299,11 +299,14 @@ class SequenceCache:
             if wanted > g.pool.n_free:
                 raise CacheFull(f"{wanted} pages wanted, {g.pool.n_free} of {g.pool.n_pages} free; "
                                 f"the cache was sized for {self.n_pages * PAGE} tokens")
+        for g in self.groups:
+            for slot, extra in growth:
+                old = self.seq_len[slot]
+                # most decode steps stay inside a sequence's last page: nothing to do without a window that moves on
+                if g.need.window > 0 or (old + extra + PAGE - 1) // PAGE > len(g.pages[slot]):
+                    g.grow(slot, old, old + extra)
         for slot, extra in growth:
-            old = self.seq_len[slot]
-            for g in self.groups:
-                g.grow(slot, old, old + extra)
-            self.seq_len[slot] = old + extra
+            self.seq_len[slot] += extra
 
     def flush(self) -> None:
         """Upload the block-table rows that changed since the last call (blocking copies; the engine's

@@ -116,7 +116,8 @@ def _stream() -> ctypes.c_void_p:
     # every wrapper evaluates this once, among the arguments of its launch: the place where a timer's first event goes
     if _timer is not None:
         _timer.begin()
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    # The raw handle: building a torch.cuda.Stream object for it took longer than the rest of a launch's host side.
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 def _ptr(t: Optional[torch.Tensor]) -> ctypes.c_void_p:
@@ -124,6 +125,9 @@ def _ptr(t: Optional[torch.Tensor]) -> ctypes.c_void_p:
 
 
 def _need(t: torch.Tensor, name: str, dtype=None, ndim=None) -> None:
+    if (isinstance(t, torch.Tensor) and t.is_cuda and (dtype is None or t.dtype == dtype) and (ndim is None or t.dim() == ndim)
+            and t.is_contiguous()):
+        return
     if not isinstance(t, torch.Tensor) or not t.is_cuda:
         raise KernelError(f"{name}: expected a CUDA tensor (the kernels have no CPU path)")
     if not t.is_contiguous():

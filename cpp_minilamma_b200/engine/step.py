@@ -20,6 +20,7 @@ which assemble their logits in a tensor of their own.
 """
 from __future__ import annotations
 
+from array import array
 from dataclasses import dataclass, field
 from typing import Any, Dict, Hashable, List, Optional, Sequence, Tuple
 
@@ -51,10 +52,16 @@ class Workspace:
     def __init__(self, device):
         self.device = device
         self._flat: Dict[str, torch.Tensor] = {}
+        self._views: Dict[str, Dict[Tuple, torch.Tensor]] = {}  # views handed out, by name, then shape and dtype
         self._zeroed: set = set()
         self.generation = 0
 
     def buffer(self, name: str, shape: Tuple[int, ...], dtype: torch.dtype) -> torch.Tensor:
+        views = self._views.get(name)
+        if views is not None:
+            view = views.get((shape, dtype))
+            if view is not None:
+                return view
         count = 1
         for dim in shape:
             count *= dim
@@ -63,7 +70,11 @@ class Workspace:
             flat = torch.empty(max(count, 1), dtype=dtype, device=self.device)
             self._flat[name] = flat
             self.generation += 1
-        return flat[:count].view(shape)
+            views = None
+        if views is None or len(views) >= 64:  # views of a buffer that is gone go with it; those of many shapes do not pile up
+            views = self._views[name] = {}
+        view = views[(shape, dtype)] = flat[:count].view(shape)
+        return view
 
     def zeros(self, name: str, shape: Tuple[int, ...], dtype: torch.dtype) -> torch.Tensor:
         """As `buffer`, but zero-filled when it is (re)allocated - for counters that the
@@ -74,6 +85,7 @@ class Workspace:
         flat = self._flat.get(name)
         if flat is None or flat.dtype != dtype or flat.numel() < count:
             self._flat[name] = torch.zeros(max(count, 64), dtype=dtype, device=self.device)
+            self._views.pop(name, None)
             self._zeroed.add(name)
             self.generation += 1
         return self._flat[name][:count].view(shape)
@@ -179,6 +191,19 @@ def make_step_state(device, slots: Sequence[int], starts: Sequence[int], lens: S
     return state_from_views(ws or Workspace(device), shape, views, small_rows)
 
 
+def _whole_numbers(tokens: Sequence[int]) -> Optional[np.ndarray]:
+    """`tokens` as an integer array where that can be had in one go (a list of whole numbers, a 1-D integer array), so that
+    a long prompt is walked through once and not for its smallest, its largest and its copy each; else None."""
+    if type(tokens) is np.ndarray:
+        return tokens if tokens.ndim == 1 and tokens.dtype in (np.int32, np.int64) else None
+    if type(tokens) is not list:
+        return None
+    try:
+        return np.frombuffer(array("q", tokens), dtype=np.int64)
+    except (TypeError, OverflowError):
+        return None
+
+
 @dataclass
 class _ChunkSeq:
     slot: int
@@ -244,8 +269,9 @@ class Engine:
         the entries and of each entry's `want`, or None when nothing is wanted.  The
         result is the caller's own tensor."""
         borrowed = self.step_borrowed(entries)
+        own = None if borrowed is None else borrowed.clone()  # enqueued before the wait below
         self.check_device_error()
-        return None if borrowed is None else borrowed.clone()
+        return own
 
     def check_device_error(self) -> None:
         """Waits for the device and raises `DeviceKernelError` if a kernel gave up since the flags were
@@ -285,8 +311,13 @@ class Engine:
             else:
                 if out is None:
                     out = torch.empty((n_want, self.vocab_size), dtype=torch.float32, device=self.device)
-                index = torch.tensor(out_rows, dtype=torch.long, device=self.device)
-                out.index_copy_(0, index, logits)
+                first = out_rows[0]
+                if out_rows == list(range(first, first + len(out_rows))):
+                    out[first:first + len(out_rows)].copy_(logits)
+                else:
+                    # from pinned memory: a copy that the host waits for would keep it from preparing the next chunk
+                    index = torch.tensor(out_rows, dtype=torch.long, pin_memory=self.device.type == "cuda")
+                    out.index_copy_(0, index.to(self.device, non_blocking=True), logits)
                 result = out
         return result
 
@@ -295,12 +326,15 @@ class Engine:
         if not entries:
             raise StepError("a step needs at least one entry")
         growth = []
+        tokens: List[Sequence[int]] = []
         vocab = self.vocab_size
         for e in entries:
             n = len(e.tokens)
             if n < 1:
                 raise StepError(f"slot {e.slot}: a step must bring at least one token")
-            lo, hi = min(e.tokens), max(e.tokens)
+            values = _whole_numbers(e.tokens)
+            lo, hi = (min(e.tokens), max(e.tokens)) if values is None else (int(values.min()), int(values.max()))
+            tokens.append(e.tokens if values is None else values)
             if lo < 0 or hi >= vocab:
                 raise StepError(f"slot {e.slot}: token {lo if lo < 0 else hi} outside the vocabulary [0, {vocab})")
             for w in e.want:
@@ -321,21 +355,21 @@ class Engine:
         chunks: List[List[_ChunkSeq]] = [[]]
         room = self.max_step_tokens
         out_row = 0
-        for e in entries:
-            n = len(e.tokens)
-            wants_by_place: Dict[int, List[int]] = {}
+        for e, values in zip(entries, tokens):
+            n = len(values)
+            wants: List[Tuple[int, int]] = []
             for w in e.want:
-                wants_by_place.setdefault(w, []).append(out_row)
+                wants.append((w, out_row))
                 out_row += 1
+            wants.sort()
             done = 0
             while done < n:
                 if room == 0:
                     chunks.append([])
                     room = self.max_step_tokens
                 take = min(room, n - done)
-                want = [(place - done, row) for place in range(done, done + take)
-                        for row in wants_by_place.get(place, [])] if wants_by_place else []
-                chunks[-1].append(_ChunkSeq(e.slot, e.tokens[done:done + take], starts[e.slot] + done, want))
+                want = [(place - done, row) for place, row in wants if done <= place < done + take]
+                chunks[-1].append(_ChunkSeq(e.slot, values[done:done + take], starts[e.slot] + done, want))
                 done += take
                 room -= take
         return chunks, out_row

@@ -84,7 +84,7 @@ class DeviceSampler:
         """The token ids of a ticket (waits for that step, not for later ones)."""
         turn, n, rows = ticket
         self.events[turn].synchronize()
-        host = self.hosts[turn]
+        host = self.hosts[turn].numpy()
         status = host[rows:rows + n]
         # row 0's word also carries, in bits 8 and up, the error flags of kernels that gave up during the step
         gave_up = int(status[0]) >> 8
