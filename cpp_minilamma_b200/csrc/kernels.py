@@ -14,7 +14,7 @@ import torch
 from ..cache.paged import PAGE  # cache positions per page; the library's MLL_PAGE is checked against it on load
 from .build import KernelBuildError, load_library
 
-ABI_VERSION = 36
+ABI_VERSION = 37
 MAX_TOP_K = 1024
 STATE_RUN = 32  # tokens a run of `state_chunks`
 
@@ -1516,7 +1516,7 @@ def state_scan(q, k, v, g, beta, head_decay, state, out, seq_slot, seq_qstart, s
             raise KernelError("state scan: one decay per head is needed")
     _check(lib().mll_state_scan(
         _ptr(q), _ptr(k), _ptr(v), _ptr(g), _ptr(beta), _ptr(head_decay), _ptr(state), _ptr(out), _ptr(seq_slot),
-        _ptr(seq_qstart), _ptr(seq_qlen), ctypes.c_int(n_seqs), ctypes.c_int(n_heads), ctypes.c_int(n_kv_heads),
+        _ptr(seq_qstart), _ptr(seq_qlen), ctypes.c_int(n_seqs), ctypes.c_int(n), ctypes.c_int(n_heads), ctypes.c_int(n_kv_heads),
         ctypes.c_int(d), ctypes.c_int(dv), ctypes.c_int(4 if scalar_delta else (1 if delta else (2 if channel else (3 if per_token else 0)))),
         _stream()),
         "state_scan (delta rule, head decay)" if scalar_delta else "state_scan (delta rule)" if delta else ("state_scan (channel decay)" if channel else
