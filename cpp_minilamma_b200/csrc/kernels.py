@@ -14,7 +14,7 @@ import torch
 from ..cache.paged import PAGE  # cache positions per page; the library's MLL_PAGE is checked against it on load
 from .build import KernelBuildError, load_library
 
-ABI_VERSION = 37
+ABI_VERSION = 38
 MAX_TOP_K = 1024
 STATE_RUN = 32  # tokens a run of `state_chunks`
 
@@ -1530,28 +1530,32 @@ def state_chunks_supported(d: int, dv: int) -> bool:
     return USE_STATE_CHUNKS and bool(lib().mll_state_chunks_supported(d, dv))
 
 
-def state_chunks_scratch(n_runs: int, n_heads: int, d: int, dv: int, delta: bool) -> int:
-    """Floats of scratch memory that `state_chunks` wants."""
+def state_chunks_scratch(n_runs: int, n_heads: int, d: int, dv: int, delta: bool, channel: bool = False) -> int:
+    """Floats of scratch memory that `state_chunks` wants (`channel`: the delta rule with a decay per key channel)."""
     lib().mll_state_chunks_scratch.restype = ctypes.c_longlong
-    return int(lib().mll_state_chunks_scratch(n_runs, n_heads, d, dv, int(delta)))
+    return int(lib().mll_state_chunks_scratch(n_runs, n_heads, d, dv, 2 if channel else int(delta)))
 
 
 def state_chunks(q, k, v, state, out, scratch, run_seq, run_row0, seq_run0, seq_slot, seq_qstart, seq_qlen, n_seqs: int,
                  n_heads: int, n_kv_heads: int, d: int, dv: int, head_decay: Optional[torch.Tensor] = None,
-                 token_decay: Optional[torch.Tensor] = None, beta: Optional[torch.Tensor] = None) -> None:
+                 token_decay: Optional[torch.Tensor] = None, beta: Optional[torch.Tensor] = None,
+                 channel_decay: Optional[torch.Tensor] = None) -> None:
     """As `state_scan` for one decay per head (`head_decay` [H]) or per token and head (`token_decay` [T, H]; with `beta` the
-    delta rule), a run of up to STATE_RUN tokens at a time: run_seq, run_row0 (int32 [runs]) list every
+    delta rule), or the delta rule with a decay per key channel (`channel_decay` [T, H * d] and `beta`), a run of up to STATE_RUN tokens at a time: run_seq, run_row0 (int32 [runs]) list every
     sequence's runs one after another, seq_run0 (int32 [sequences]) its first.  Decays lie in [0, 1]."""
     n = q.shape[0]
     for name, t, width in (("q", q, n_kv_heads * d), ("k", k, n_kv_heads * d), ("v", v, n_heads * dv),
-                           ("out", out, n_heads * dv), ("token decay", token_decay, n_heads), ("beta", beta, n_heads)):
+                           ("out", out, n_heads * dv), ("token decay", token_decay, n_heads), ("beta", beta, n_heads),
+                           ("channel decay", channel_decay, n_heads * d)):
         if t is None:
             continue
         _need(t, f"state chunks {name}", torch.float32, 2)
         if tuple(t.shape) != (n, width):
             raise KernelError(f"state chunks: {name} {tuple(t.shape)}, expected {(n, width)}")
-    if (head_decay is None) == (token_decay is None) or (beta is not None and token_decay is None):
-        raise KernelError("state chunks: one decay per head or one per token and head; the delta rule goes with the latter")
+    if (sum(t is not None for t in (head_decay, token_decay, channel_decay)) != 1
+            or (head_decay if beta is not None else channel_decay) is not None):
+        raise KernelError("state chunks: one decay per head or one per token and head, the delta rule with the latter or with one "
+                          "per token, head and key channel")
     if head_decay is not None:
         _need(head_decay, "state chunks decay", torch.float32, 1)
         if head_decay.shape[0] != n_heads:
@@ -1565,13 +1569,13 @@ def state_chunks(q, k, v, state, out, scratch, run_seq, run_row0, seq_run0, seq_
     if run_row0.shape[0] != n_runs or seq_run0.shape[0] < n_seqs:
         raise KernelError("state chunks: the lists of runs differ in length")
     _need(scratch, "state chunks scratch", torch.float32)
-    if scratch.numel() < state_chunks_scratch(n_runs, n_heads, d, dv, beta is not None):
+    if scratch.numel() < state_chunks_scratch(n_runs, n_heads, d, dv, beta is not None, channel_decay is not None):
         raise KernelError("state chunks: scratch too small")
     _check(lib().mll_state_chunks(
-        _ptr(q), _ptr(k), _ptr(v), _ptr(beta), _ptr(token_decay), _ptr(head_decay), _ptr(state), _ptr(out), _ptr(scratch),
-        _ptr(run_seq), _ptr(run_row0), _ptr(seq_run0), _ptr(seq_slot), _ptr(seq_qstart), _ptr(seq_qlen), ctypes.c_int(n_runs),
+        _ptr(q), _ptr(k), _ptr(v), _ptr(beta), _ptr(token_decay), _ptr(head_decay), _ptr(channel_decay), _ptr(state), _ptr(out),
+        _ptr(scratch), _ptr(run_seq), _ptr(run_row0), _ptr(seq_run0), _ptr(seq_slot), _ptr(seq_qstart), _ptr(seq_qlen), ctypes.c_int(n_runs),
         ctypes.c_int(n_seqs), ctypes.c_int(n_heads), ctypes.c_int(n_kv_heads), ctypes.c_int(d), ctypes.c_int(dv), _stream()),
-        "state_chunks (delta rule)" if beta is not None else
+        "state_chunks (delta rule, channel decay)" if channel_decay is not None else "state_chunks (delta rule)" if beta is not None else
         ("state_chunks (token decay)" if token_decay is not None else "state_chunks (head decay)"), kernels=2 if beta is not None else 4)
 
 

@@ -1,5 +1,5 @@
-// The recurrences of recurrent.cu whose decay is one number per head (fixed, or per token), over prompts, a run of 32
-// tokens at a time instead of token by token:
+// The recurrences of recurrent.cu whose decay is one number per head (fixed, or per token), and the delta rule with a decay per
+// key channel, over prompts, a run of 32 tokens at a time instead of token by token:
 //
 //   S_t = g_t S_(t-1) + k_t u_t^T,   o_t = S_t^T q_t,   u_t = v_t   or   u_t = beta_t (v_t - g_t S_(t-1)^T k_t)  (delta rule)
 //
@@ -11,14 +11,22 @@
 //   and for the delta rule  u = U - W S  with  (I + A) U = diag(beta) V,  (I + A) W = diag(beta e^c) K,
 //                           A_ij = beta_i e^(c_i - c_j) k_i . k_j  for j < i
 //
+// With a decay per key channel the factors e^(c_i - c_j) stand inside the products, a vector over the channels each.  They
+// are formed as products of the decays themselves, never as a quotient (a decay may be 0): D_ij = g_(j+1) .. g_i, and for
+// tokens of different blocks of 8 in two parts that meet at the first token a of i's block, (g_(a+1) .. g_i)(g_(j+1) .. g_a),
+// neither larger than 1, so that a block's rows meet all earlier columns in plain products.
+//
 // Kernels:
 //   * state_chunk_inputs   a block per (run, head): the sums c (double), P, and for the delta rule U and W by forward
 //                          substitution, a column a thread
 //   * without the delta rule nothing but the sum of the states hangs from run to run: state_chunk_sums (what every run adds),
 //                          state_chunk_prefix (the state in front of every run) and state_chunk_outputs
+//   * state_chunk_channel_inputs  the same for the delta rule with a decay per key channel, which also writes Q and K with the
+//                          decays between them and the run's ends
 //   * state_chunk_scan     the delta rule: a block per (16 columns of the state, head, sequence) walks the runs; the columns
 //                          of S in registers and in shared memory, the runs' matrices through cp.async, W and Q of the
 //                          next run on their way while this one is worked on
+// 2,047 tokens of 16 heads of 128 x 128 with a decay per key channel: 718 us token by token, 238 here (inputs 63, scan 175).
 // All products are float32 FMAs: the recurrence stays exact to float32, which bfloat16 tensor-core products would not be,
 // and products cut into enough bfloat16 terms to be exact take as long on the tensor cores.
 #include "common.cuh"
@@ -37,12 +45,15 @@ struct ChunkArgs {
   const float* beta;        // [T, H] (delta rule) or null
   const float* token_decay; // [T, H], or null:
   const float* head_decay;  // [H]
+  const float* channel_decay;  // [T, H, d], or null
   float* state;             // [slots, H, d, dv]
   float* out;               // [T, H, dv]
   float* p;                 // [runs, H, 32, 32]
   float* w;                 // [runs, H, 32, d]    (delta rule)
   float* u;                 // [runs, H, 32, dv]   (delta rule)
-  float* factors;           // [runs, H, CH_FACTORS]
+  float* factors;           // [runs, H, CH_FACTORS]; with a decay per channel [runs, H, d]: the product of a run's decays
+  float* qd;                // [runs, H, 32, d]    (a decay per channel) q_i g_1 .. g_i
+  float* kd;                // [runs, H, 32, d]    likewise              k_j g_(j+1) .. g_n
   float* sums;              // [runs, H, d, dv]    (not the delta rule)
   const int* run_seq;       // [runs]
   const int* run_row0;      // [runs] first row among the sequence's new tokens
@@ -58,6 +69,23 @@ __device__ __forceinline__ void ch_copy16(float* dst, const float* src, bool val
   const unsigned s = (unsigned)__cvta_generic_to_shared(dst);
   const int bytes = valid ? 16 : 0;
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(src), "r"(bytes));
+}
+
+// x <- (I + A)^-1 x, A strictly lower triangular with rows of CH + 4 floats in shared memory
+__device__ __forceinline__ void ch_substitute(float (&x)[CH], const float* a_s) {
+#pragma unroll
+  for (int i = 1; i < CH; ++i) {
+    float s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int m = 0; m < i; m += 4) {  // the row's entries from i on are zero, as are x's uses of them
+      const float4 row = *reinterpret_cast<const float4*>(a_s + i * (CH + 4) + m);
+      s[0] = fmaf(row.x, x[m], s[0]);
+      if (m + 1 < i) s[1] = fmaf(row.y, x[m + 1], s[1]);
+      if (m + 2 < i) s[2] = fmaf(row.z, x[m + 2], s[2]);
+      if (m + 3 < i) s[3] = fmaf(row.w, x[m + 3], s[3]);
+    }
+    x[i] -= (s[0] + s[1]) + (s[2] + s[3]);
+  }
 }
 
 // grid (runs, H), 128 threads.  Rows of q and k lie in shared memory as 16-byte words whose index is XORed with the row's
@@ -170,24 +198,185 @@ __global__ void __launch_bounds__(128, 3) state_chunk_inputs_kernel(ChunkArgs a)
 #pragma unroll
         for (int i = 0; i < CH; ++i) x[i] = grow_s[i] * k_s[i * DP + (((e >> 2) ^ (i & 7)) << 2) + (e & 3)];
       }
-#pragma unroll
-      for (int i = 1; i < CH; ++i) {
-        float s[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-        for (int m = 0; m < i; m += 4) {  // the row's entries from i on are zero, as are x's uses of them
-          const float4 row = *reinterpret_cast<const float4*>(a_s + i * A_LD + m);
-          s[0] = fmaf(row.x, x[m], s[0]);
-          if (m + 1 < i) s[1] = fmaf(row.y, x[m + 1], s[1]);
-          if (m + 2 < i) s[2] = fmaf(row.z, x[m + 2], s[2]);
-          if (m + 3 < i) s[3] = fmaf(row.w, x[m + 3], s[3]);
-        }
-        x[i] -= (s[0] + s[1]) + (s[2] + s[3]);
-      }
+      ch_substitute(x, a_s);
       float* dst = value ? a.u + at * CH * dv + e : a.w + at * CH * d + e;
       const int ld = value ? dv : d;
 #pragma unroll
       for (int i = 0; i < CH; ++i) dst[(size_t)i * ld] = x[i];
     }
+  }
+}
+
+// ---- a decay per key channel ------------------------------------------------------------------------------------------ //
+constexpr int CH_SUB = 8;  // tokens of a block inside a run
+
+template <int DP>
+struct ChannelInputsSmem {  // offsets in floats
+  static constexpr int ROWS = CH * DP, A_LD = CH + 4;
+  static constexpr int Q = 0, K = Q + ROWS, G = K + ROWS, C = G + ROWS, R = C + (CH - CH_SUB) * DP, A = R + 2 * CH_SUB * DP;
+  static constexpr int BETA = A + CH * A_LD, FLOATS = BETA + CH;
+  static constexpr size_t BYTES = (size_t)FLOATS * sizeof(float);
+};
+
+// grid (runs, H), 128 threads.  Rows of DP floats lie in shared memory with their 16-byte words XORed as above.  Bound by
+// shared memory: a word of a row of q, one of k and one of a column feed 8 products.
+template <int DP>
+__global__ void __launch_bounds__(128, 3) state_chunk_channel_inputs_kernel(ChunkArgs a) {
+  using L = ChannelInputsSmem<DP>;
+  constexpr int WORDS = DP / 4, A_LD = L::A_LD;
+  extern __shared__ __align__(16) float sm[];
+  float *q_s = sm + L::Q, *k_s = sm + L::K, *g_s = sm + L::G, *c_s = sm + L::C, *r_s = sm + L::R, *a_s = sm + L::A;
+  float* beta_s = sm + L::BETA;
+  const int run = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int H = a.n_heads, G = a.n_kv_heads, d = a.d, dv = a.dv, kvh = h / (H / G);
+  const int seq = a.run_seq[run], row0 = a.run_row0[run];
+  const int n = min(CH, a.seq_qlen[seq] - row0);
+  const size_t tok0 = (size_t)a.seq_qstart[seq] + row0;
+  const size_t at = (size_t)run * H + h;
+  auto place = [&](int row, int channel) { return row * DP + (((channel >> 2) ^ (row & 7)) << 2) + (channel & 3); };
+  for (int i = tid; i < CH * WORDS; i += 128) {
+    const int r = i / WORDS, wd = i % WORDS;
+    const bool in = r < n && wd * 4 < d;
+    const int dst = r * DP + ((wd ^ (r & 7)) << 2);
+    const size_t src = in ? ((tok0 + r) * G + kvh) * d + wd * 4 : 0;
+    ch_copy16(q_s + dst, a.q + src, in);
+    ch_copy16(k_s + dst, a.k + src, in);
+    if (r < n) ch_copy16(g_s + dst, in ? a.channel_decay + ((tok0 + r) * H + h) * d + wd * 4 : a.channel_decay, in);
+    else *reinterpret_cast<float4*>(g_s + dst) = make_float4(1.f, 1.f, 1.f, 1.f);  // nothing decays past the run's end
+  }
+  cp_async_commit();
+  if (tid < CH) beta_s[tid] = tid < n ? a.beta[(tok0 + tid) * H + h] : 0.f;
+  for (int i = tid; i < CH * A_LD; i += 128) a_s[i] = 0.f;
+  cp_async_wait<0>();
+  __syncthreads();
+
+  // Q and K as seen from the run's ends, a channel a thread
+  if (tid < d) {
+    float* qd = a.qd + at * CH * d + tid;
+    float* kd = a.kd + at * CH * d + tid;
+    float grown = 1.f, left = 1.f;
+#pragma unroll 8
+    for (int i = 0; i < CH; ++i) {
+      grown *= g_s[place(i, tid)];
+      qd[(size_t)i * d] = grown * q_s[place(i, tid)];
+    }
+    a.factors[at * d + tid] = grown;
+#pragma unroll 8
+    for (int j = CH - 1; j >= 0; --j) {
+      kd[(size_t)j * d] = left * k_s[place(j, tid)];
+      left *= g_s[place(j, tid)];
+    }
+  }
+
+  // Pairs of one block of 8 tokens: warp b has block b, a lane the column j and a quarter of the channels; it carries
+  // k_j g_(j+1) .. g_i from row to row.
+  {
+    const int first = warp * CH_SUB, j = lane & 7, part = lane >> 3;
+    float p[CH_SUB], w[CH_SUB];
+#pragma unroll
+    for (int i = 0; i < CH_SUB; ++i) p[i] = w[i] = 0.f;
+#pragma unroll 1
+    for (int wd = part; wd < WORDS; wd += 4) {
+      float4 c = *reinterpret_cast<const float4*>(k_s + (first + j) * DP + ((wd ^ j) << 2));
+#pragma unroll
+      for (int i = 0; i < CH_SUB; ++i) {
+        const int word = (first + i) * DP + ((wd ^ i) << 2);
+        const float4 q4 = *reinterpret_cast<const float4*>(q_s + word), k4 = *reinterpret_cast<const float4*>(k_s + word);
+        const float4 g4 = *reinterpret_cast<const float4*>(g_s + word);
+        if (i > j) { c.x *= g4.x; c.y *= g4.y; c.z *= g4.z; c.w *= g4.w; }
+        p[i] = fmaf(q4.x, c.x, fmaf(q4.y, c.y, fmaf(q4.z, c.z, fmaf(q4.w, c.w, p[i]))));
+        w[i] = fmaf(k4.x, c.x, fmaf(k4.y, c.y, fmaf(k4.z, c.z, fmaf(k4.w, c.w, w[i]))));
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < CH_SUB; ++i) {
+#pragma unroll
+      for (int o = 8; o < 32; o <<= 1) {
+        p[i] += __shfl_xor_sync(0xffffffffu, p[i], o);
+        w[i] += __shfl_xor_sync(0xffffffffu, w[i], o);
+      }
+      if (part == (i & 3)) {  // four lanes hold the sums: each writes its share of the rows
+        a.p[(at * CH + first + i) * CH + first + j] = i >= j ? p[i] : 0.f;
+        if (i > j) a_s[(first + i) * A_LD + first + j] = beta_s[first + i] * w[i];
+      }
+    }
+  }
+  for (int i = tid; i < CH * CH; i += 128) {  // what lies right of the diagonal blocks
+    const int r = i / CH, c = i % CH;
+    if (c / CH_SUB > r / CH_SUB) a.p[at * CH * CH + i] = 0.f;
+  }
+  // Pairs of different blocks, block by block of rows
+#pragma unroll 1
+  for (int block = 1; block < CH / CH_SUB; ++block) {
+    const int first = block * CH_SUB;
+    __syncthreads();  // the columns and rows below have been read for the block before
+    for (int e = tid; e < DP; e += 128) {
+      float back = g_s[place(first, e)];  // g_(j+1) .. g_first
+#pragma unroll
+      for (int j = first - 1; j >= first - CH_SUB; --j) {
+        c_s[place(j, e)] = back * k_s[place(j, e)];
+        if (j > first - CH_SUB) back *= g_s[place(j, e)];
+      }
+      // back is now g_(first - 7) .. g_first: what the columns before, which reach to first - 8, still lack
+      for (int j = 0; j < first - CH_SUB; ++j) c_s[place(j, e)] *= back;
+      float grown = 1.f;
+#pragma unroll
+      for (int i = 0; i < CH_SUB; ++i) {
+        if (i > 0) grown *= g_s[place(first + i, e)];
+        r_s[place(i, e)] = grown * q_s[place(first + i, e)];
+        r_s[CH_SUB * DP + place(i, e)] = grown * k_s[place(first + i, e)];
+      }
+    }
+    __syncthreads();
+    const int i = tid & 7, j0 = tid >> 3;  // row i, columns j0 and j0 + 16
+    if (j0 < first) {
+      const bool two = j0 + 16 < first;
+      float p0 = 0.f, p1 = 0.f, w0 = 0.f, w1 = 0.f;
+#pragma unroll 4
+      for (int wd = 0; wd < WORDS; ++wd) {
+        const float4 q4 = *reinterpret_cast<const float4*>(r_s + i * DP + ((wd ^ i) << 2));
+        const float4 k4 = *reinterpret_cast<const float4*>(r_s + (CH_SUB + i) * DP + ((wd ^ i) << 2));
+        const float4 c = *reinterpret_cast<const float4*>(c_s + j0 * DP + ((wd ^ (j0 & 7)) << 2));
+        p0 = fmaf(q4.x, c.x, fmaf(q4.y, c.y, fmaf(q4.z, c.z, fmaf(q4.w, c.w, p0))));
+        w0 = fmaf(k4.x, c.x, fmaf(k4.y, c.y, fmaf(k4.z, c.z, fmaf(k4.w, c.w, w0))));
+        if (two) {
+          const float4 c2 = *reinterpret_cast<const float4*>(c_s + (j0 + 16) * DP + ((wd ^ (j0 & 7)) << 2));
+          p1 = fmaf(q4.x, c2.x, fmaf(q4.y, c2.y, fmaf(q4.z, c2.z, fmaf(q4.w, c2.w, p1))));
+          w1 = fmaf(k4.x, c2.x, fmaf(k4.y, c2.y, fmaf(k4.z, c2.z, fmaf(k4.w, c2.w, w1))));
+        }
+      }
+      const int row = first + i;
+      a.p[(at * CH + row) * CH + j0] = p0;
+      a_s[row * A_LD + j0] = beta_s[row] * w0;
+      if (two) {
+        a.p[(at * CH + row) * CH + j0 + 16] = p1;
+        a_s[row * A_LD + j0 + 16] = beta_s[row] * w1;
+      }
+    }
+  }
+  __syncthreads();
+  float x[CH];
+  for (int col = tid; col < dv + d; col += 128) {
+    const bool value = col < dv;
+    const int e = value ? col : col - dv;
+    if (value) {  // rows past the run's end: the last row, times a beta of 0
+#pragma unroll
+      for (int i = 0; i < CH; ++i) x[i] = a.v[((tok0 + min(i, n - 1)) * H + h) * dv + e];
+#pragma unroll
+      for (int i = 0; i < CH; ++i) x[i] *= beta_s[i];
+    } else {
+      float grown = 1.f;
+#pragma unroll
+      for (int i = 0; i < CH; ++i) {
+        grown *= g_s[place(i, e)];
+        x[i] = beta_s[i] * grown * k_s[place(i, e)];
+      }
+    }
+    ch_substitute(x, a_s);
+    float* dst = value ? a.u + at * CH * dv + e : a.w + at * CH * d + e;
+    const int ld = value ? dv : d;
+#pragma unroll
+    for (int i = 0; i < CH; ++i) dst[(size_t)i * ld] = x[i];
   }
 }
 
@@ -395,11 +584,11 @@ __global__ void __launch_bounds__(128) state_chunk_outputs_kernel(ChunkArgs a) {
 }
 
 // ---- with the delta rule -------------------------------------------------------------------------------------------- //
-template <int DP>
+template <int DP, bool CHANNEL>
 struct ChunkScanSmem {  // offsets in floats
   static constexpr int ROWS = CH * DP, COL_LD = CH_COLS + 4;
   static constexpr int Q = 0, W = Q + 2 * ROWS, K = W + 2 * ROWS, P = K + ROWS, U = P + CH * CH;
-  static constexpr int F = U + CH * COL_LD, S = F + CH_FACTORS, X = S + DP * COL_LD, Y = X + CH * COL_LD;
+  static constexpr int F = U + CH * COL_LD, S = F + (CHANNEL ? DP : CH_FACTORS), X = S + DP * COL_LD, Y = X + CH * COL_LD;
   static constexpr int FLOATS = Y + CH * COL_LD;
   static constexpr size_t BYTES = (size_t)FLOATS * sizeof(float);
 };
@@ -433,9 +622,10 @@ __device__ __forceinline__ int ch_place(int row, int cg) { return row * LD + ((c
 
 // grid (ceil(dv / 16), H, sequences), 128 threads.  For products with S a thread owns rows rg + 8 i (i < 4) of the run,
 // four columns and a quarter of the contraction (every fourth 16-byte word).
-template <int DP>
+// CHANNEL: a decay per key channel, whose Q and K the inputs' kernel has written, 32 whole rows a run.
+template <int DP, bool CHANNEL>
 __global__ void __launch_bounds__(128, 2) state_chunk_scan_kernel(ChunkArgs a) {
-  using L = ChunkScanSmem<DP>;
+  using L = ChunkScanSmem<DP, CHANNEL>;
   constexpr int WORDS = DP / 4, LD = L::COL_LD, RS = DP / 32;
   extern __shared__ __align__(16) float sm[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -451,29 +641,32 @@ __global__ void __launch_bounds__(128, 2) state_chunk_scan_kernel(ChunkArgs a) {
   constexpr int STEP = 128 / WORDS;
   const int load_row = tid / WORDS, load_word = (tid % WORDS) * 4;
   const bool load_col = load_word < d;
-  const size_t qk_ld = (size_t)G * d;
-  const float* q_at = a.q + (tok_base + load_row) * qk_ld + (size_t)kvh * d + load_word;
-  const float* k_at = a.k + (tok_base + load_row) * qk_ld + (size_t)kvh * d + load_word;
+  const size_t qk_ld = CHANNEL ? d : (size_t)G * d, qk_run = CHANNEL ? (size_t)H * CH * d : CH * qk_ld;
+  const size_t qk_first = CHANNEL ? (((size_t)run0 * H + h) * CH + load_row) * d + load_word
+                                  : (tok_base + load_row) * qk_ld + (size_t)kvh * d + load_word;
+  const float* q_at = (CHANNEL ? a.qd : a.q) + qk_first;
+  const float* k_at = (CHANNEL ? a.kd : a.k) + qk_first;
+  const int f_ld = CHANNEL ? d : CH_FACTORS;
   const float* w_at = a.w + (((size_t)run0 * H + h) * CH + load_row) * d + load_word;
   const float* p_at = a.p + ((size_t)run0 * H + h) * CH * CH + tid * 4;
   const float* u_at = a.u + (((size_t)run0 * H + h) * CH + (tid >> 2)) * dv + col0 + (tid & 3) * 4;
-  const float* f_at = a.factors + ((size_t)run0 * H + h) * CH_FACTORS + tid * 4;
+  const float* f_at = a.factors + ((size_t)run0 * H + h) * f_ld + tid * 4;
   auto load_products = [&](int c) {  // Q and W of run c, which follow those of run c - 1
     float* q_s = sm + L::Q + (c & 1) * L::ROWS + tid * 4;
     float* w_s = sm + L::W + (c & 1) * L::ROWS + tid * 4;
-    const int rows = load_col ? len - c * CH - load_row : 0;
+    const int rows = load_col ? (CHANNEL ? CH : len - c * CH - load_row) : 0;
 #pragma unroll 2
     for (int j = 0; j < CH / STEP; ++j) {
       const bool in = j * STEP < rows;
       ch_copy16(q_s + j * 512, in ? q_at + j * STEP * qk_ld : a.q, in);
       ch_copy16(w_s + j * 512, load_col ? w_at + (size_t)j * STEP * d : a.w, load_col);
     }
-    q_at += CH * qk_ld;
+    q_at += qk_run;
     w_at += (size_t)H * CH * d;
   };
   auto load_writes = [&](int c) {  // K, P, U and the factors of run c, likewise
     float* k_s = sm + L::K + tid * 4;
-    const int rows = load_col ? len - c * CH - load_row : 0;
+    const int rows = load_col ? (CHANNEL ? CH : len - c * CH - load_row) : 0;
 #pragma unroll 2
     for (int j = 0; j < CH / STEP; ++j) {
       const bool in = j * STEP < rows;
@@ -483,11 +676,15 @@ __global__ void __launch_bounds__(128, 2) state_chunk_scan_kernel(ChunkArgs a) {
     ch_copy16(sm + L::P + tid * 4 + 512, p_at + 512, true);
     const bool in = col0 + (tid & 3) * 4 < dv;
     ch_copy16(sm + L::U + (tid >> 2) * LD + (tid & 3) * 4, in ? u_at : a.u, in);
-    if (tid < CH_FACTORS / 4) ch_copy16(sm + L::F + tid * 4, f_at, true);
-    k_at += CH * qk_ld;
+    if constexpr (CHANNEL) {
+      if (tid < WORDS) ch_copy16(sm + L::F + tid * 4, tid * 4 < d ? f_at : a.factors, tid * 4 < d);
+    } else if (tid < CH_FACTORS / 4) {
+      ch_copy16(sm + L::F + tid * 4, f_at, true);
+    }
+    k_at += qk_run;
     p_at += (size_t)H * CH * CH;
     u_at += (size_t)H * CH * dv;
-    f_at += (size_t)H * CH_FACTORS;
+    f_at += (size_t)H * f_ld;
   };
 
   // this thread's piece of the state: rows dg RS .. + RS - 1, columns 4 sc .. 4 sc + 3
@@ -536,13 +733,13 @@ __global__ void __launch_bounds__(128, 2) state_chunk_scan_kernel(ChunkArgs a) {
       float4 x = *reinterpret_cast<const float4*>(sm + L::U + row_of_lane * LD + cg * 4);
       const float4 y = ch_reduce(corr, kg);
       x.x -= y.x; x.y -= y.y; x.z -= y.z; x.w -= y.w;
-      const float left = f[CH + row_of_lane];
+      const float left = CHANNEL ? 1.f : f[CH + row_of_lane];
       *reinterpret_cast<float4*>(sm + L::X + ch_place<LD>(row_of_lane, cg)) = x;
       *reinterpret_cast<float4*>(sm + L::Y + row_of_lane * LD + cg * 4) = make_float4(left * x.x, left * x.y, left * x.z, left * x.w);
     }
     __syncthreads();
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < (CHANNEL ? 0 : 4); ++i) {
       const float grown = f[rg + 8 * i];
 #pragma unroll
       for (int j = 0; j < 4; ++j) acc[i][j] *= grown;
@@ -561,11 +758,12 @@ __global__ void __launch_bounds__(128, 2) state_chunk_scan_kernel(ChunkArgs a) {
       if (t < len && col0 + cg * 4 < dv)
         *reinterpret_cast<float4*>(a.out + ((tok_base + t) * H + h) * dv + col0 + cg * 4) = o;
     }
-    const float left = f[2 * CH];
 #pragma unroll
-    for (int i = 0; i < RS; ++i)
+    for (int i = 0; i < RS; ++i) {
+      const float left = f[CHANNEL ? dg * RS + i : 2 * CH];
 #pragma unroll
       for (int j = 0; j < 4; ++j) s[i][j] *= left;
+    }
 #pragma unroll 8
     for (int t = 0; t < CH; ++t) {
       float kr[RS];
@@ -603,12 +801,22 @@ static int reserve(Kernel kernel, size_t smem) {
 
 template <int DP>
 static int launch_chunks(const ChunkArgs& a, int n_runs, int n_seqs, cudaStream_t stream) {
+  if (a.channel_decay) {
+    constexpr size_t in_smem = ChannelInputsSmem<DP>::BYTES, smem = ChunkScanSmem<DP, true>::BYTES;
+    if (const int err = reserve(state_chunk_channel_inputs_kernel<DP>, in_smem)) return err;
+    MLL_LAUNCH((state_chunk_channel_inputs_kernel<DP>), dim3(n_runs, a.n_heads), 128, in_smem, stream, a);
+    MLL_LAUNCH_CHECK();
+    if (const int err = reserve(state_chunk_scan_kernel<DP, true>, smem)) return err;
+    MLL_LAUNCH((state_chunk_scan_kernel<DP, true>), dim3((a.dv + CH_COLS - 1) / CH_COLS, a.n_heads, n_seqs), 128, smem, stream, a);
+    MLL_LAUNCH_CHECK();
+    return 0;
+  }
   if (a.beta) {
     MLL_LAUNCH((state_chunk_inputs_kernel<DP, true>), dim3(n_runs, a.n_heads), 128, 0, stream, a);
     MLL_LAUNCH_CHECK();
-    constexpr size_t smem = ChunkScanSmem<DP>::BYTES;
-    if (const int err = reserve(state_chunk_scan_kernel<DP>, smem)) return err;
-    MLL_LAUNCH((state_chunk_scan_kernel<DP>), dim3((a.dv + CH_COLS - 1) / CH_COLS, a.n_heads, n_seqs), 128, smem, stream, a);
+    constexpr size_t smem = ChunkScanSmem<DP, false>::BYTES;
+    if (const int err = reserve(state_chunk_scan_kernel<DP, false>, smem)) return err;
+    MLL_LAUNCH((state_chunk_scan_kernel<DP, false>), dim3((a.dv + CH_COLS - 1) / CH_COLS, a.n_heads, n_seqs), 128, smem, stream, a);
     MLL_LAUNCH_CHECK();
     return 0;
   }
@@ -634,31 +842,36 @@ MLL_API int mll_state_chunk_tokens() { return mll::CH; }
 
 MLL_API int mll_state_chunks_supported(int d, int dv) { return d > 0 && d <= 128 && d % 4 == 0 && dv > 0 && dv % 4 == 0; }
 
-// Floats of scratch memory for `n_runs` runs.
+// Floats of scratch memory for `n_runs` runs (delta: 0 none, 1 the delta rule, 2 the delta rule with a decay per channel).
 MLL_API long long mll_state_chunks_scratch(int n_runs, int n_heads, int d, int dv, int delta) {
-  return (long long)n_runs * n_heads * (mll::CH * mll::CH + mll::CH_FACTORS + (delta ? mll::CH * (d + dv) : d * dv));
+  const int own = delta == 2 ? d + mll::CH * (3 * d + dv) : mll::CH_FACTORS + (delta ? mll::CH * (d + dv) : d * dv);
+  return (long long)n_runs * n_heads * (mll::CH * mll::CH + own);
 }
 
-// As mll_state_scan modes 0, 3 (token_decay given) and 4 (beta too), a run of tokens at a time.  run_seq, run_row0
+// As mll_state_scan modes 0, 3 (token_decay given), 4 (beta too) and 1 (channel_decay [T, H, d] and beta), a run of tokens at a time.  run_seq, run_row0
 // [n_runs]: every sequence's runs one after another, each of up to 32 tokens; seq_run0 [n_seqs]: its first run.
 MLL_API int mll_state_chunks(const float* q, const float* k, const float* v, const float* beta, const float* token_decay,
-                             const float* head_decay, float* state, float* out, float* scratch, const int* run_seq,
-                             const int* run_row0, const int* seq_run0, const int* seq_slot, const int* seq_qstart,
+                             const float* head_decay, const float* channel_decay, float* state, float* out, float* scratch,
+                             const int* run_seq, const int* run_row0, const int* seq_run0, const int* seq_slot, const int* seq_qstart,
                              const int* seq_qlen, int n_runs, int n_seqs, int n_heads, int n_kv_heads, int d, int dv,
                              cudaStream_t stream) {
   MLL_REQUIRE(n_runs >= 0 && n_seqs >= 0 && n_heads > 0 && n_kv_heads > 0 && n_heads % n_kv_heads == 0, "state chunks: bad head counts");
   MLL_REQUIRE(mll_state_chunks_supported(d, dv), "state chunks: head sizes %d / %d", d, dv);
   MLL_REQUIRE(n_heads <= 65535 && n_seqs <= 65535, "state chunks: too many heads or sequences for one launch");
-  MLL_REQUIRE((token_decay == nullptr) != (head_decay == nullptr) && (!beta || token_decay), "state chunks: the decay's inputs do not fit");
-  MLL_REQUIRE(((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)state | (uintptr_t)out | (uintptr_t)scratch) % 16 == 0,
+  MLL_REQUIRE((token_decay != nullptr) + (head_decay != nullptr) + (channel_decay != nullptr) == 1 && (beta ? !head_decay : !channel_decay),
+              "state chunks: the decay's inputs do not fit");
+  MLL_REQUIRE(((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)channel_decay | (uintptr_t)state | (uintptr_t)out | (uintptr_t)scratch) % 16 == 0,
               "state chunks: operands must be 16-byte aligned");
   if (n_seqs == 0 || n_runs == 0) return 0;
   const size_t pairs = (size_t)n_runs * n_heads;
   float* p = scratch;
   float* factors = p + pairs * mll::CH * mll::CH;
-  float* u = factors + pairs * mll::CH_FACTORS;
+  float* u = factors + pairs * (channel_decay ? d : mll::CH_FACTORS);
   float* w = u + pairs * mll::CH * dv;  // without the delta rule the runs' sums stand in the place of u and w
-  mll::ChunkArgs a{q, k, v, beta, token_decay, head_decay, state, out, p, beta ? w : nullptr, beta ? u : nullptr, factors, beta ? nullptr : u,
+  float* qd = channel_decay ? w + pairs * mll::CH * d : nullptr;
+  float* kd = channel_decay ? qd + pairs * mll::CH * d : nullptr;
+  mll::ChunkArgs a{q, k, v, beta, token_decay, head_decay, channel_decay, state, out, p, beta ? w : nullptr, beta ? u : nullptr, factors,
+                   qd, kd, beta ? nullptr : u,
                    run_seq, run_row0, seq_run0, seq_slot, seq_qstart, seq_qlen, n_heads, n_kv_heads, d, dv};
   if (d <= 32) return mll::launch_chunks<32>(a, n_runs, n_seqs, stream);
   if (d <= 64) return mll::launch_chunks<64>(a, n_runs, n_seqs, stream);

@@ -27,8 +27,9 @@ write, and normalise o by its root mean square (per head, or a row at once) befo
                      o + D_h x, times silu(z), normalised in a few equal parts of the row, times a weight, then W_o;
                      the last taps - 1 convolution inputs of a sequence are state too
 
-Where the decay is one number per head - fixed or per token - prompts take the recurrence a run of tokens at a time
-(`_recur`); decays per key channel and single tokens take it token by token.
+Where the decay is one number per head - fixed or per token - and for the delta rule with a decay per key channel, prompts
+take the recurrence a run of tokens at a time (`_recur`); single tokens, and decays per key channel without the delta rule,
+are taken token by token.
 
 What enters the recurrence is float32 (decays, step sizes, gates, unit vectors, the state); the projections are
 products in the run's dtype.  Sizes, decays, tap counts and eps are parameters.
@@ -73,18 +74,19 @@ def _run_lists(shape):
 
 
 def _recur(step, q, k, v, state, o, H: int, G: int, d: int, dv: int, head_decay=None, token_decay=None, beta=None,
-           runs: bool = True) -> None:
-    """The recurrence with one decay per head over the step's tokens: a run of tokens at a time in prompt steps, token by
+           channel_decay=None, runs: bool = True) -> None:
+    """The recurrence with one decay per head, or the delta rule with one per key channel, over the step's tokens: a run of tokens at a time in prompt steps, token by
     token otherwise (and where `runs` is off: a decay outside [0, 1] has no logarithm to work with)."""
     lists = step.meta.get(RUNS) if runs and not step.all_decode else None
     if lists and step.n_tokens >= CHUNK_FROM * step.n_seqs and K.state_chunks_supported(d, dv):
-        scratch = step.ws.buffer("state.runs", (K.state_chunks_scratch(lists["run_seq"].shape[0], H, d, dv, beta is not None),),
+        scratch = step.ws.buffer("state.runs", (K.state_chunks_scratch(lists["run_seq"].shape[0], H, d, dv, beta is not None,
+                                                                  channel_decay is not None),),
                                  torch.float32)
         K.state_chunks(q, k, v, state, o, scratch, lists["run_seq"], lists["run_row0"], lists["seq_run0"], step.seq_slot,
                        step.seq_qstart, step.seq_qlen, step.n_seqs, H, G, d, dv, head_decay=head_decay,
-                       token_decay=token_decay, beta=beta)
+                       token_decay=token_decay, beta=beta, channel_decay=channel_decay)
         return
-    K.state_scan(q, k, v, None, beta, head_decay, state, o, step.seq_slot, step.seq_qstart, step.seq_qlen, step.n_seqs, H, G,
+    K.state_scan(q, k, v, channel_decay, beta, head_decay, state, o, step.seq_slot, step.seq_qstart, step.seq_qlen, step.n_seqs, H, G,
                  d, dv, token_decay=token_decay)
 
 
@@ -165,7 +167,7 @@ class Retention(_RecursInRuns):
         return self.o.forward(step, gated, "o")
 
 
-class GatedDeltaRule(Mixer):
+class GatedDeltaRule(_RecursInRuns):
     """params: n_heads, n_kv_heads (q and k heads; value head h reads q/k head h // (n_heads / n_kv_heads)),
     head_dim, v_head_dim, conv (taps), eps (of the head norm), unit_eps (inside the root of the unit length),
     names: tensor names for "q","k","v" (their convolution taps are "<name>.conv"), "b", "a1", "a2", "dt_bias",
@@ -254,8 +256,7 @@ class GatedDeltaRule(Mixer):
         K.conv_state_update(proj, cache.state["conv"], step.seq_slot, step.seq_qstart, step.seq_qlen, step.n_seqs,
                             self.channels, self.taps)
         o = ws.buffer("mix.o", (T, H * dv), torch.float32)
-        K.state_scan(q, k, v, g, beta, None, cache.state["S"], o, step.seq_slot, step.seq_qstart, step.seq_qlen,
-                     step.n_seqs, H, G, d, dv)
+        _recur(step, q, k, v, cache.state["S"], o, H, G, d, dv, beta=beta, channel_decay=g)
         gated = ws.buffer("mix.gated", (T, H * dv), self.ctx.act_dtype)
         K.head_norm_gate(o, self.norm_w, high, gated, H, dv, self.eps, K.GATE_SIGMOID, gate_col=H * d)
         return self.o.forward(step, gated, "o")
