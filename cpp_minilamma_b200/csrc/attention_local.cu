@@ -138,8 +138,8 @@ __global__ void __launch_bounds__(256) local_prepare_kernel(LocalPrepArgs a) {
   }
 }
 
-// The same for bfloat16 rows that are whole 16-byte words and rotated halves of whole words: a thread owns eight
-// neighbouring dimensions.  The row waits in shared memory between the norm's sums and the rotation, which needs the
+// The same for bfloat16 rows that are whole 16-byte words and rotated halves of whole words, or neighbours rotated in pairs
+// (inside a word): a thread owns eight neighbouring dimensions.  The row waits in shared memory between the norm's sums and the rotation, which needs the
 // partner half.
 __global__ void __launch_bounds__(256) local_prepare_vec_kernel(LocalPrepArgs a) {
   extern __shared__ __align__(16) uint4 row_s[];
@@ -197,7 +197,14 @@ __global__ void __launch_bounds__(256) local_prepare_vec_kernel(LocalPrepArgs a)
     const int c = is_q ? i : i - nq, head = c / dw, e = c - head * dw;
     float x[8];
     scaled(i, is_q, x);
-    if (cs && e < 2 * hw) {
+    if (cs && a.interleaved && e * 8 < a.rot) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float co = cs[e * 4 + k], si = sn[e * 4 + k], u = x[2 * k], v = x[2 * k + 1];
+        x[2 * k] = u * co - v * si;
+        x[2 * k + 1] = v * co + u * si;
+      }
+    } else if (cs && !a.interleaved && e < 2 * hw) {
       const bool first = e < hw;
       float y[8];
       scaled(first ? i + hw : i - hw, is_q, y);
@@ -716,7 +723,7 @@ MLL_API int mll_local_attention_prepare(const void* qkv, const float* q_weight, 
                        v_from_k ? n_heads * d : n_heads * d + n_kv_heads * d, write_kv ? 1 : 0};
   const auto whole = [](const void* p) { return (uintptr_t)p % 16 == 0; };
   const size_t row_bytes = (size_t)(n_heads + (write_kv ? n_kv_heads : 0)) * d * 2;
-  if (dtype == MLL_BF16 && d % 8 == 0 && dv % 8 == 0 && ld % 8 == 0 && (rot == 0 || (!interleaved && rot % 16 == 0)) &&
+  if (dtype == MLL_BF16 && d % 8 == 0 && dv % 8 == 0 && ld % 8 == 0 && rot % (interleaved ? 8 : 16) == 0 &&
       row_bytes <= 48 * 1024 && whole(qkv) && whole(q_out) && whole(k_cache) && whole(v_cache) && whole(q_weight) && whole(k_weight)) {
     MLL_LAUNCH((mll::local_prepare_vec_kernel), n_tokens, 256, row_bytes, stream, a);
     MLL_LAUNCH_CHECK();

@@ -383,12 +383,14 @@ MLL_API int mll_moe_route(const void* h, const float* w, const float* bias, cons
     groups = groups_kept = 0;
   }
   const size_t smem = (size_t)(2 * n_experts + 1 + groups) * sizeof(float);
+  // with the logits given there is work for one warp a token only (5,957 tokens, 16 experts: 29 us with blocks of 512, 7.4 with one warp)
+  const int threads = logits ? 32 : 512;
   const mll::RouteForm form{all_scores, scale, gate_out, groups, groups_kept};
   if (dtype == MLL_F32)
-    MLL_LAUNCH((mll::moe_route_kernel<float>), n_tokens, 512, smem, stream, (const float*)h, w, bias, logits, chosen,
+    MLL_LAUNCH((mll::moe_route_kernel<float>), n_tokens, threads, smem, stream, (const float*)h, w, bias, logits, chosen,
                weight, n_tokens, width, n_experts, top, form);
   else if (dtype == MLL_BF16)
-    MLL_LAUNCH((mll::moe_route_kernel<__nv_bfloat16>), n_tokens, 512, smem, stream, (const __nv_bfloat16*)h, w, bias,
+    MLL_LAUNCH((mll::moe_route_kernel<__nv_bfloat16>), n_tokens, threads, smem, stream, (const __nv_bfloat16*)h, w, bias,
                logits, chosen, weight, n_tokens, width, n_experts, top, form);
   else
     MLL_REQUIRE(false, "moe route: unknown dtype %d", dtype);

@@ -88,7 +88,10 @@ __global__ void __launch_bounds__(256) retention_prepare_kernel(RetPrepArgs a) {
   }
 }
 
-// Without a rotation every column is by itself: eight neighbouring ones a thread (all sizes multiples of 8).
+// The same, eight neighbouring columns a thread (all sizes multiples of 8; rotated halves of whole words, or pairs of
+// neighbours inside a word).  A block a token, a column a thread, left 16 tokens on 16 multiprocessors: 9.3 us for them, 22.6
+// for 2,047 tokens of 8 heads of 128 and 256 (50 MB: 7.7 us at the copy peak), here 3.5 and
+// 12.1.
 template <typename T>
 __global__ void __launch_bounds__(256) retention_prepare_vec_kernel(RetPrepArgs a, long long words) {
   const int n = a.n_heads * a.d, nv = a.n_heads * a.dv, per_row = (2 * n + nv) / 8;
@@ -96,7 +99,33 @@ __global__ void __launch_bounds__(256) retention_prepare_vec_kernel(RetPrepArgs 
     const size_t t = (size_t)(i / per_row);
     const int c = (int)(i % per_row) * 8;
     float x[8];
-    load_floats<T, 8>((const T*)a.proj + t * a.ld + c, x);
+    const T* src = (const T*)a.proj + t * a.ld + c;
+    load_floats<T, 8>(src, x);
+    const int e = a.cos_table && c < 2 * n ? c % a.d : a.rot;
+    if (e < a.rot) {
+      const int half = a.rot >> 1;
+      const float* cs = a.cos_table + (size_t)a.tok_pos[t] * half;
+      const float* sn = a.sin_table + (size_t)a.tok_pos[t] * half;
+      float co[8], si[8];
+      if (a.interleaved) {
+        load_floats<float, 4>(cs + e / 2, co);
+        load_floats<float, 4>(sn + e / 2, si);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float first = x[2 * j], second = x[2 * j + 1];
+          x[2 * j] = first * co[j] - second * si[j];
+          x[2 * j + 1] = second * co[j] + first * si[j];
+        }
+      } else {
+        const bool first = e < half;
+        float y[8];
+        load_floats<T, 8>(first ? src + half : src - half, y);
+        load_floats<float, 8>(cs + (first ? e : e - half), co);
+        load_floats<float, 8>(sn + (first ? e : e - half), si);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) x[j] = first ? x[j] * co[j] - y[j] * si[j] : x[j] * co[j] + y[j] * si[j];
+      }
+    }
     const float f = c >= n && c < 2 * n ? a.k_scale : 1.f;
 #pragma unroll
     for (int j = 0; j < 8; ++j) x[j] = (a.silu ? silu_f(x[j]) : x[j]) * f;
@@ -375,6 +404,84 @@ __global__ void __launch_bounds__(256) ssd_prepare_kernel(SsdPrepArgs a, int per
       a.q[(size_t)t * gn + (c - inner - gn)] = y;
     }
   }
+}
+
+// The same for channels in words of eight (every size a multiple of 8) and up to four taps: a thread owns eight channels and
+// walks WALK consecutive tokens, whose rows it asks for together; the inputs that the taps look back on stay in registers.  5,957
+// tokens of 6,144 channels (317 MB in and out, 49 us at the copy peak): 231 us a channel a thread, 24 single tokens 12.3 us;
+// here 95 us.
+template <typename T, int TAPS, int WALK>
+__global__ void __launch_bounds__(128) ssd_prepare_walk_kernel(SsdPrepArgs a, int n_tokens) {
+  const int H = a.n_heads, G = a.n_groups, d = a.d, dv = a.dv, inner = H * dv, gn = G * d, C = inner + 2 * gn;
+  const int c = (blockIdx.x * 128 + threadIdx.x) * 8;
+  if (c >= C) return;
+  const int first = blockIdx.y * WALK, n = min(WALK, n_tokens - first);
+  const T* proj = (const T*)a.proj + inner + c;
+  RawWord<T, 8> raw[WALK];
+#pragma unroll
+  for (int i = 0; i < WALK; ++i) raw[i].fetch(proj + (size_t)(first + min(i, n - 1)) * a.ld);
+  float w[8 * TAPS], b[8], before[TAPS][8];  // before[j]: the input j + 1 tokens ago (the last one is not used)
+#pragma unroll
+  for (int i = 0; i < 8 * TAPS; i += 4) load_floats<float, 4>(a.conv_w + (size_t)c * TAPS + i, w + i);
+  load_floats<float, 8>(a.conv_b + c, b);
+  const bool x_part = c < inner;
+  const int h = x_part ? c / dv : 0;
+  const float dt_bias = x_part ? a.dt_bias[h] : 0.f, rate = x_part ? expf(a.a_log[h]) : 0.f;
+#pragma unroll
+  for (int i = 0; i < WALK; ++i) {
+    if (i >= n) break;
+    const int t = first + i, seq = a.tok_seq[t], local = t - a.seq_qstart[seq];
+    if (i == 0 || local == 0) {
+      const float* state = a.conv_state + (size_t)a.seq_slot[seq] * (TAPS - 1) * C + c;
+#pragma unroll
+      for (int back = 1; back < TAPS; ++back) {
+        if (back <= local) load_floats<T, 8>(proj + (size_t)(t - back) * a.ld, before[back - 1]);
+        else load_floats<float, 8>(state + (size_t)(local - back + TAPS - 1) * C, before[back - 1]);
+      }
+    }
+    float y[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      float s = fmaf(w[j * TAPS + TAPS - 1], raw[i][j], b[j]);
+#pragma unroll
+      for (int back = 1; back < TAPS; ++back) s = fmaf(w[j * TAPS + TAPS - 1 - back], before[back - 1][j], s);
+      y[j] = silu_f(s);
+#pragma unroll
+      for (int back = TAPS - 1; back > 1; --back) before[back - 1][j] = before[back - 2][j];
+      if (TAPS > 1) before[0][j] = raw[i][j];
+    }
+    if (x_part) {
+      const float dt = softplus_f(to_float(((const T*)a.proj)[(size_t)t * a.ld + inner + C + h]) + dt_bias);
+      if (c % dv == 0) a.decay[(size_t)t * H + h] = expf(-rate * dt);
+      store_floats<float, 8>(a.xs + (size_t)t * inner + c, y);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) y[j] *= dt;
+      store_floats<float, 8>(a.u + (size_t)t * inner + c, y);
+    } else if (c < inner + gn) {
+      store_floats<float, 8>(a.k + (size_t)t * gn + (c - inner), y);
+    } else {
+      store_floats<float, 8>(a.q + (size_t)t * gn + (c - inner - gn), y);
+    }
+  }
+}
+
+template <typename T, int TAPS>
+int launch_ssd_walk(const SsdPrepArgs& a, int n_tokens, cudaStream_t stream) {
+  const int pieces = ((a.n_heads * a.dv + 2 * a.n_groups * a.d) / 8 + 127) / 128;
+  // tokens enough for several blocks a multiprocessor: walks of eight, else every token by itself
+  if (n_tokens >= 4 * mll_sm_count())
+    MLL_LAUNCH((ssd_prepare_walk_kernel<T, TAPS, 8>), dim3(pieces, (n_tokens + 7) / 8), 128, 0, stream, a, n_tokens);
+  else
+    MLL_LAUNCH((ssd_prepare_walk_kernel<T, TAPS, 1>), dim3(pieces, n_tokens), 128, 0, stream, a, n_tokens);
+  MLL_LAUNCH_CHECK();
+  return 0;
+}
+
+template <typename T>
+int launch_ssd_walk_taps(const SsdPrepArgs& a, int n_tokens, cudaStream_t stream) {
+  if (a.taps == 2) return launch_ssd_walk<T, 2>(a, n_tokens, stream);
+  if (a.taps == 3) return launch_ssd_walk<T, 3>(a, n_tokens, stream);
+  return launch_ssd_walk<T, 4>(a, n_tokens, stream);
 }
 
 // grid (ceil(C / 128), sequences): new state = the last taps - 1 of (old state, this step's inputs)
@@ -890,6 +997,76 @@ __global__ void __launch_bounds__(256) row_norm_gate_kernel(const float* __restr
   }
 }
 
+// The kernel below for parts of up to 128 WORDS columns in words of four: a warp a (token, part), which keeps
+// the part in registers between the sum and the scaling.  5,957 tokens of 4,096 columns in 8 parts (293 MB, 45 us at the copy
+// peak): 110 us a block a part, here 47.
+template <typename T, typename GateT, int WORDS>
+__global__ void __launch_bounds__(256) gated_group_norm_warp_kernel(const float* __restrict__ o, const float* __restrict__ xs,
+                                                                    const float* __restrict__ skip,
+                                                                    const GateT* __restrict__ gate, int gate_ld,
+                                                                    const float* __restrict__ weight, T* __restrict__ out,
+                                                                    int n_tokens, int width, int dv, int parts, float eps) {
+  const int lane = threadIdx.x & 31;
+  const long long at = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (at >= (long long)n_tokens * parts) return;
+  const size_t t = (size_t)(at / parts);
+  const int n = width / parts, c0 = (int)(at % parts) * n;
+  float held[WORDS][4], ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < WORDS; ++i) {
+    const int c = c0 + (lane + 32 * i) * 4;
+    const bool in = (lane + 32 * i) * 4 < n;
+    float y[4] = {0.f, 0.f, 0.f, 0.f}, x[4], z[4];
+    if (in) {
+      load_floats<float, 4>(o + t * width + c, y);
+      load_floats<GateT, 4>(gate + t * gate_ld + c, z);
+      if (xs) {
+        load_floats<float, 4>(xs + t * width + c, x);
+        const float f = skip[c / dv];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) y[j] = fmaf(f, x[j], y[j]);
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) y[j] *= silu_f(z[j]);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      held[i][j] = y[j];
+      ss += y[j] * y[j];
+    }
+  }
+  const float f = 1.f / sqrtf(warp_sum(ss) / (float)n + eps);
+#pragma unroll
+  for (int i = 0; i < WORDS; ++i) {
+    const int c = c0 + (lane + 32 * i) * 4;
+    if ((lane + 32 * i) * 4 >= n) continue;
+    float w[4];
+    load_floats<float, 4>(weight + c, w);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) w[j] *= held[i][j] * f;
+    store_floats<T, 4>(out + t * width + c, w);
+  }
+}
+
+template <typename T, typename GateT>
+int launch_group_norm_warp(const float* o, const float* xs, const float* skip, const GateT* gate, int gate_ld, const float* weight,
+                           T* out, int n_tokens, int width, int dv, int parts, float eps, cudaStream_t stream) {
+  const int words = (width / parts + 127) / 128;
+  const long long pieces = (long long)n_tokens * parts;
+  const int warps = pieces < (long long)mll_sm_count() * 32 ? 1 : 8;  // few: one a block, spread over the device
+  const unsigned blocks = (unsigned)((pieces + warps - 1) / warps);
+#define MLL_GGN_WARP(W)                                                                                                     \
+  MLL_LAUNCH((gated_group_norm_warp_kernel<T, GateT, W>), blocks, warps * 32, 0, stream, o, xs, skip, gate, gate_ld, weight, out, \
+             n_tokens, width, dv, parts, eps)
+  if (words <= 1) MLL_GGN_WARP(1);
+  else if (words <= 2) MLL_GGN_WARP(2);
+  else if (words <= 4) MLL_GGN_WARP(4);
+  else MLL_GGN_WARP(8);
+#undef MLL_GGN_WARP
+  MLL_LAUNCH_CHECK();
+  return 0;
+}
+
 // grid (tokens, parts), 256 threads: a row of o [H dv] in `parts` equal pieces, each normalised by its own root mean
 // square after the skip and the gate:   y = (o + skip[h] xs) * silu(z);   out = y / sqrt(mean_part(y^2) + eps) * weight
 template <typename T, typename GateT>
@@ -963,6 +1140,11 @@ MLL_API int mll_ssd_prepare(const void* proj, const float* conv_w, const float* 
   if (n_tokens == 0) return 0;
   mll::SsdPrepArgs a{proj, conv_w, conv_b, conv_state, a_log, dt_bias, tok_seq, seq_slot, seq_qstart, q, k, u, xs, decay,
                      ld, n_heads, n_groups, d, dv, taps};
+  if ((dtype == MLL_F32 || dtype == MLL_BF16) && taps >= 2 && taps <= 4 && dv % 8 == 0 && (n_groups * d) % 8 == 0 && ld % 8 == 0 &&
+      n_tokens <= 65535 && ((uintptr_t)proj | (uintptr_t)conv_w | (uintptr_t)conv_b | (uintptr_t)conv_state | (uintptr_t)q |
+                            (uintptr_t)k | (uintptr_t)u | (uintptr_t)xs) % 16 == 0)
+    return dtype == MLL_F32 ? mll::launch_ssd_walk_taps<float>(a, n_tokens, stream)
+                            : mll::launch_ssd_walk_taps<__nv_bfloat16>(a, n_tokens, stream);
   const size_t smem = (size_t)n_heads * sizeof(float);
   const int channels = n_heads * dv + 2 * n_groups * d;
   // a prompt fills the device with a block a token, which walks its channels (2,048 tokens of 6,144 channels: 115 us
@@ -988,6 +1170,17 @@ MLL_API int mll_gated_group_norm(const float* o, const float* xs, const float* s
   MLL_REQUIRE((xs == nullptr) == (skip == nullptr), "gated group norm: a skip needs its input and its factors");
   MLL_REQUIRE(parts <= 65535, "gated group norm: too many parts for one launch");
   if (n_tokens == 0) return 0;
+  const int columns = width / parts;
+  if (columns % 4 == 0 && columns <= 1024 && dv % 4 == 0 && gate_ld % 4 == 0 && out_dtype == gate_dtype &&
+      (long long)n_tokens * parts < (1ll << 31) &&
+      ((uintptr_t)o | (uintptr_t)xs | (uintptr_t)gate | (uintptr_t)weight | (uintptr_t)out) % 16 == 0) {
+    if (out_dtype == MLL_F32)
+      return mll::launch_group_norm_warp<float, float>(o, xs, skip, (const float*)gate, gate_ld, weight, (float*)out, n_tokens,
+                                                       width, dv, parts, eps, stream);
+    if (out_dtype == MLL_BF16)
+      return mll::launch_group_norm_warp<__nv_bfloat16, __nv_bfloat16>(o, xs, skip, (const __nv_bfloat16*)gate, gate_ld, weight,
+                                                                       (__nv_bfloat16*)out, n_tokens, width, dv, parts, eps, stream);
+  }
   const dim3 grid(n_tokens, parts);
 #define MLL_GGN(T, GT)                                                                                             \
   MLL_LAUNCH((mll::gated_group_norm_kernel<T, GT>), grid, 256, 0, stream, o, xs, skip, (const GT*)gate, gate_ld, \
@@ -1010,7 +1203,9 @@ MLL_API int mll_retention_prepare(const void* proj, const float* cos_table, cons
   if (n_tokens == 0) return 0;
   mll::RetPrepArgs a{proj, rot > 0 ? cos_table : nullptr, sin_table, tok_pos, q, k, v, ld, n_heads, d, dv, rot,
                      interleaved, k_scale, silu};
-  if (rot == 0 && (n_heads * d) % 8 == 0 && (n_heads * dv) % 8 == 0 && ld % 8 == 0 && (uintptr_t)proj % 16 == 0 &&
+  const bool words_rotate = rot == 0 || (d % 8 == 0 && rot % (interleaved ? 8 : 16) == 0 &&
+                                         ((uintptr_t)cos_table | (uintptr_t)sin_table) % 16 == 0);
+  if (words_rotate && (n_heads * d) % 8 == 0 && (n_heads * dv) % 8 == 0 && ld % 8 == 0 && (uintptr_t)proj % 16 == 0 &&
       (uintptr_t)q % 16 == 0 && (uintptr_t)k % 16 == 0 && (uintptr_t)v % 16 == 0 && (dtype == MLL_F32 || dtype == MLL_BF16)) {
     const long long words = (long long)n_tokens * (n_heads * (2 * d + dv) / 8);
     const long long want = (words + 255) / 256, most = (long long)mll_sm_count() * 16;
