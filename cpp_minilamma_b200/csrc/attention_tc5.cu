@@ -194,8 +194,7 @@ __device__ __forceinline__ void a_tmem_ld64(unsigned addr, float* v) {
   for (int i = 0; i < 64; ++i) v[i] = __uint_as_float(r[i]);
 }
 // Two float32 values in one 64-bit register and the arithmetic that works on both at once (sm_100): the
-// softmax is bound by the instructions it issues and by the special-function unit (16 exponentials per
-// clock and multiprocessor), not by the tensor cores.
+// softmax is bound by the instructions it issues, not by the tensor cores.
 typedef unsigned long long a_f32x2;
 __device__ __forceinline__ a_f32x2 a_pack2(float lo, float hi) {
   a_f32x2 r;
@@ -220,30 +219,6 @@ __device__ __forceinline__ float a_max3(float a, float b, float c) {
   asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
   return d;
 }
-// 2^x for both halves of x on the FMA pipe: x = n + f with n = round(x) (the magic-number add leaves n in the
-// low mantissa bits of t), 2^f on [-0.5, 0.5] by a cubic whose relative error is below 7.5e-5 (P is rounded to
-// 8 bits of mantissa afterwards, and the same values go into the row's sum), and n added to the exponent bits.
-// x is clamped at -126 (a masked score is -infinity; 2^-126 is nothing against a row's largest term, which is 1
-// or more).  Every other pair of exponentials goes this way, the rest to the special-function unit, so that
-// both run side by side.
-__device__ __forceinline__ void a_exp2_pair_fma(a_f32x2 x, float& p0, float& p1) {
-  float x0, x1;
-  a_unpack2(x, x0, x1);
-  x = a_pack2(fmaxf(x0, -126.f), fmaxf(x1, -126.f));
-  const a_f32x2 magic = a_pack2(12582912.f, 12582912.f), minus_magic = a_pack2(-12582912.f, -12582912.f);
-  const a_f32x2 t = a_add2(x, magic);
-  const a_f32x2 n = a_add2(t, minus_magic);
-  const a_f32x2 f = a_fma2(n, a_pack2(-1.f, -1.f), x);
-  a_f32x2 p = a_fma2(f, a_pack2(0.055171654f, 0.055171654f), a_pack2(0.24261113f, 0.24261113f));
-  p = a_fma2(p, f, a_pack2(0.69326097f, 0.69326097f));
-  p = a_fma2(p, f, a_pack2(0.99992806f, 0.99992806f));
-  float t0, t1, q0, q1;
-  a_unpack2(t, t0, t1);
-  a_unpack2(p, q0, q1);
-  p0 = __int_as_float(__float_as_int(q0) + (__float_as_int(t0) << 23));
-  p1 = __int_as_float(__float_as_int(q1) + (__float_as_int(t1) << 23));
-}
-
 // 32 consecutive 32-bit columns of this thread's lane, written from registers
 __device__ __forceinline__ void a_tmem_st32(unsigned addr, const unsigned* r) {
   asm volatile(
@@ -536,23 +511,20 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_c
       if (moved && i == 0) l_run *= a_exp2(m_used - mx);  // nothing in O yet; the sink's share of the sum, if any
       if (moved) m_used = mx;
       const float shift = m_used > -INFINITY ? m_used : 0.f;  // a fully masked row stays at zero weight
-      // p = 2^(s * scale - shift), two columns per instruction; the pairs alternate between the special-function
-      // unit and the FMA pipe
+      // p = 2^(s * scale - shift), two columns per instruction, the exponentials on the special-function unit.  Every other
+      // pair's on the FMA pipe instead (a cubic, a dozen instructions a pair) was the slower form: two softmax warps a
+      // scheduler live by the length of their own instruction streams, with every pipe less than half busy.  8,192 tokens, 32
+      // heads: 567 us with half of the pairs on the FMA pipe, 534 with a quarter, 518 with none at head size 128; 482 and 472
+      // at 64; 2,048 tokens at 128 64.7 and 60.6.
       const a_f32x2 scale2 = a_pack2(a.scale_log2, a.scale_log2), shift2 = a_pack2(-shift, -shift);
       a_f32x2 sum2[2] = {a_pack2(0.f, 0.f), a_pack2(0.f, 0.f)};
       unsigned packed[MLL_PAGE / 2];
 #pragma unroll
       for (int c = 0; c < MLL_PAGE; c += 2) {
         const a_f32x2 x = a_fma2(a_pack2(s[c], s[c + 1]), scale2, shift2);
-        float p0, p1;
-        if ((c >> 1) & 1) {
-          a_exp2_pair_fma(x, p0, p1);
-        } else {
-          float x0, x1;
-          a_unpack2(x, x0, x1);
-          p0 = a_exp2(x0);
-          p1 = a_exp2(x1);
-        }
+        float x0, x1;
+        a_unpack2(x, x0, x1);
+        const float p0 = a_exp2(x0), p1 = a_exp2(x1);
         sum2[(c >> 2) & 1] = a_add2(sum2[(c >> 2) & 1], a_pack2(p0, p1));
         __nv_bfloat162 pair = __floats2bfloat162_rn(p0, p1);
         packed[c >> 1] = *reinterpret_cast<unsigned*>(&pair);
