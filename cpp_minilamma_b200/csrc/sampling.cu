@@ -585,6 +585,13 @@ constexpr int SC_CAND = 1024;
 // a pass).  As soon as no more than 1,024 keys are left at or above the digit's lower bound - with a few dozen
 // kept out of 128,256 that is after the first pass - they all go to block 0, which sorts them and draws among the
 // first k.  Only when more than 1,024 keys tie with the k-th does the exact rule need the counts of every block.
+//
+// In front of that, a bound: every block finds the j-th largest of its threads' largest keys, j = ceil(k / 8), by two digits
+// of 11 bits in its own shared memory; the blocks' smallest such key has k keys at or above it in the row, so nothing below it
+// can be kept, and as a rule few more than k reach it and the passes are not needed.  What a pass costs is the sum of eight
+// histograms of 2,048 bins over distributed shared memory, in every block, and its atomic additions to the few bins that a
+// vocabulary's logits crowd into.  64 rows of 128,256 logits, k = 40 (33 MB, 5 us at the copy peak): 102 us without the bound,
+// 42 us with it.
 template <int VPT>
 __global__ void __cluster_dims__(SC_CLUSTER, 1, 1) __launch_bounds__(SC_THREADS, (VPT <= 32 ? 2 : 1))
 sample_top_k_cluster_kernel(const float* __restrict__ logits, int vocab, int top_k, float temperature,
@@ -623,6 +630,64 @@ sample_top_k_cluster_kernel(const float* __restrict__ logits, int vocab, int top
   int remaining = top_k;     // its rank among the keys that share them
   int at_or_above = vocab;   // keys at or above the lower bound that the digits give
   int passes = 0;
+  unsigned bound = 0;        // no key below it is kept
+  {
+    unsigned largest = 0;
+#pragma unroll
+    for (int j = 0; j < VPT; ++j)
+      if (first + j < end) largest = max(largest, key[j]);
+    constexpr int PER = SC_BINS / SC_THREADS;
+    int wanted = (top_k + SC_CLUSTER - 1) / SC_CLUSTER;
+    if (tid == 0) sel_prefix = 0;
+    bool in = first < end;
+#pragma unroll
+    for (int digit = 0; digit < 2; ++digit) {  // two of 11 bits
+      const int shift = digit == 0 ? SC_BITS1 + SC_BITS2 : SC_BITS2;
+      int* bins = hist[digit];
+      for (int i = tid; i < SC_BINS; i += SC_THREADS) bins[i] = 0;
+      __syncthreads();
+      if (in) atomicAdd(&bins[(largest >> shift) & (SC_BINS - 1)], 1);
+      __syncthreads();
+      int c[PER], mine = 0;
+#pragma unroll
+      for (int i = 0; i < PER; ++i) mine += c[i] = bins[SC_BINS - 1 - (tid * PER + i)];
+      int total;
+      int above = block_exclusive_scan_int(mine, iscratch, &total);
+      if (above < wanted && wanted <= above + mine) {  // one thread, or none where a block has fewer maxima than wanted
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+          if (above < wanted && wanted <= above + c[i]) {
+            sel_prefix |= (unsigned)(SC_BINS - 1 - (tid * PER + i)) << shift;
+            sel_remaining = wanted - above;
+            above = wanted;  // done
+          } else {
+            above += c[i];
+          }
+        }
+      }
+      if (total < wanted) break;  // the same in every thread: the bound stays 0
+      __syncthreads();
+      wanted = sel_remaining;
+      in = in && (largest >> shift) == (sel_prefix >> shift);
+    }
+    cluster.sync();
+    bound = 0xffffffffu;
+#pragma unroll
+    for (int r = 0; r < SC_CLUSTER; ++r) bound = min(bound, *cluster.map_shared_rank(&sel_prefix, r));
+    int n = 0, total;
+#pragma unroll
+    for (int j = 0; j < VPT; ++j) n += first + j < end && key[j] >= bound;
+    block_exclusive_scan_int(n, iscratch, &total);
+    if (tid == 0) blk_greater = total;
+    cluster.sync();  // every block's count stands, and every block has read the bounds
+    int all = 0;
+#pragma unroll
+    for (int r = 0; r < SC_CLUSTER; ++r) all += *cluster.map_shared_rank(&blk_greater, r);
+    if (all <= SC_CAND) {  // few enough: the passes are not needed
+      at_or_above = all;
+      prefix = bound;
+    }
+  }
   for (; passes < 3 && at_or_above > SC_CAND; ++passes) {
     const int bits = passes == 0 ? SC_BITS0 : passes == 1 ? SC_BITS1 : SC_BITS2;
     const int shift = passes == 0 ? SC_BITS1 + SC_BITS2 : passes == 1 ? SC_BITS2 : 0;
@@ -633,7 +698,7 @@ sample_top_k_cluster_kernel(const float* __restrict__ logits, int vocab, int top
     __syncthreads();
 #pragma unroll
     for (int j = 0; j < VPT; ++j)
-      if (first + j < end && (key[j] & mask) == prefix) atomicAdd(&mine_hist[(key[j] >> shift) & (unsigned)(bins - 1)], 1);
+      if (first + j < end && key[j] >= bound && (key[j] & mask) == prefix) atomicAdd(&mine_hist[(key[j] >> shift) & (unsigned)(bins - 1)], 1);
     cluster.sync();  // every block's histogram stands (block-wide barrier included)
     // thread t sums bins[bins - 1 - per t - i], i < per, over the blocks: a scan over the threads then counts from the top
     const int per = bins / SC_THREADS;
