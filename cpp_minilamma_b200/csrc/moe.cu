@@ -59,24 +59,26 @@ __global__ void __launch_bounds__(512) moe_route_kernel(const T* __restrict__ h,
       const float* we = w + (size_t)e * width;
       float s[4] = {0.f, 0.f, 0.f, 0.f};  // four partial sums a lane
       if (vec) {
-        // 16 bytes of the weight row and four activations a lane and trip, eight trips' loads in flight together
-#pragma unroll 8
-        for (int i = lane * 4; i < width; i += 128) {
-          const float4 wv = *reinterpret_cast<const float4*>(we + i);
-          float hv[4];
-          if constexpr (sizeof(T) == 4) {
-            const float4 x = *reinterpret_cast<const float4*>(row + i);
-            hv[0] = x.x; hv[1] = x.y; hv[2] = x.z; hv[3] = x.w;
-          } else {
-            const uint2 x = *reinterpret_cast<const uint2*>(row + i);
-            const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x.x));
-            const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x.y));
-            hv[0] = lo.x; hv[1] = lo.y; hv[2] = hi.x; hv[3] = hi.y;
-          }
-          s[0] = fmaf(hv[0], wv.x, s[0]);
-          s[1] = fmaf(hv[1], wv.y, s[1]);
-          s[2] = fmaf(hv[2], wv.z, s[2]);
-          s[3] = fmaf(hv[3], wv.w, s[3]);
+        // 16 bytes of the weight row and four activations a lane and trip, all of a round (16 trips, of float32 rows 8) asked
+        // for before the first is used: left to itself the compiler keeps 40 registers and a few loads in flight
+        constexpr int TRIPS = sizeof(T) == 4 ? 8 : 16;
+        for (int i0 = lane * 4; i0 < width; i0 += TRIPS * 128) {
+          float4 wv[TRIPS];
+          RawWord<T, 4> hv[TRIPS];
+#pragma unroll
+          for (int u = 0; u < TRIPS; ++u)
+            if (i0 + u * 128 < width) {
+              wv[u] = __ldg(reinterpret_cast<const float4*>(we + i0 + u * 128));
+              hv[u].fetch(row + i0 + u * 128);
+            }
+#pragma unroll
+          for (int u = 0; u < TRIPS; ++u)
+            if (i0 + u * 128 < width) {
+              s[0] = fmaf(hv[u][0], wv[u].x, s[0]);
+              s[1] = fmaf(hv[u][1], wv[u].y, s[1]);
+              s[2] = fmaf(hv[u][2], wv[u].z, s[2]);
+              s[3] = fmaf(hv[u][3], wv[u].w, s[3]);
+            }
         }
       } else {
         for (int i = lane; i < width; i += 32) s[0] = fmaf(to_float(row[i]), we[i], s[0]);
@@ -139,7 +141,7 @@ __global__ void __launch_bounds__(512) moe_route_kernel(const T* __restrict__ h,
     }
     }
     __syncwarp();
-    float chosen_sum = 0.f;
+    float chosen_sum = 0.f, mine = 0.f;  // lane j keeps the j-th choice's score: no way through memory before the division
     for (int j = 0; j < top; ++j) {
       float best = -INFINITY;
       int at = 0x7fffffff;
@@ -156,17 +158,17 @@ __global__ void __launch_bounds__(512) moe_route_kernel(const T* __restrict__ h,
       if (at >= n_experts) at = j;
       const float sc = z[at];
       chosen_sum += sc;
+      if (lane == j) mine = sc;
       if (lane == 0) {
         chosen[(size_t)t * top + j] = at;
-        weight[(size_t)t * top + j] = sc;
         choice[at] = -INFINITY;
       }
       __syncwarp();
     }
-    if (lane < top) weight[(size_t)t * top + lane] = weight[(size_t)t * top + lane] / (chosen_sum + 1e-20f) * form.scale;
+    if (lane < top) weight[(size_t)t * top + lane] = mine / (chosen_sum + 1e-20f) * form.scale;
     return;
   }
-  float first = 0.f, total = 0.f;
+  float first = 0.f, total = 0.f, mine = 0.f;
   for (int j = 0; j < top; ++j) {
     float best = -INFINITY;
     int at = 0x7fffffff;
@@ -184,14 +186,14 @@ __global__ void __launch_bounds__(512) moe_route_kernel(const T* __restrict__ h,
     if (j == 0) first = best;
     const float p = expf(best - first);
     total += p;
+    if (lane == j) mine = p;
     if (lane == 0) {
       chosen[(size_t)t * top + j] = at;
-      weight[(size_t)t * top + j] = p;
       z[at] = -INFINITY;
     }
     __syncwarp();
   }
-  if (lane < top) weight[(size_t)t * top + lane] /= total;
+  if (lane < top) weight[(size_t)t * top + lane] = mine / total;
 }
 
 // ---- sort ----------------------------------------------------------------------------------------------------- //

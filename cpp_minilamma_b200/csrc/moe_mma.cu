@@ -1,6 +1,6 @@
 // The two products of the routed feed-forward (moe.cu) for steps with few rows per expert (single tokens), bfloat16:
 // mma.sync m16n8k16 with float32 accumulation on tiles of 16 rows of one expert - one MMA row tile - times 64 weight rows,
-// four warps side by side, operands through a four-stage cp.async ring (64 columns of k a stage), four such blocks a
+// four warps side by side, operands through a cp.async ring (four stages of 64 columns of k, gate_up three of 128), three or four such blocks a
 // multiprocessor (256 weight rows, one block a multiprocessor: the same time; two warps on 128 weight rows: a quarter
 // slower).  Such a step streams every touched expert's weights once for a handful of rows: memory bounds it.
 // Between 12 and 32 rows per expert on average a second instance has tiles of 32 rows (two MMA row tiles a warp): with
@@ -25,7 +25,12 @@ struct MoeMmaShape {
   static constexpr int BM = 16 * MT * WM, BN = 8 * NT * WN, LD = BK + 8, THREADS = 32 * WM * WN;
   static constexpr size_t SMEM = (size_t)STAGES * (BM + BN) * LD * sizeof(__nv_bfloat16);
 };
-using MoeMmaSmall = MoeMmaShape<1, 2, 1, 4, 64, 4>;  // 16 rows x 64 weight rows: single tokens
+// 16 rows x 64 weight rows: single tokens.  gate_up has three stages of 128 columns: whole 256-byte runs of a weight row a
+// stage and half the barriers, three blocks a multiprocessor (16 experts of 2,048 x 2,048, us, 4 stages of 64 / 3 of 128: one
+// token 25.7 / 19.8, 8 tokens 50.2 / 38.8, 24 tokens 52.2 / 52.9; of 3,584 x 4,096, 24 tokens: 172.6 / 152.7; 64 experts of
+// 1,408 x 2,048, 32 tokens: 123.2 / 112.5).  down, with half the blocks, keeps four blocks a multiprocessor, which hold a
+// batch's tiles at once (24 tokens: 27.5 / 34.0; of 2,048 x 3,584: 86.2 / 91.6).
+using MoeMmaSmall = MoeMmaShape<1, 2, 1, 4, 64, 4>;
 using MoeMmaMedium = MoeMmaShape<2, 2, 1, 4, 64, 4>;  // 32 rows x 64 weight rows: single tokens, 12 to 32 rows an expert
 
 // KIND 0: down; 1: gate_up (silu(gate) * up); 2: up alone with gelu (erf form) - the layout of `down`, rows gathered
@@ -182,7 +187,10 @@ int launch_moe_mma(const MoeProductArgs& a, int max_tiles, cudaStream_t stream) 
 
 template <int KIND>
 int launch_moe_mma_rows(const MoeProductArgs& a, int max_tiles, int tile_rows, cudaStream_t stream) {
-  if (tile_rows == MoeMmaSmall::BM) return launch_moe_mma<KIND, 1, 2, 1, 4, 64, 4>(a, max_tiles, stream);
+  if (tile_rows == MoeMmaSmall::BM) {
+    if constexpr (KIND == 1) return launch_moe_mma<KIND, 1, 2, 1, 4, 128, 3>(a, max_tiles, stream);
+    else return launch_moe_mma<KIND, 1, 2, 1, 4, 64, 4>(a, max_tiles, stream);
+  }
   if (tile_rows == MoeMmaMedium::BM) return launch_moe_mma<KIND, 2, 2, 1, 4, 64, 4>(a, max_tiles, stream);
   mll_set_error("moe (mma): tiles of %d rows (known: %d, %d, %d)", tile_rows, MoeMmaSmall::BM, MoeMmaMedium::BM, mll_moe_tc5_rows());
   return -1;
