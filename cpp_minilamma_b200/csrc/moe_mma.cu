@@ -27,7 +27,7 @@ struct MoeMmaShape {
 };
 // 16 rows x 64 weight rows: single tokens.  gate_up has three stages of 128 columns: whole 256-byte runs of a weight row a
 // stage and half the barriers, three blocks a multiprocessor (16 experts of 2,048 x 2,048, us, 4 stages of 64 / 3 of 128: one
-// token 25.7 / 19.8, 8 tokens 50.2 / 38.8, 24 tokens 52.2 / 52.9; of 3,584 x 4,096, 24 tokens: 172.6 / 152.7; 64 experts of
+// token 25.7 / 19.8, 8 tokens 50.2 / 38.8, 24 tokens 52.2 / 52.9 (in a decode step 56 / 57); of 3,584 x 4,096, 24 tokens: 172.6 / 152.7; 64 experts of
 // 1,408 x 2,048, 32 tokens: 123.2 / 112.5).  down, with half the blocks, keeps four blocks a multiprocessor, which hold a
 // batch's tiles at once (24 tokens: 27.5 / 34.0; of 2,048 x 3,584: 86.2 / 91.6).
 using MoeMmaSmall = MoeMmaShape<1, 2, 1, 4, 64, 4>;
