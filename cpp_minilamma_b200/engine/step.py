@@ -21,6 +21,7 @@ which assemble their logits in a tensor of their own.
 from __future__ import annotations
 
 from array import array
+from bisect import bisect_left
 from dataclasses import dataclass, field
 from typing import Any, Dict, Hashable, List, Optional, Sequence, Tuple
 
@@ -362,13 +363,15 @@ class Engine:
                 wants.append((w, out_row))
                 out_row += 1
             wants.sort()
-            done = 0
+            done = met = 0  # tokens and wanted places that the chunks so far hold
             while done < n:
                 if room == 0:
                     chunks.append([])
                     room = self.max_step_tokens
                 take = min(room, n - done)
-                want = [(place - done, row) for place, row in wants if done <= place < done + take]
+                upto = bisect_left(wants, (done + take,), met)
+                want = [(place - done, row) for place, row in wants[met:upto]]
+                met = upto
                 chunks[-1].append(_ChunkSeq(e.slot, values[done:done + take], starts[e.slot] + done, want))
                 done += take
                 room -= take

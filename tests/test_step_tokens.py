@@ -47,3 +47,33 @@ def test_chunks_and_wanted_places(kind):
     assert [t for chunk in chunks for seq in chunk for t in seq.tokens] == tokens
     assert [seq.start for chunk in chunks for seq in chunk] == [5, 25, 45]
     assert [seq.want for chunk in chunks for seq in chunk] == [[(0, 1), (0, 4), (19, 2)], [(0, 3)], [(9, 0)]]
+
+
+def test_wanted_places_are_walked_once():
+    """A prompt in many chunks with every place wanted: the planning compares each place with a few others, not with every chunk."""
+    compared = [0]
+
+    class Place(int):
+        def __lt__(self, other):
+            compared[0] += 1
+            return int(self) < int(other)
+
+        def __le__(self, other):
+            compared[0] += 1
+            return int(self) <= int(other)
+
+        def __gt__(self, other):
+            compared[0] += 1
+            return int(self) > int(other)
+
+        def __ge__(self, other):
+            compared[0] += 1
+            return int(self) >= int(other)
+
+        __eq__, __hash__ = int.__eq__, int.__hash__
+
+    n = 2000
+    chunks, n_want = _planner(20)._plan([StepEntry(0, [1] * n, [Place(i) for i in range(n)])])
+    assert n_want == n and len(chunks) == n // 20
+    assert [seq.want for chunk in chunks for seq in chunk] == [[(i, c * 20 + i) for i in range(20)] for c in range(n // 20)]
+    assert compared[0] < 20 * n
