@@ -190,6 +190,12 @@ moe_tc5_kernel(const __grid_constant__ CUtensorMap rows_map, const __grid_consta
         }
       }
     }
+    // The commits that free the last stages arrive in both blocks and nothing above waits for them: a block that left before
+    // could have one arrive in shared memory that is another's by then.  (A stage that was never filled passes at once.)
+    for (int left = 0; left < MT5_STAGES && ok; ++left, ++it) {
+      ok = g_mbar_wait(empty + 8 * (it % MT5_STAGES), ((it / MT5_STAGES) & 1) ^ 1, gave_up, a.error);
+      ok = __all_sync(0xffffffffu, ok);
+    }
   } else if (warp == 5) {
     // ---- products ---------------------------------------------------------------------------------------------- //
     if (rank == 0 && lane == 0) {

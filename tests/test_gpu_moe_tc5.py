@@ -59,3 +59,32 @@ def test_routed_products(counts, width, inter, form):
         want = weight.view(-1)[order[at]].double()[:, None] * (a @ d.T)
         slack = (a.abs() @ d.abs().T) * inter ** 0.5 * 2.0 ** -23
         assert ((y[order[at]].double() - want).abs() <= slack + 1e-6).all(), (e, form)
+
+
+@pytest.mark.parametrize("width", [8, 64, 5 * 64, 6 * 64, 6 * 64 + 8, 13 * 64])
+def test_back_to_back(width):
+    """Launches on each other's heels, with fewer, as many and more fills of the ring than it has stages: the pairs leave with
+    nothing on its way into their shared memory, so that every launch finds what the first found."""
+    from cpp_minilamma_b200.csrc import kernels as K
+    dev = torch.device("cuda:0")
+    gen = torch.Generator(device=dev).manual_seed(width)
+    draw = lambda *shape: torch.randn(shape, generator=gen, device=dev)
+    E, inter, n_pairs = 3, 256, 400
+    chosen = torch.randint(0, E, (n_pairs, 1), generator=gen, device=dev, dtype=torch.int32)
+    h, first = draw(n_pairs, width).to(torch.bfloat16), (0.2 * draw(E, 2 * inter, width)).to(torch.bfloat16)
+    down, weight = (0.2 * draw(E, inter, width)).to(torch.bfloat16), torch.rand((n_pairs, 1), generator=gen, device=dev)
+    rows = K.moe_tile_rows(True, 1 << 30, 1)
+    tiles = K.moe_max_tiles(n_pairs, E, rows)
+    ints = lambda n: torch.zeros(n, dtype=torch.int32, device=dev)
+    plan = K.MoePlan(ints(n_pairs), ints(E + 1), ints(tiles), ints(tiles), ints(1), rows, True)
+    K.moe_sort(chosen, plan, E)
+    act = torch.empty((40, n_pairs, inter), dtype=torch.bfloat16, device=dev)
+    y = torch.empty((40, n_pairs, inter), dtype=torch.float32, device=dev)
+    room = torch.empty_like(h)
+    for i in range(40):
+        K.moe_gate_up(h, first, act[i], plan, 1, rows=room)
+        K.moe_down(h, down, y[i], weight, plan, 1)  # any rows in the experts' order do
+    torch.cuda.synchronize()
+    assert K.take_device_error() == 0
+    assert (act == act[:1]).all() and (y == y[:1]).all()
+    assert torch.isfinite(y).all() and y.abs().max() > 0
