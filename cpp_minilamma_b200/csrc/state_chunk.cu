@@ -113,8 +113,8 @@ __global__ void __launch_bounds__(128, 3) state_chunk_inputs_kernel(ChunkArgs a)
     ch_copy16(k_s + dst, a.k + src, in);
   }
   cp_async_commit();
-  // the delta rule's first columns of values, on their way while the products run (rows past the run's end: the last row,
-  // which a beta of 0 takes out again)
+  // the delta rule's first columns of values, on their way while the products run (rows past the run's end: the last row
+  // again, which is not stored)
   float x[DELTA ? CH : 1];
   auto load_values = [&](int e) {
 #pragma unroll
@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(128, 3) state_chunk_inputs_kernel(ChunkArgs a)
       float* dst = value ? a.u + at * CH * dv + e : a.w + at * CH * d + e;
       const int ld = value ? dv : d;
 #pragma unroll
-      for (int i = 0; i < CH; ++i) dst[(size_t)i * ld] = x[i];
+      for (int i = 0; i < CH; ++i) dst[(size_t)i * ld] = i < n ? x[i] : 0.f;
     }
   }
 }
@@ -359,7 +359,7 @@ __global__ void __launch_bounds__(128, 3) state_chunk_channel_inputs_kernel(Chun
   for (int col = tid; col < dv + d; col += 128) {
     const bool value = col < dv;
     const int e = value ? col : col - dv;
-    if (value) {  // rows past the run's end: the last row, times a beta of 0
+    if (value) {  // rows past the run's end: the last row again, which is not stored
 #pragma unroll
       for (int i = 0; i < CH; ++i) x[i] = a.v[((tok0 + min(i, n - 1)) * H + h) * dv + e];
 #pragma unroll
@@ -376,7 +376,7 @@ __global__ void __launch_bounds__(128, 3) state_chunk_channel_inputs_kernel(Chun
     float* dst = value ? a.u + at * CH * dv + e : a.w + at * CH * d + e;
     const int ld = value ? dv : d;
 #pragma unroll
-    for (int i = 0; i < CH; ++i) dst[(size_t)i * ld] = x[i];
+    for (int i = 0; i < CH; ++i) dst[(size_t)i * ld] = i < n ? x[i] : 0.f;
   }
 }
 
@@ -390,6 +390,27 @@ __device__ __forceinline__ void ch_step(float (&acc)[R][4], const float4 (&m)[4]
     acc[i][1] = fmaf(x.x, m[0].y, fmaf(x.y, m[1].y, fmaf(x.z, m[2].y, fmaf(x.w, m[3].y, acc[i][1]))));
     acc[i][2] = fmaf(x.x, m[0].z, fmaf(x.y, m[1].z, fmaf(x.z, m[2].z, fmaf(x.w, m[3].z, acc[i][2]))));
     acc[i][3] = fmaf(x.x, m[0].w, fmaf(x.y, m[1].w, fmaf(x.z, m[2].w, fmaf(x.w, m[3].w, acc[i][3]))));
+  }
+}
+
+// The same where row i of the left matrix is P's row `row0 + i * rows_apart` and the word its columns 4 wd .. + 3: places right of
+// the diagonal are left out, not multiplied by P's zeros there, so that a later token's infinity or not-a-number stays out of
+// the earlier tokens of its run.
+template <int R>
+__device__ __forceinline__ void ch_step_lower(float (&acc)[R][4], const float4 (&m)[4], const float* row, int row_stride, int row0,
+                                              int rows_apart, int wd) {
+#pragma unroll
+  for (int i = 0; i < R; ++i) {
+    const float4 x = *reinterpret_cast<const float4*>(row + i * row_stride);
+    const float xs[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+    for (int e = 3; e >= 0; --e)
+      if (4 * wd + e <= row0 + i * rows_apart) {
+        acc[i][0] = fmaf(xs[e], m[e].x, acc[i][0]);
+        acc[i][1] = fmaf(xs[e], m[e].y, acc[i][1]);
+        acc[i][2] = fmaf(xs[e], m[e].z, acc[i][2]);
+        acc[i][3] = fmaf(xs[e], m[e].w, acc[i][3]);
+      }
   }
 }
 
@@ -539,17 +560,18 @@ __global__ void __launch_bounds__(128) state_chunk_outputs_kernel(ChunkArgs a) {
   for (int i = 0; i < 8; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j) lo[i][j] = hi[i][j] = 0.f;
-  auto word = [&](const float* rows, int row_stride, const float* m_s, int wd) {
-    float4 m[4];
+  auto fetch = [&](float4 (&m)[4], const float* m_s, int wd, int half) {
 #pragma unroll
-    for (int e = 0; e < 4; ++e) m[e] = *reinterpret_cast<const float4*>(m_s + (4 * wd + e) * CH_WIDE + cg * 4);
-    ch_step<8>(lo, m, rows + rg * row_stride + wd * 4, 4 * row_stride);
-#pragma unroll
-    for (int e = 0; e < 4; ++e) m[e] = *reinterpret_cast<const float4*>(m_s + (4 * wd + e) * CH_WIDE + 32 + cg * 4);
-    ch_step<8>(hi, m, rows + rg * row_stride + wd * 4, 4 * row_stride);
+    for (int e = 0; e < 4; ++e) m[e] = *reinterpret_cast<const float4*>(m_s + (4 * wd + e) * CH_WIDE + half * 32 + cg * 4);
   };
 #pragma unroll 2
-  for (int wd = warp; wd < WORDS; wd += 4) word(sm + L::Q, DP, sm + L::S, wd);
+  for (int wd = warp; wd < WORDS; wd += 4) {
+    float4 m[4];
+    fetch(m, sm + L::S, wd, 0);
+    ch_step<8>(lo, m, sm + L::Q + rg * DP + wd * 4, 4 * DP);
+    fetch(m, sm + L::S, wd, 1);
+    ch_step<8>(hi, m, sm + L::Q + rg * DP + wd * 4, 4 * DP);
+  }
 #pragma unroll
   for (int i = 0; i < 8; ++i)
 #pragma unroll
@@ -558,7 +580,13 @@ __global__ void __launch_bounds__(128) state_chunk_outputs_kernel(ChunkArgs a) {
       hi[i][j] *= grown[i];
     }
 #pragma unroll
-  for (int wd = warp; wd < CH / 4; wd += 4) word(sm + L::P, CH, sm + L::V, wd);
+  for (int wd = warp; wd < CH / 4; wd += 4) {
+    float4 m[4];
+    fetch(m, sm + L::V, wd, 0);
+    ch_step_lower<8>(lo, m, sm + L::P + rg * CH + wd * 4, 4 * CH, rg, 4, wd);
+    fetch(m, sm + L::V, wd, 1);
+    ch_step_lower<8>(hi, m, sm + L::P + rg * CH + wd * 4, 4 * CH, rg, 4, wd);
+  }
   __syncthreads();
   float* part = sm + L::S + warp * CH * CH_WIDE;
 #pragma unroll
@@ -750,7 +778,7 @@ __global__ void __launch_bounds__(128, 2) state_chunk_scan_kernel(ChunkArgs a) {
       float4 m[4];
 #pragma unroll
       for (int e = 0; e < 4; ++e) m[e] = *reinterpret_cast<const float4*>(sm + L::X + ch_place<LD>(4 * wd + e, cg));
-      ch_step<4>(acc, m, sm + L::P + rg * CH + wd * 4, 8 * CH);
+      ch_step_lower<4>(acc, m, sm + L::P + rg * CH + wd * 4, 8 * CH, rg, 8, wd);
     }
     {
       const float4 o = ch_reduce(acc, kg);

@@ -78,3 +78,39 @@ def test_refused():
     i = torch.zeros(1, dtype=torch.int32, device=DEV)
     with pytest.raises(K.KernelError):  # a decay per channel without the delta rule
         K.state_chunks(z(4, 8), z(4, 8), z(4, 8), z(1, 1, 8, 8), z(4, 8), z(99999), i, i, i, i, i, i, 1, 1, 1, 8, 8, channel_decay=z(4, 8))
+
+
+@pytest.mark.parametrize("form", ["head", "token", "delta_head", "delta"])
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_later_tokens_stay_out_of_earlier_ones(form, bad):
+    """A value that is not finite reaches its own token and those behind it, as token by token: not the earlier tokens of its
+    run, nor another head or sequence; and where nothing follows it, the state is infinite where it is token by token."""
+    from cpp_minilamma_b200.csrc import kernels as K
+    H, d, dv, lens, at = 2, 64, 36, [83, 40], [43, 83 + 39]  # inside a block of 8 of the second run; the last token of all
+    gen = torch.Generator().manual_seed(7)
+    T, n_seqs = sum(lens), len(lens)
+    draw = lambda *shape: torch.randn(shape, generator=gen).to(DEV)
+    ints = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    q, k, v = draw(T, H * d) / d ** 0.5, draw(T, H * d) / d ** 0.5, draw(T, H * dv)
+    for t in at:
+        v[t, 5] = bad  # head 0
+    unit = lambda *shape: 0.5 + 0.5 * torch.rand(shape, generator=gen).to(DEV)
+    channel = unit(T, H * d) if form == "delta" else None
+    token = unit(T, H) if form in ("token", "delta_head") else None
+    head = unit(H) if form == "head" else None
+    beta = unit(T, H) if form in ("delta", "delta_head") else None
+    runs = [(i, row0) for i, n in enumerate(lens) for row0 in range(0, n, K.STATE_RUN)]
+    first = [next(j for j, (s, _) in enumerate(runs) if s == i) for i in range(n_seqs)]
+    state = draw(n_seqs, H, d, dv)
+    walked, out, walked_out = state.clone(), torch.empty((T, H * dv), device=DEV), torch.empty((T, H * dv), device=DEV)
+    lists = (ints([0, 1]), ints([0, lens[0]]), ints(lens), n_seqs, H, H, d, dv)
+    K.state_scan(q, k, v, channel, beta, head, walked, walked_out, *lists, token_decay=token)
+    scratch = torch.full((K.state_chunks_scratch(len(runs), H, d, dv, beta is not None, channel is not None),), float("nan"), device=DEV)
+    K.state_chunks(q, k, v, state, out, scratch, ints([s for s, _ in runs]), ints([r for _, r in runs]), ints(first), *lists,
+                   head_decay=head, token_decay=token, beta=beta, channel_decay=channel)
+    ok = torch.isfinite(walked_out)
+    assert not ok.all() and ok[:at[0]].all() and ok[83:at[1]].all()
+    assert torch.equal(torch.isfinite(out), ok)
+    assert (out - walked_out)[ok].abs().max() <= 4e-5 * walked_out[ok].abs().max()  # two float32 sums, 2e-5 each
+    assert torch.equal(torch.isfinite(state), torch.isfinite(walked))
+    assert torch.equal(torch.isnan(state[1]), torch.isnan(walked[1]))
