@@ -218,8 +218,22 @@ struct ChannelInputsSmem {  // offsets in floats
   static constexpr size_t BYTES = (size_t)FLOATS * sizeof(float);
 };
 
+// sum + error <- sum + error + x, where `error` takes what the addition to `sum` rounds off (Knuth's sum of two)
+__device__ __forceinline__ void ch_add(float& sum, float& error, float x) {
+  const float next = sum + x, part = next - sum;
+  error += (sum - (next - part)) + (x - part);
+  sum = next;
+}
+__device__ __forceinline__ float ch_dot(const float4& x, const float4& y) {
+  return fmaf(x.x, y.x, fmaf(x.y, y.y, fmaf(x.z, y.z, x.w * y.w)));
+}
+
 // grid (runs, H), 128 threads.  Rows of DP floats lie in shared memory with their 16-byte words XORed as above.  Bound by
 // shared memory: a word of a row of q, one of k and one of a column feed 8 products.
+// P stands between every token and its run's other tokens, where token by token a single sum over the channels did: summed up
+// in one float32 chain over the channels it made the outputs' error against 64 bits 1.1 to 1.6 times the token-by-token
+// scan's.  So the sums over the words of four channels keep what their additions round off, and the products of decays from
+// the run's ends are formed in 64 bits.
 template <int DP>
 __global__ void __launch_bounds__(128, 3) state_chunk_channel_inputs_kernel(ChunkArgs a) {
   using L = ChannelInputsSmem<DP>;
@@ -254,17 +268,17 @@ __global__ void __launch_bounds__(128, 3) state_chunk_channel_inputs_kernel(Chun
   if (tid < d) {
     float* qd = a.qd + at * CH * d + tid;
     float* kd = a.kd + at * CH * d + tid;
-    float grown = 1.f, left = 1.f;
+    double grown = 1.0, left = 1.0;
 #pragma unroll 8
     for (int i = 0; i < CH; ++i) {
-      grown *= g_s[place(i, tid)];
-      qd[(size_t)i * d] = grown * q_s[place(i, tid)];
+      grown *= (double)g_s[place(i, tid)];
+      qd[(size_t)i * d] = (float)grown * q_s[place(i, tid)];
     }
-    a.factors[at * d + tid] = grown;
+    a.factors[at * d + tid] = (float)grown;
 #pragma unroll 8
     for (int j = CH - 1; j >= 0; --j) {
-      kd[(size_t)j * d] = left * k_s[place(j, tid)];
-      left *= g_s[place(j, tid)];
+      kd[(size_t)j * d] = (float)left * k_s[place(j, tid)];
+      left *= (double)g_s[place(j, tid)];
     }
   }
 
@@ -272,9 +286,9 @@ __global__ void __launch_bounds__(128, 3) state_chunk_channel_inputs_kernel(Chun
   // k_j g_(j+1) .. g_i from row to row.
   {
     const int first = warp * CH_SUB, j = lane & 7, part = lane >> 3;
-    float p[CH_SUB], w[CH_SUB];
+    float p[CH_SUB], w[CH_SUB], p_err[CH_SUB], w_err[CH_SUB];
 #pragma unroll
-    for (int i = 0; i < CH_SUB; ++i) p[i] = w[i] = 0.f;
+    for (int i = 0; i < CH_SUB; ++i) p[i] = w[i] = p_err[i] = w_err[i] = 0.f;
 #pragma unroll 1
     for (int wd = part; wd < WORDS; wd += 4) {
       float4 c = *reinterpret_cast<const float4*>(k_s + (first + j) * DP + ((wd ^ j) << 2));
@@ -284,20 +298,23 @@ __global__ void __launch_bounds__(128, 3) state_chunk_channel_inputs_kernel(Chun
         const float4 q4 = *reinterpret_cast<const float4*>(q_s + word), k4 = *reinterpret_cast<const float4*>(k_s + word);
         const float4 g4 = *reinterpret_cast<const float4*>(g_s + word);
         if (i > j) { c.x *= g4.x; c.y *= g4.y; c.z *= g4.z; c.w *= g4.w; }
-        p[i] = fmaf(q4.x, c.x, fmaf(q4.y, c.y, fmaf(q4.z, c.z, fmaf(q4.w, c.w, p[i]))));
-        w[i] = fmaf(k4.x, c.x, fmaf(k4.y, c.y, fmaf(k4.z, c.z, fmaf(k4.w, c.w, w[i]))));
+        ch_add(p[i], p_err[i], ch_dot(q4, c));
+        ch_add(w[i], w_err[i], ch_dot(k4, c));
       }
     }
 #pragma unroll
     for (int i = 0; i < CH_SUB; ++i) {
 #pragma unroll
       for (int o = 8; o < 32; o <<= 1) {
-        p[i] += __shfl_xor_sync(0xffffffffu, p[i], o);
-        w[i] += __shfl_xor_sync(0xffffffffu, w[i], o);
+        const float pe = __shfl_xor_sync(0xffffffffu, p_err[i], o), we = __shfl_xor_sync(0xffffffffu, w_err[i], o);
+        ch_add(p[i], p_err[i], __shfl_xor_sync(0xffffffffu, p[i], o));
+        ch_add(w[i], w_err[i], __shfl_xor_sync(0xffffffffu, w[i], o));
+        p_err[i] += pe;
+        w_err[i] += we;
       }
       if (part == (i & 3)) {  // four lanes hold the sums: each writes its share of the rows
-        a.p[(at * CH + first + i) * CH + first + j] = i >= j ? p[i] : 0.f;
-        if (i > j) a_s[(first + i) * A_LD + first + j] = beta_s[first + i] * w[i];
+        a.p[(at * CH + first + i) * CH + first + j] = i >= j ? p[i] + p_err[i] : 0.f;
+        if (i > j) a_s[(first + i) * A_LD + first + j] = beta_s[first + i] * (w[i] + w_err[i]);
       }
     }
   }
@@ -331,26 +348,26 @@ __global__ void __launch_bounds__(128, 3) state_chunk_channel_inputs_kernel(Chun
     const int i = tid & 7, j0 = tid >> 3;  // row i, columns j0 and j0 + 16
     if (j0 < first) {
       const bool two = j0 + 16 < first;
-      float p0 = 0.f, p1 = 0.f, w0 = 0.f, w1 = 0.f;
+      float p0 = 0.f, p1 = 0.f, w0 = 0.f, w1 = 0.f, p0_err = 0.f, p1_err = 0.f, w0_err = 0.f, w1_err = 0.f;
 #pragma unroll 4
       for (int wd = 0; wd < WORDS; ++wd) {
         const float4 q4 = *reinterpret_cast<const float4*>(r_s + i * DP + ((wd ^ i) << 2));
         const float4 k4 = *reinterpret_cast<const float4*>(r_s + (CH_SUB + i) * DP + ((wd ^ i) << 2));
         const float4 c = *reinterpret_cast<const float4*>(c_s + j0 * DP + ((wd ^ (j0 & 7)) << 2));
-        p0 = fmaf(q4.x, c.x, fmaf(q4.y, c.y, fmaf(q4.z, c.z, fmaf(q4.w, c.w, p0))));
-        w0 = fmaf(k4.x, c.x, fmaf(k4.y, c.y, fmaf(k4.z, c.z, fmaf(k4.w, c.w, w0))));
+        ch_add(p0, p0_err, ch_dot(q4, c));
+        ch_add(w0, w0_err, ch_dot(k4, c));
         if (two) {
           const float4 c2 = *reinterpret_cast<const float4*>(c_s + (j0 + 16) * DP + ((wd ^ (j0 & 7)) << 2));
-          p1 = fmaf(q4.x, c2.x, fmaf(q4.y, c2.y, fmaf(q4.z, c2.z, fmaf(q4.w, c2.w, p1))));
-          w1 = fmaf(k4.x, c2.x, fmaf(k4.y, c2.y, fmaf(k4.z, c2.z, fmaf(k4.w, c2.w, w1))));
+          ch_add(p1, p1_err, ch_dot(q4, c2));
+          ch_add(w1, w1_err, ch_dot(k4, c2));
         }
       }
       const int row = first + i;
-      a.p[(at * CH + row) * CH + j0] = p0;
-      a_s[row * A_LD + j0] = beta_s[row] * w0;
+      a.p[(at * CH + row) * CH + j0] = p0 + p0_err;
+      a_s[row * A_LD + j0] = beta_s[row] * (w0 + w0_err);
       if (two) {
-        a.p[(at * CH + row) * CH + j0 + 16] = p1;
-        a_s[row * A_LD + j0 + 16] = beta_s[row] * w1;
+        a.p[(at * CH + row) * CH + j0 + 16] = p1 + p1_err;
+        a_s[row * A_LD + j0 + 16] = beta_s[row] * (w1 + w1_err);
       }
     }
   }
@@ -365,11 +382,11 @@ __global__ void __launch_bounds__(128, 3) state_chunk_channel_inputs_kernel(Chun
 #pragma unroll
       for (int i = 0; i < CH; ++i) x[i] *= beta_s[i];
     } else {
-      float grown = 1.f;
+      double grown = 1.0;
 #pragma unroll
       for (int i = 0; i < CH; ++i) {
-        grown *= g_s[place(i, e)];
-        x[i] = beta_s[i] * grown * k_s[place(i, e)];
+        grown *= (double)g_s[place(i, e)];
+        x[i] = beta_s[i] * (float)grown * k_s[place(i, e)];
       }
     }
     ch_substitute(x, a_s);
