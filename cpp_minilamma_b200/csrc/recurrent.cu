@@ -760,8 +760,19 @@ int launch_scan(const ScanArgs& args, int n_seqs, cudaStream_t stream) {
 // and 24.9; one sequence 4.0 and 3.9.
 constexpr int STEP_COLS = 64, STEP_GROUPS = 16;  // columns a block; groups of rows
 
+__device__ __forceinline__ float step_sum(const float (&x)[STEP_GROUPS / 2]) {
+  static_assert(STEP_GROUPS == 16, "eight sums");
+  return ((x[0] + x[1]) + (x[2] + x[3])) + ((x[4] + x[5]) + (x[6] + x[7]));
+}
+
+// Blocks a multiprocessor that the register allocation aims at: with fewer the loads in flight no longer fill the memory's pipe.
+constexpr int step_blocks(int rows, int mode) {
+  const bool delta = mode == 1 || mode == 4;
+  return rows <= 2 ? (delta ? 4 : 6) : rows <= 4 ? (delta ? 3 : 4) : rows <= 8 ? (delta || mode == 2 ? 2 : 3) : 1;
+}
+
 template <int ROWS, int MODE>
-__global__ void __launch_bounds__(256) state_step_kernel(ScanArgs a) {
+__global__ void __launch_bounds__(256, step_blocks(ROWS, MODE)) state_step_kernel(ScanArgs a) {
   constexpr bool CHANNEL = MODE == 1 || MODE == 2, DELTA = MODE == 1 || MODE == 4;
   constexpr int SUMS = DELTA ? 2 : 1;  // S'^T q, and S'^T k
   __shared__ __align__(16) float part[SUMS][STEP_GROUPS / 2][STEP_COLS];
@@ -785,23 +796,44 @@ __global__ void __launch_bounds__(256) state_step_kernel(ScanArgs a) {
     if (col < dv) v = *reinterpret_cast<const float4*>(a.v + ((size_t)t * H + h) * dv + col);
     const float beta = DELTA ? a.beta[(size_t)t * H + h] : 1.f;
     const float decay = MODE == 0 ? a.head_decay[h] : MODE == 3 ? a.beta[(size_t)t * H + h] : MODE == 4 ? a.g[(size_t)t * H + h] : 1.f;
+    // no chain of additions is longer than four: with more rows they are taken two by two
     float kv[ROWS], o[4] = {0.f, 0.f, 0.f, 0.f}, c[4] = {0.f, 0.f, 0.f, 0.f}, kq = 0.f;
+    float held[5];  // the first of two rows' products: with q, and k with q
+    float held_k[4];
 #pragma unroll
     for (int i = 0; i < ROWS; ++i) {
       const bool in = row_first + i < d;
       const float qi = in ? q[i] : 0.f, gi = CHANNEL ? (in ? g[i] : 1.f) : decay;
       kv[i] = in ? k[i] : 0.f;
-      s[i].x *= gi; s[i].y *= gi; s[i].z *= gi; s[i].w *= gi;
-      if (DELTA) {
-        c[0] = fmaf(s[i].x, kv[i], c[0]); c[1] = fmaf(s[i].y, kv[i], c[1]);
-        c[2] = fmaf(s[i].z, kv[i], c[2]); c[3] = fmaf(s[i].w, kv[i], c[3]);
-        kq = fmaf(kv[i], qi, kq);
-      } else {
-        s[i].x = fmaf(kv[i], v.x, s[i].x); s[i].y = fmaf(kv[i], v.y, s[i].y);
-        s[i].z = fmaf(kv[i], v.z, s[i].z); s[i].w = fmaf(kv[i], v.w, s[i].w);
+      if (MODE == 1) {
+        s[i].x *= gi; s[i].y *= gi; s[i].z *= gi; s[i].w *= gi;
+      } else if (!DELTA) {  // of the two products the write's is rounded by itself: it is the smaller one once a state has grown
+        s[i].x = fmaf(gi, s[i].x, kv[i] * v.x); s[i].y = fmaf(gi, s[i].y, kv[i] * v.y);
+        s[i].z = fmaf(gi, s[i].z, kv[i] * v.z); s[i].w = fmaf(gi, s[i].w, kv[i] * v.w);
       }
-      o[0] = fmaf(s[i].x, qi, o[0]); o[1] = fmaf(s[i].y, qi, o[1]);
-      o[2] = fmaf(s[i].z, qi, o[2]); o[3] = fmaf(s[i].w, qi, o[3]);
+      if constexpr (ROWS <= 4) {
+        if (DELTA) {
+          c[0] = fmaf(s[i].x, kv[i], c[0]); c[1] = fmaf(s[i].y, kv[i], c[1]);
+          c[2] = fmaf(s[i].z, kv[i], c[2]); c[3] = fmaf(s[i].w, kv[i], c[3]);
+          kq = fmaf(kv[i], qi, kq);
+        }
+        o[0] = fmaf(s[i].x, qi, o[0]); o[1] = fmaf(s[i].y, qi, o[1]);
+        o[2] = fmaf(s[i].z, qi, o[2]); o[3] = fmaf(s[i].w, qi, o[3]);
+      } else if (i % 2 == 0) {
+        if (DELTA) {
+          held_k[0] = s[i].x * kv[i]; held_k[1] = s[i].y * kv[i]; held_k[2] = s[i].z * kv[i]; held_k[3] = s[i].w * kv[i];
+          held[4] = kv[i] * qi;
+        }
+        held[0] = s[i].x * qi; held[1] = s[i].y * qi; held[2] = s[i].z * qi; held[3] = s[i].w * qi;
+      } else {
+        if (DELTA) {
+          c[0] += fmaf(s[i].x, kv[i], held_k[0]); c[1] += fmaf(s[i].y, kv[i], held_k[1]);
+          c[2] += fmaf(s[i].z, kv[i], held_k[2]); c[3] += fmaf(s[i].w, kv[i], held_k[3]);
+          kq += fmaf(kv[i], qi, held[4]);
+        }
+        o[0] += fmaf(s[i].x, qi, held[0]); o[1] += fmaf(s[i].y, qi, held[1]);
+        o[2] += fmaf(s[i].z, qi, held[2]); o[3] += fmaf(s[i].w, qi, held[3]);
+      }
     }
     // a warp holds two groups of rows
 #pragma unroll
@@ -818,27 +850,31 @@ __global__ void __launch_bounds__(256) state_step_kernel(ScanArgs a) {
     __syncthreads();
     if (tid < SUMS * STEP_COLS) {
       const float* p = &part[tid / STEP_COLS][0][tid % STEP_COLS];
-      float sum = p[0];
+      float sum[STEP_GROUPS / 2];
 #pragma unroll
-      for (int w = 1; w < STEP_GROUPS / 2; ++w) sum += p[w * STEP_COLS];
-      total[tid / STEP_COLS][tid % STEP_COLS] = sum;
+      for (int w = 0; w < STEP_GROUPS / 2; ++w) sum[w] = p[w * STEP_COLS];
+      total[tid / STEP_COLS][tid % STEP_COLS] = step_sum(sum);
     }
     __syncthreads();
     float y[4];
     load_floats<float, 4>(&total[0][cg * 4], y);
     if constexpr (DELTA) {
-      float x[4], all = kq_part[0];
+      float x[4], kqs[STEP_GROUPS / 2];
       load_floats<float, 4>(&total[SUMS - 1][cg * 4], x);
 #pragma unroll
-      for (int w = 1; w < STEP_GROUPS / 2; ++w) all += kq_part[w];
-      const float u[4] = {beta * (v.x - x[0]), beta * (v.y - x[1]), beta * (v.z - x[2]), beta * (v.w - x[3])};
+      for (int w = 0; w < STEP_GROUPS / 2; ++w) kqs[w] = kq_part[w];
+      const float all = step_sum(kqs);
+      // mode 4: one decay for all rows, which meets their sums instead of every row
+      const float gs = MODE == 4 ? decay : 1.f;
+      const float u[4] = {beta * fmaf(-gs, x[0], v.x), beta * fmaf(-gs, x[1], v.y), beta * fmaf(-gs, x[2], v.z), beta * fmaf(-gs, x[3], v.w)};
 #pragma unroll
       for (int i = 0; i < ROWS; ++i) {
+        if (MODE == 4) { s[i].x *= gs; s[i].y *= gs; s[i].z *= gs; s[i].w *= gs; }
         s[i].x = fmaf(kv[i], u[0], s[i].x); s[i].y = fmaf(kv[i], u[1], s[i].y);
         s[i].z = fmaf(kv[i], u[2], s[i].z); s[i].w = fmaf(kv[i], u[3], s[i].w);
       }
 #pragma unroll
-      for (int j = 0; j < 4; ++j) y[j] = fmaf(u[j], all, y[j]);
+      for (int j = 0; j < 4; ++j) y[j] = MODE == 4 ? fmaf(gs, y[j], u[j] * all) : fmaf(u[j], all, y[j]);
     }
     if (rg == 0 && col < dv) store_floats<float, 4>(a.out + ((size_t)t * H + h) * dv + col, y);
     if (t + 1 < row0 + n_tok) __syncthreads();  // the next token's sums take the same places
