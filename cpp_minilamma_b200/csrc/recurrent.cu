@@ -897,10 +897,30 @@ int launch_step(const ScanArgs& a, int n_seqs, cudaStream_t stream) {
   return 0;
 }
 
-// How a column of S is spread over lanes.  With enough columns to fill the device (a decode step of a batch) a
-// thread holds a whole column (keys up to 64; two lanes up to 128, four up to 256: 64 rows are what a thread's
-// registers hold): a warp then reads and writes 128, 64 or 32 consecutive bytes of a row of the state.  Measured
-// on 128 sequences of 16 heads of 128 x 128 (134 MB of state in and out): 64 rows a lane 112 us (2.4 TB/s); 32
+// Where the step kernel is not the faster one (us, the scan below / the step kernel):
+//   * states of fewer than 32 value columns leave half of a block and more without work: with the delta rule from 65 rows (8,192
+//     heads of 128 x 16: 57 / 76), and from 33 rows while they do not fill the scan's columns (512 heads of 64 x 16: 4.0 / 4.4; 4,096:
+//     24.5 / 21.4); without it from 65 rows, many waves of blocks (4,096 heads of 128 x 16, a decay per channel 26 / 32; 2,048 21 / 17)
+//   * a handful of blocks on an idle device: the delta rule's sums over a block's rows go through shared memory twice where the
+//     scan's eight lanes shuffle (one sequence of 8 heads of 128 x 128: 3.1 / 3.4, of 2 heads of 256 x 256: 3.8 / 4.6; from 32
+//     blocks on 3.6 / 3.3).  With one decay per head that is so beyond 192 rows only.  (From 129 to 192 rows the scan is padded to
+//     256: 5.9 / 4.2.)
+template <int MODE>
+bool step_pays(const ScanArgs& a, int n_seqs) {
+  constexpr bool DELTA = MODE == 1 || MODE == 4;
+  const long long blocks = (long long)((a.dv + STEP_COLS - 1) / STEP_COLS) * a.n_heads * n_seqs;
+  if (a.dv < 32 && a.d > 32) {
+    const long long sm = mll_sm_count();
+    if (DELTA && (a.d > 64 || (blocks > 2 * sm && blocks * a.dv < 256 * sm))) return false;
+    if (!DELTA && a.d > 64 && blocks > 16 * sm) return false;
+  }
+  return blocks >= 32 || !((MODE == 1 && a.d > 64 && a.d <= 128) || (DELTA && a.d > 192));
+}
+
+// How a column of S is spread over lanes.  With enough columns to fill the device (many sequences: portions of a few tokens
+// each, or single tokens that the step kernel does not take) a thread holds a whole column (keys up to 64; two lanes up to
+// 128, four up to 256: 64 rows are what a thread's registers hold): a warp then reads and writes 128, 64 or 32 consecutive bytes of a row of the state.  Measured
+// on single tokens of 128 sequences of 16 heads of 128 x 128 (134 MB of state in and out), before there was a step kernel: 64 rows a lane 112 us (2.4 TB/s); 32
 // rows a lane and four lanes a column, with twice the resident blocks, 142 us.  That layout starts at 256 columns a
 // multiprocessor (64 sequences of 8 heads of 128 value columns: 51 us with eight lanes a column, whose 16-byte pieces
 // of a row use half of every sector, 29 us with two).  Otherwise (a prompt of one or a few sequences) eight lanes
@@ -910,7 +930,8 @@ template <int MODE>
 int dispatch_scan(const ScanArgs& a, int n_seqs, int n_tokens, cudaStream_t stream) {
   // A token a sequence, on average, is a decode step: whole rows of the state instead of columns (value columns in words of
   // 16 bytes; a state of more than 256 rows would take more registers than a thread has).
-  if (n_tokens <= n_seqs && a.d <= 256 && a.dv % 4 == 0 && ((uintptr_t)a.state | (uintptr_t)a.v | (uintptr_t)a.out) % 16 == 0)
+  if (n_tokens <= n_seqs && a.d <= 256 && a.dv % 4 == 0 && ((uintptr_t)a.state | (uintptr_t)a.v | (uintptr_t)a.out) % 16 == 0 &&
+      step_pays<MODE>(a, n_seqs))
     return launch_step<MODE>(a, n_seqs, stream);
   const int d = a.d;
   const bool many = (long long)n_seqs * a.n_heads * a.dv >= (long long)mll_sm_count() * 256;

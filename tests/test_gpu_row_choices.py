@@ -1,0 +1,15 @@
+"""Kernels that a rule on sizes picks between, at sizes on either side of its lines that the tests of the kernels themselves do not
+reach: the checks are theirs."""
+import pytest
+import torch
+
+import test_gpu_state_step as state
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("form", ["head", "delta", "channel", "token", "delta_head"])
+@pytest.mark.parametrize("n,H,d,dv", [(1, 8, 128, 128), (2, 8, 128, 128), (4, 2, 256, 256), (1, 2, 256, 256), (1, 4, 192, 128), (3, 2, 33, 16),
+                                      (2, 2, 32, 16), (600, 2, 72, 16), (300, 2, 72, 16), (70, 1, 64, 28)])
+def test_single_tokens(form, n, H, d, dv):
+    state.test_single_tokens(form, [1] * n, H, H, d, dv)
