@@ -59,6 +59,27 @@ RUNS = ("state_mixers.runs",)  # key of the step's lists of runs, shared by all 
 CHUNK_FROM = 8                 # tokens a sequence (on average) from which a step takes its recurrences a run at a time
 
 
+def channel_runs_pay(lens, n_heads: int, d: int, dv: int, multiprocessors: int = 148) -> bool:
+    """Whether a step takes the delta rule with a decay per key channel a run at a time.  Token by token costs the longest sequence's
+    chain or, with enough columns of states to fill the device, all tokens' work; in runs a chain is eight times shorter and the
+    work about the same at heads of 128, 1.7 times as much at heads of 32 and 64.  Measured (us, token by token / in runs):
+      * a chain has to be worth a run's start: 16 heads of 128 x 128, 32 tokens 13.7 / 23.4, 65 tokens 25.9 / 28.6, 96 tokens 36 / 29,
+        257 tokens 93 / 45; 4 heads of 64 x 64 11 / 17, 20.7 / 20.5, 28.8 / 20.6, 74 / 32
+      * a full device has to wait for few long sequences: 64 sequences of 128 tokens, 16 heads of 128 x 128 727 / 763, of 64 x 64
+        197 / 320; one of 600 tokens beside 63 of one 402 / 280 and 311 / 129, 32 heads of 128 x 128 491 / 529
+      * below that, with blocks for more than one wave, the last runs have to be full (4 heads of 64 x 64, 32 sequences of 100 tokens
+        42 / 53, 64 of 128 95 / 87) or one sequence the longest by far (600 tokens beside 63 of one 173 / 60)
+    and from heads of 32 on the runs' outputs are no further from 64 bits than token by token (of 16: 1.03 to 1.06 times)."""
+    longest = max(lens)
+    if d < 32 or longest < 80:
+        return False
+    padded = sum(-(-n // K.STATE_RUN) * K.STATE_RUN for n in lens)
+    if len(lens) * n_heads * dv < 256 * multiprocessors:
+        return (len(lens) * n_heads * -(-dv // 16) <= 2 * multiprocessors or 8 * padded <= 9 * sum(lens)
+                or padded * n_heads * dv <= 40 * multiprocessors * longest)
+    return padded * n_heads * dv <= 80 * multiprocessors * longest
+
+
 def _run_lists(shape):
     """The index arrays of a prompt step's recurrences taken a run of tokens at a time: (sequence, first row among its new
     tokens) of every run, and every sequence's first run.  Steps of single tokens need no list."""
@@ -75,9 +96,12 @@ def _run_lists(shape):
 
 def _recur(step, q, k, v, state, o, H: int, G: int, d: int, dv: int, head_decay=None, token_decay=None, beta=None,
            channel_decay=None, runs: bool = True) -> None:
-    """The recurrence with one decay per head, or the delta rule with one per key channel, over the step's tokens: a run of tokens at a time in prompt steps, token by
-    token otherwise (and where `runs` is off: a decay outside [0, 1] has no logarithm to work with)."""
+    """The recurrence with one decay per head, or the delta rule with one per key channel, over the step's tokens: a run of tokens
+    at a time in prompt steps (the latter where `channel_runs_pay`), token by token otherwise (and where `runs` is off: a decay
+    outside [0, 1] has no logarithm to work with)."""
     lists = step.meta.get(RUNS) if runs and not step.all_decode else None
+    if lists and channel_decay is not None and not channel_runs_pay(step.shape.lens, H, d, dv):
+        lists = None
     if lists and step.n_tokens >= CHUNK_FROM * step.n_seqs and K.state_chunks_supported(d, dv):
         scratch = step.ws.buffer("state.runs", (K.state_chunks_scratch(lists["run_seq"].shape[0], H, d, dv, beta is not None,
                                                                   channel_decay is not None),),
