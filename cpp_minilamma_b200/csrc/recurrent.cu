@@ -1227,8 +1227,12 @@ MLL_API int mll_gated_group_norm(const float* o, const float* xs, const float* s
   MLL_REQUIRE((xs == nullptr) == (skip == nullptr), "gated group norm: a skip needs its input and its factors");
   MLL_REQUIRE(parts <= 65535, "gated group norm: too many parts for one launch");
   if (n_tokens == 0) return 0;
+  // A warp a part takes a part's words one after the other: beyond 128 columns it needs other parts beside it to hide that (parts of
+  // 512 columns, us, a block / a warp a part: 128 parts 3.1 / 4.9, 1,024 parts 5.6 / 5.3, 4,096 parts 14.2 / 7.0; of 1,024 columns:
+  // 1,536 parts 8.8 / 8.4).
   const int columns = width / parts;
-  if (columns % 4 == 0 && columns <= 1024 && dv % 4 == 0 && gate_ld % 4 == 0 && out_dtype == gate_dtype &&
+  const bool enough = columns <= 128 || (long long)n_tokens * parts >= 10ll * mll_sm_count();
+  if (enough && columns % 4 == 0 && columns <= 1024 && dv % 4 == 0 && gate_ld % 4 == 0 && out_dtype == gate_dtype &&
       (long long)n_tokens * parts < (1ll << 31) &&
       ((uintptr_t)o | (uintptr_t)xs | (uintptr_t)gate | (uintptr_t)weight | (uintptr_t)out) % 16 == 0) {
     if (out_dtype == MLL_F32)

@@ -3,9 +3,17 @@ reach: the checks are theirs."""
 import pytest
 import torch
 
+import test_gpu_row_words as rows
 import test_gpu_state_step as state
 
 pytestmark = pytest.mark.gpu
+both = pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+
+
+@both
+@pytest.mark.parametrize("columns,parts,T", [(132, 2, 739), (132, 2, 741), (256, 1, 1481), (1024, 2, 745), (1020, 8, 186), (8, 1, 3)])
+def test_gated_norm(dtype, columns, parts, T):
+    rows.test_gated_norm_in_parts(dtype, columns, parts, T)
 
 
 @pytest.mark.parametrize("form", ["head", "delta", "channel", "token", "delta_head"])
