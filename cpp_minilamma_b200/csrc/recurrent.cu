@@ -465,11 +465,20 @@ __global__ void __launch_bounds__(128) ssd_prepare_walk_kernel(SsdPrepArgs a, in
   }
 }
 
+// A thread's eight channels in a row are worth their latency once they, or the tokens, are many (us, a channel a thread / words;
+// 6,144 channels: 16 tokens 3.5 / 4.0, 48 tokens 6.2 / 4.8, 2,048 tokens 137 / 52; 1,152 channels: 128 tokens 4.2 / 4.8, 512 tokens
+// 10.4 / 8.4), and rows of a few words leave most of a block idle (96 channels, 1,024 tokens: 5.5 / 10.8).
+inline bool ssd_walk_pays(const SsdPrepArgs& a, int n_tokens) {
+  const long long channels = a.n_heads * a.dv + 2 * a.n_groups * a.d;
+  return channels >= 384 && channels * n_tokens >= (channels >= 1536 ? 240000 : 400000);
+}
+
 template <typename T, int TAPS>
 int launch_ssd_walk(const SsdPrepArgs& a, int n_tokens, cudaStream_t stream) {
   const int pieces = ((a.n_heads * a.dv + 2 * a.n_groups * a.d) / 8 + 127) / 128;
-  // tokens enough for several blocks a multiprocessor: walks of eight, else every token by itself
-  if (n_tokens >= 4 * mll_sm_count())
+  // walks of eight where they make two blocks a multiprocessor and more, else every token by itself (512 channels, 1,024 tokens: walks
+  // of eight 9.6 us, a channel a thread 6.4)
+  if ((long long)pieces * (n_tokens / 8) >= 2 * mll_sm_count())
     MLL_LAUNCH((ssd_prepare_walk_kernel<T, TAPS, 8>), dim3(pieces, (n_tokens + 7) / 8), 128, 0, stream, a, n_tokens);
   else
     MLL_LAUNCH((ssd_prepare_walk_kernel<T, TAPS, 1>), dim3(pieces, n_tokens), 128, 0, stream, a, n_tokens);
@@ -1197,7 +1206,7 @@ MLL_API int mll_ssd_prepare(const void* proj, const float* conv_w, const float* 
   if (n_tokens == 0) return 0;
   mll::SsdPrepArgs a{proj, conv_w, conv_b, conv_state, a_log, dt_bias, tok_seq, seq_slot, seq_qstart, q, k, u, xs, decay,
                      ld, n_heads, n_groups, d, dv, taps};
-  if ((dtype == MLL_F32 || dtype == MLL_BF16) && taps >= 2 && taps <= 4 && dv % 8 == 0 && (n_groups * d) % 8 == 0 && ld % 8 == 0 &&
+  if (mll::ssd_walk_pays(a, n_tokens) && (dtype == MLL_F32 || dtype == MLL_BF16) && taps >= 2 && taps <= 4 && dv % 8 == 0 && (n_groups * d) % 8 == 0 && ld % 8 == 0 &&
       n_tokens <= 65535 && ((uintptr_t)proj | (uintptr_t)conv_w | (uintptr_t)conv_b | (uintptr_t)conv_state | (uintptr_t)q |
                             (uintptr_t)k | (uintptr_t)u | (uintptr_t)xs) % 16 == 0)
     return dtype == MLL_F32 ? mll::launch_ssd_walk_taps<float>(a, n_tokens, stream)

@@ -16,6 +16,13 @@ def test_gated_norm(dtype, columns, parts, T):
     rows.test_gated_norm_in_parts(dtype, columns, parts, T)
 
 
+@both
+@pytest.mark.parametrize("H,G,N,P,taps,lens", [(12, 2, 128, 64, 4, [1] * 190), (12, 2, 128, 64, 4, [180]), (12, 2, 128, 64, 4, [1, 300, 2, 1000]),
+                                               (4, 1, 64, 64, 2, [1043, 3]), (6, 1, 64, 64, 3, [2500]), (24, 2, 128, 64, 3, [3, 1, 117])])
+def test_state_space_rows(dtype, H, G, N, P, taps, lens):
+    rows.test_state_space_rows(dtype, H, G, N, P, taps, lens)
+
+
 @pytest.mark.parametrize("form", ["head", "delta", "channel", "token", "delta_head"])
 @pytest.mark.parametrize("n,H,d,dv", [(1, 8, 128, 128), (2, 8, 128, 128), (4, 2, 256, 256), (1, 2, 256, 256), (1, 4, 192, 128), (3, 2, 33, 16),
                                       (2, 2, 32, 16), (600, 2, 72, 16), (300, 2, 72, 16), (70, 1, 64, 28)])
