@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(256) retention_prepare_kernel(RetPrepArgs a) {
 // neighbours inside a word).  A block a token, a column a thread, left 16 tokens on 16 multiprocessors: 9.3 us for them, 22.6
 // for 2,047 tokens of 8 heads of 128 and 256 (50 MB: 7.7 us at the copy peak), here 3.5 and
 // 12.1.
-template <typename T>
+template <typename T, bool ROTATE>
 __global__ void __launch_bounds__(256) retention_prepare_vec_kernel(RetPrepArgs a, long long words) {
   const int n = a.n_heads * a.d, nv = a.n_heads * a.dv, per_row = (2 * n + nv) / 8;
   for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < words; i += (long long)gridDim.x * 256) {
@@ -101,8 +101,8 @@ __global__ void __launch_bounds__(256) retention_prepare_vec_kernel(RetPrepArgs 
     float x[8];
     const T* src = (const T*)a.proj + t * a.ld + c;
     load_floats<T, 8>(src, x);
-    const int e = a.cos_table && c < 2 * n ? c % a.d : a.rot;
-    if (e < a.rot) {
+    const int e = ROTATE && c < 2 * n ? c % a.d : a.rot;
+    if (ROTATE && e < a.rot) {
       const int half = a.rot >> 1;
       const float* cs = a.cos_table + (size_t)a.tok_pos[t] * half;
       const float* sn = a.sin_table + (size_t)a.tok_pos[t] * half;
@@ -1273,17 +1273,22 @@ MLL_API int mll_retention_prepare(const void* proj, const float* cos_table, cons
   if (n_tokens == 0) return 0;
   mll::RetPrepArgs a{proj, rot > 0 ? cos_table : nullptr, sin_table, tok_pos, q, k, v, ld, n_heads, d, dv, rot,
                      interleaved, k_scale, silu};
+  // A rotation in words pays with rows that give a block's threads something to do, or many of them (us, a column / a word a thread:
+  // rows of 384 columns, 64 tokens 2.5 / 2.7, 1,024 tokens 3.4 / 3.1; of 768, 64 tokens 2.9 / 2.5).
   const bool words_rotate = rot == 0 || (d % 8 == 0 && rot % (interleaved ? 8 : 16) == 0 &&
+                                         (n_heads * (2 * d + dv) >= 768 || n_tokens >= 512) &&
                                          ((uintptr_t)cos_table | (uintptr_t)sin_table) % 16 == 0);
   if (words_rotate && (n_heads * d) % 8 == 0 && (n_heads * dv) % 8 == 0 && ld % 8 == 0 && (uintptr_t)proj % 16 == 0 &&
       (uintptr_t)q % 16 == 0 && (uintptr_t)k % 16 == 0 && (uintptr_t)v % 16 == 0 && (dtype == MLL_F32 || dtype == MLL_BF16)) {
     const long long words = (long long)n_tokens * (n_heads * (2 * d + dv) / 8);
     const long long want = (words + 255) / 256, most = (long long)mll_sm_count() * 16;
     const int blocks = (int)(want < most ? want : most);
-    if (dtype == MLL_F32)
-      MLL_LAUNCH((mll::retention_prepare_vec_kernel<float>), blocks, 256, 0, stream, a, words);
-    else
-      MLL_LAUNCH((mll::retention_prepare_vec_kernel<__nv_bfloat16>), blocks, 256, 0, stream, a, words);
+#define MLL_RET(T, ROTATE) MLL_LAUNCH((mll::retention_prepare_vec_kernel<T, ROTATE>), blocks, 256, 0, stream, a, words)
+    if (dtype == MLL_F32 && rot > 0) MLL_RET(float, true);
+    else if (dtype == MLL_F32) MLL_RET(float, false);
+    else if (rot > 0) MLL_RET(__nv_bfloat16, true);
+    else MLL_RET(__nv_bfloat16, false);
+#undef MLL_RET
     MLL_LAUNCH_CHECK();
     return 0;
   }

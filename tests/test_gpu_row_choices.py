@@ -23,6 +23,12 @@ def test_state_space_rows(dtype, H, G, N, P, taps, lens):
     rows.test_state_space_rows(dtype, H, G, N, P, taps, lens)
 
 
+@both
+@pytest.mark.parametrize("H,d,dv,rot,interleaved", [(2, 128, 128, 64, False), (4, 64, 64, 64, True), (3, 128, 8, 128, True), (4, 48, 96, 32, False)])
+def test_retention_rows(dtype, H, d, dv, rot, interleaved):
+    rows.test_retention_rows(dtype, H, d, dv, rot, interleaved)
+
+
 @pytest.mark.parametrize("form", ["head", "delta", "channel", "token", "delta_head"])
 @pytest.mark.parametrize("n,H,d,dv", [(1, 8, 128, 128), (2, 8, 128, 128), (4, 2, 256, 256), (1, 2, 256, 256), (1, 4, 192, 128), (3, 2, 33, 16),
                                       (2, 2, 32, 16), (600, 2, 72, 16), (300, 2, 72, 16), (70, 1, 64, 28)])
