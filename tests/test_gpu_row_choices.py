@@ -29,6 +29,11 @@ def test_retention_rows(dtype, H, d, dv, rot, interleaved):
     rows.test_retention_rows(dtype, H, d, dv, rot, interleaved)
 
 
+@pytest.mark.parametrize("d,rot", [(112, 16), (120, 120), (128, 128), (256, 64)])
+def test_chunked_attention_rows(d, rot):
+    rows.test_chunked_attention_rows_rotated_in_pairs(d, rot)
+
+
 @pytest.mark.parametrize("form", ["head", "delta", "channel", "token", "delta_head"])
 @pytest.mark.parametrize("n,H,d,dv", [(1, 8, 128, 128), (2, 8, 128, 128), (4, 2, 256, 256), (1, 2, 256, 256), (1, 4, 192, 128), (3, 2, 33, 16),
                                       (2, 2, 32, 16), (600, 2, 72, 16), (300, 2, 72, 16), (70, 1, 64, 28)])
