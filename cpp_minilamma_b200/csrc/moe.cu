@@ -39,7 +39,11 @@ struct RouteForm {
   int groups, groups_kept;
 };
 
-template <typename T>
+// DEEP: a round of 16 trips along the rows (8 of float32) is asked for before the first is used; left to itself the compiler keeps a
+// few loads in flight (24 tokens, 16 experts of 2,048, in a decode step: 11.2 us, so 7.0).  The registers that takes leave a
+// multiprocessor one block: it serves steps of no more tokens than multiprocessors (256 tokens, 16 experts: 6.9 us, deep 8.1), and
+// rows of a round or so (width 256: no difference, 100: 5 % slower).
+template <typename T, bool DEEP>
 __global__ void __launch_bounds__(512) moe_route_kernel(const T* __restrict__ h, const float* __restrict__ w,
                                                         const float* __restrict__ bias, const float* __restrict__ logits,
                                                         int* __restrict__ chosen, float* __restrict__ weight,
@@ -59,27 +63,38 @@ __global__ void __launch_bounds__(512) moe_route_kernel(const T* __restrict__ h,
       const float* we = w + (size_t)e * width;
       float s[4] = {0.f, 0.f, 0.f, 0.f};  // four partial sums a lane
       if (vec) {
-        // 16 bytes of the weight row and four activations a lane and trip, all of a round (16 trips, of float32 rows 8) asked
-        // for before the first is used: left to itself the compiler keeps a few loads in flight
-        // (24 tokens, 16 experts of 2,048, in a decode step: 11.2 us, now 7.0)
-        constexpr int TRIPS = sizeof(T) == 4 ? 8 : 16;
-        for (int i0 = lane * 4; i0 < width; i0 += TRIPS * 128) {
-          float4 wv[TRIPS];
-          RawWord<T, 4> hv[TRIPS];
+        // 16 bytes of the weight row and four activations a lane and trip
+        if constexpr (DEEP) {
+          constexpr int TRIPS = sizeof(T) == 4 ? 8 : 16;
+          for (int i0 = lane * 4; i0 < width; i0 += TRIPS * 128) {
+            float4 wv[TRIPS];
+            RawWord<T, 4> hv[TRIPS];
 #pragma unroll
-          for (int u = 0; u < TRIPS; ++u)
-            if (i0 + u * 128 < width) {
-              wv[u] = __ldg(reinterpret_cast<const float4*>(we + i0 + u * 128));
-              hv[u].fetch(row + i0 + u * 128);
-            }
+            for (int u = 0; u < TRIPS; ++u)
+              if (i0 + u * 128 < width) {
+                wv[u] = __ldg(reinterpret_cast<const float4*>(we + i0 + u * 128));
+                hv[u].fetch(row + i0 + u * 128);
+              }
 #pragma unroll
-          for (int u = 0; u < TRIPS; ++u)
-            if (i0 + u * 128 < width) {
-              s[0] = fmaf(hv[u][0], wv[u].x, s[0]);
-              s[1] = fmaf(hv[u][1], wv[u].y, s[1]);
-              s[2] = fmaf(hv[u][2], wv[u].z, s[2]);
-              s[3] = fmaf(hv[u][3], wv[u].w, s[3]);
-            }
+            for (int u = 0; u < TRIPS; ++u)
+              if (i0 + u * 128 < width) {
+                s[0] = fmaf(hv[u][0], wv[u].x, s[0]);
+                s[1] = fmaf(hv[u][1], wv[u].y, s[1]);
+                s[2] = fmaf(hv[u][2], wv[u].z, s[2]);
+                s[3] = fmaf(hv[u][3], wv[u].w, s[3]);
+              }
+          }
+        } else {
+#pragma unroll 8
+          for (int i = lane * 4; i < width; i += 128) {
+            const float4 wv = *reinterpret_cast<const float4*>(we + i);
+            float hv[4];
+            load_floats<T, 4>(row + i, hv);
+            s[0] = fmaf(hv[0], wv.x, s[0]);
+            s[1] = fmaf(hv[1], wv.y, s[1]);
+            s[2] = fmaf(hv[2], wv.z, s[2]);
+            s[3] = fmaf(hv[3], wv.w, s[3]);
+          }
         }
       } else {
         for (int i = lane; i < width; i += 32) s[0] = fmaf(to_float(row[i]), we[i], s[0]);
@@ -142,7 +157,8 @@ __global__ void __launch_bounds__(512) moe_route_kernel(const T* __restrict__ h,
     }
     }
     __syncwarp();
-    float chosen_sum = 0.f, mine = 0.f;  // lane j keeps the j-th choice's score: no way through memory before the division
+    // DEEP: lane j keeps the j-th choice's score, no way through memory before the division (a register that the other form lacks)
+    float chosen_sum = 0.f, mine = 0.f;
     for (int j = 0; j < top; ++j) {
       float best = -INFINITY;
       int at = 0x7fffffff;
@@ -159,14 +175,15 @@ __global__ void __launch_bounds__(512) moe_route_kernel(const T* __restrict__ h,
       if (at >= n_experts) at = j;
       const float sc = z[at];
       chosen_sum += sc;
-      if (lane == j) mine = sc;
+      if (DEEP && lane == j) mine = sc;
       if (lane == 0) {
         chosen[(size_t)t * top + j] = at;
+        if (!DEEP) weight[(size_t)t * top + j] = sc;
         choice[at] = -INFINITY;
       }
       __syncwarp();
     }
-    if (lane < top) weight[(size_t)t * top + lane] = mine / (chosen_sum + 1e-20f) * form.scale;
+    if (lane < top) weight[(size_t)t * top + lane] = (DEEP ? mine : weight[(size_t)t * top + lane]) / (chosen_sum + 1e-20f) * form.scale;
     return;
   }
   float first = 0.f, total = 0.f, mine = 0.f;
@@ -187,14 +204,15 @@ __global__ void __launch_bounds__(512) moe_route_kernel(const T* __restrict__ h,
     if (j == 0) first = best;
     const float p = expf(best - first);
     total += p;
-    if (lane == j) mine = p;
+    if (DEEP && lane == j) mine = p;
     if (lane == 0) {
       chosen[(size_t)t * top + j] = at;
+      if (!DEEP) weight[(size_t)t * top + j] = p;
       z[at] = -INFINITY;
     }
     __syncwarp();
   }
-  if (lane < top) weight[(size_t)t * top + lane] = mine / total;
+  if (lane < top) weight[(size_t)t * top + lane] = (DEEP ? mine : weight[(size_t)t * top + lane]) / total;
 }
 
 // ---- sort ----------------------------------------------------------------------------------------------------- //
@@ -386,15 +404,20 @@ MLL_API int mll_moe_route(const void* h, const float* w, const float* bias, cons
     groups = groups_kept = 0;
   }
   const size_t smem = (size_t)(2 * n_experts + 1 + groups) * sizeof(float);
-  // with the logits given there is work for one warp a token only (5,957 tokens, 16 experts: 29 us with blocks of 512, 7.4 with one warp)
-  const int threads = logits ? 32 : 512;
+  // With the logits given there is work for one warp a token only (5,957 tokens, 16 experts: 29 us with blocks of 512, 7.4 with one
+  // warp), except that a few tokens' many logits are fetched sooner by many warps (400 tokens, with 512 threads and with one warp:
+  // 256 experts 5.4 and 6.7 us, 128 experts 5.3 and 5.5; from 600 tokens one warp is the faster form at up to 512 experts).
+  const int threads = logits && (n_experts <= 64 || n_tokens >= 4 * mll_sm_count()) ? 32 : 512;
   const mll::RouteForm form{all_scores, scale, gate_out, groups, groups_kept};
-  if (dtype == MLL_F32)
-    MLL_LAUNCH((mll::moe_route_kernel<float>), n_tokens, threads, smem, stream, (const float*)h, w, bias, logits, chosen,
-               weight, n_tokens, width, n_experts, top, form);
-  else if (dtype == MLL_BF16)
-    MLL_LAUNCH((mll::moe_route_kernel<__nv_bfloat16>), n_tokens, threads, smem, stream, (const __nv_bfloat16*)h, w, bias,
-               logits, chosen, weight, n_tokens, width, n_experts, top, form);
+  const bool deep = !logits && n_tokens <= mll_sm_count() && width >= 1024;
+#define MLL_ROUTE(T, DEEP)                                                                                                      \
+  MLL_LAUNCH((mll::moe_route_kernel<T, DEEP>), n_tokens, threads, smem, stream, (const T*)h, w, bias, logits, chosen, weight, \
+             n_tokens, width, n_experts, top, form)
+  if (dtype == MLL_F32 && deep) MLL_ROUTE(float, true);
+  else if (dtype == MLL_F32) MLL_ROUTE(float, false);
+  else if (dtype == MLL_BF16 && deep) MLL_ROUTE(__nv_bfloat16, true);
+  else if (dtype == MLL_BF16) MLL_ROUTE(__nv_bfloat16, false);
+#undef MLL_ROUTE
   else
     MLL_REQUIRE(false, "moe route: unknown dtype %d", dtype);
   MLL_LAUNCH_CHECK();

@@ -39,3 +39,24 @@ def test_chunked_attention_rows(d, rot):
                                       (2, 2, 32, 16), (600, 2, 72, 16), (300, 2, 72, 16), (70, 1, 64, 28)])
 def test_single_tokens(form, n, H, d, dv):
     state.test_single_tokens(form, [1] * n, H, H, d, dv)
+
+
+@pytest.mark.parametrize("rows_,experts,width,tokens", [(1, 16, 1024, 149), (2, 130, 1028, 148), (1, 130, 64, 400), (1, 130, 64, 600), (2, 64, 64, 400)])
+@pytest.mark.parametrize("given", [False, True])
+def test_route(rows_, experts, width, tokens, given):
+    """Every form of the routing kernel: deep and plain loads, one warp a token and sixteen."""
+    from cpp_minilamma_b200.csrc import kernels as K
+    dev = torch.device("cuda:0")
+    gen = torch.Generator(device=dev).manual_seed(experts + tokens)
+    top = 4
+    h = torch.randn((tokens, width), generator=gen, device=dev).to((torch.float32, torch.bfloat16)[rows_ - 1])
+    w = torch.randn((experts, width), generator=gen, device=dev) / width ** 0.5
+    z = h.double() @ w.double().T
+    chosen = torch.full((tokens, top), -1, dtype=torch.int32, device=dev)
+    weight = torch.zeros((tokens, top), device=dev)
+    K.moe_route(h, w, None, chosen, weight, top, logits=z.float() if given else None)
+    best = z.topk(top + 1, dim=1)
+    clear = (best.values[:, :-1] - best.values[:, 1:]).min(1).values > 1e-4  # float32 sums of `width` terms of a few tell them apart
+    assert clear.float().mean() > 0.9
+    assert torch.equal(chosen[clear].long(), best.indices[clear][:, :top])
+    assert (weight.double() - best.values[:, :top].softmax(1))[clear].abs().max() <= 1e-5
