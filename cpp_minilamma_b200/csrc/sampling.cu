@@ -577,6 +577,7 @@ sample_temperature_cluster_kernel(const float* __restrict__ logits, int vocab, f
 constexpr int SC_BITS0 = 11, SC_BITS1 = 11, SC_BITS2 = 10;  // radix digits of the three selection passes
 constexpr int SC_BINS = 1 << SC_BITS0;
 constexpr int SC_CAND = 1024;
+constexpr int SC_BOUND_TOP_K = 640, SC_BOUND_TOP_K_ROWS = 800;  // see sample_top_k_cluster_kernel
 
 // Top-k (k <= 1024) then temperature sampling over the kept candidates in descending order, equal logits by
 // lower id (the rule of sample_top_k_kernel).  The k-th largest key is narrowed down by a radix selection over the
@@ -591,8 +592,12 @@ constexpr int SC_CAND = 1024;
 // can be kept, and as a rule few more than k reach it and the passes are not needed.  What a pass costs is the sum of eight
 // histograms of 2,048 bins over distributed shared memory, in every block, and its atomic additions to the few bins that a
 // vocabulary's logits crowd into.  64 rows of 128,256 logits, k = 40 (33 MB, 5 us at the copy peak): 102 us without the bound,
-// 42 us with it.
-template <int VPT>
+// 42 us with it.  With hundreds kept the blocks' smallest key lies so low that more than 1,024 reach it and the passes follow all
+// the same, with fewer keys to count.  At 16 and 64 keys a thread that is still the faster way (k = 1,024: 0.9 times); at 32, where
+// two blocks share a multiprocessor, it is not (128,256 logits, one row: k = 600 36 us without, 25 with; 800 to 1,024 49 and 53; 64
+// rows, of which some still need no passes: 700 105 and 56, 800 144 and 118, 900 175 and 184) and BOUND is off, nor does it help rows
+// whose logits are all equal (44 and 50 us).
+template <int VPT, bool BOUND>
 __global__ void __cluster_dims__(SC_CLUSTER, 1, 1) __launch_bounds__(SC_THREADS, (VPT <= 32 ? 2 : 1))
 sample_top_k_cluster_kernel(const float* __restrict__ logits, int vocab, int top_k, float temperature,
                             unsigned long long seed, const int* __restrict__ request, const int* __restrict__ step,
@@ -631,7 +636,7 @@ sample_top_k_cluster_kernel(const float* __restrict__ logits, int vocab, int top
   int at_or_above = vocab;   // keys at or above the lower bound that the digits give
   int passes = 0;
   unsigned bound = 0;        // no key below it is kept
-  {
+  if constexpr (BOUND) {
     unsigned largest = 0;
 #pragma unroll
     for (int j = 0; j < VPT; ++j)
@@ -878,8 +883,11 @@ void launch_sample_cluster(const float* logits, int n_rows, int vocab, float tem
   if (top_k == 0)
     MLL_LAUNCH((sample_temperature_cluster_kernel<VPT>), dim3(SC_CLUSTER, n_rows), SC_THREADS, 0, stream, logits, vocab,
                temperature, seed, request, step, tokens, status, errors);
+  else if (VPT != 32 || top_k <= (n_rows >= 32 ? SC_BOUND_TOP_K_ROWS : SC_BOUND_TOP_K))
+    MLL_LAUNCH((sample_top_k_cluster_kernel<VPT, true>), dim3(SC_CLUSTER, n_rows), SC_THREADS, 0, stream, logits, vocab, top_k,
+               temperature, seed, request, step, tokens, status, errors);
   else
-    MLL_LAUNCH((sample_top_k_cluster_kernel<VPT>), dim3(SC_CLUSTER, n_rows), SC_THREADS, 0, stream, logits, vocab, top_k,
+    MLL_LAUNCH((sample_top_k_cluster_kernel<VPT, VPT != 32>), dim3(SC_CLUSTER, n_rows), SC_THREADS, 0, stream, logits, vocab, top_k,
                temperature, seed, request, step, tokens, status, errors);
 }
 
@@ -908,12 +916,12 @@ MLL_API int mll_sample_resident_rows(int vocab, int top_k) {
   if (run == 0) return 0;
   if (run == 16)
     return top_k == 0 ? mll::sample_clusters_resident(mll::sample_temperature_cluster_kernel<16>)
-                      : mll::sample_clusters_resident(mll::sample_top_k_cluster_kernel<16>);
+                      : mll::sample_clusters_resident(mll::sample_top_k_cluster_kernel<16, true>);
   if (run == 32)
     return top_k == 0 ? mll::sample_clusters_resident(mll::sample_temperature_cluster_kernel<32>)
-                      : mll::sample_clusters_resident(mll::sample_top_k_cluster_kernel<32>);
+                      : mll::sample_clusters_resident(mll::sample_top_k_cluster_kernel<32, true>);
   return top_k == 0 ? mll::sample_clusters_resident(mll::sample_temperature_cluster_kernel<64>)
-                    : mll::sample_clusters_resident(mll::sample_top_k_cluster_kernel<64>);
+                    : mll::sample_clusters_resident(mll::sample_top_k_cluster_kernel<64, true>);
 }
 
 // temperature > 0; top_k == 0 samples from the whole vocabulary, 2 <= top_k <= 1024 from the

@@ -5,6 +5,7 @@ import torch
 
 import test_gpu_row_words as rows
 import test_gpu_state_step as state
+import test_gpu_top_k_bound as top_k
 
 pytestmark = pytest.mark.gpu
 both = pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
@@ -39,6 +40,12 @@ def test_chunked_attention_rows(d, rot):
                                       (2, 2, 32, 16), (600, 2, 72, 16), (300, 2, 72, 16), (70, 1, 64, 28)])
 def test_single_tokens(form, n, H, d, dv):
     state.test_single_tokens(form, [1] * n, H, H, d, dv)
+
+
+@pytest.mark.parametrize("k", [640, 641, 1000])
+@pytest.mark.parametrize("vocab", [40000, 100000, 131072, 140000])
+def test_kept_ids(vocab, k):
+    top_k.test_kept_ids(vocab, k)
 
 
 @pytest.mark.parametrize("rows_,experts,width,tokens", [(1, 16, 1024, 149), (2, 130, 1028, 148), (1, 130, 64, 400), (1, 130, 64, 600), (2, 64, 64, 400)])
