@@ -25,17 +25,22 @@ def test_product(rows, n, k):
             K.linear_f32(x, w, b, out, slices=slices)
             exact = want if b is None else want + b
             assert ((out.double() - exact).abs() <= slack + exact.abs() * 2.0 ** -23).all(), (slices, b is None)
-    if n % 16 == 0:
-        assert K.linear_f32_supported(x, w, K.EPI_SWIGLU)
+    for epilogue in ((K.EPI_SWIGLU, K.EPI_GEGLU) if n % 16 == 0 else ()):
+        assert K.linear_f32_supported(x, w, epilogue)
         blocks = want.view(rows, n // 16, 2, 8)
         gate, up = blocks[:, :, 0].reshape(rows, -1), blocks[:, :, 1].reshape(rows, -1)
         s = slack.view(rows, n // 16, 2, 8)
-        bound = 1.2 * s[:, :, 0].reshape(rows, -1) * up.abs() + gate.abs() * s[:, :, 1].reshape(rows, -1)  # silu is 1.1-Lipschitz
-        exact = torch.nn.functional.silu(gate) * up
-        for slices in (0, 2, 8):
+        # silu is 1.1-Lipschitz and gelu (tanh form) 1.13; both are no larger than their argument
+        bound = 1.2 * s[:, :, 0].reshape(rows, -1) * up.abs() + gate.abs() * s[:, :, 1].reshape(rows, -1)
+        if epilogue == K.EPI_SWIGLU:
+            exact, own = torch.nn.functional.silu(gate) * up, 0.0
+        else:
+            # formed as g sigmoid(y): y is rounded by no more than 2^-22 |y|, and |y| times sigmoid's slope stays below 0.28
+            exact, own = torch.nn.functional.gelu(gate, approximate="tanh") * up, 2.0 ** -23 * (gate * up).abs()
+        for slices in (0, 1, 2, 4, 8):
             out = torch.full((rows, n // 2), 7.0, device=dev)
-            K.linear_f32(x, w, None, out, K.EPI_SWIGLU, slices)
-            assert ((out.double() - exact).abs() <= bound + exact.abs() * 2.0 ** -20).all(), slices
+            K.linear_f32(x, w, None, out, epilogue, slices)
+            assert ((out.double() - exact).abs() <= bound + own + exact.abs() * 2.0 ** -20).all(), (epilogue, slices)
 
 
 def test_refused_and_left_to_the_library():
