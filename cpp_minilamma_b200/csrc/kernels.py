@@ -14,7 +14,7 @@ import torch
 from ..cache.paged import PAGE  # cache positions per page; the library's MLL_PAGE is checked against it on load
 from .build import KernelBuildError, load_library
 
-ABI_VERSION = 38
+ABI_VERSION = 39
 MAX_TOP_K = 1024
 STATE_RUN = 32  # tokens a run of `state_chunks`
 
@@ -334,6 +334,11 @@ def linear_f32_supported(x: torch.Tensor, w: torch.Tensor, epilogue: int = EPI_F
     return (SMALL_LINEAR != "none" and x.dtype == torch.float32 and w.dtype == torch.float32 and x.dim() == 2
             and x.is_contiguous() and w.is_contiguous() and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
             and bool(lib().mll_linear_f32_supported(x.shape[0], w.shape[0], w.shape[1], epilogue)))
+
+
+def linear_f32_pays(x: torch.Tensor, w: torch.Tensor) -> bool:
+    """Whether `linear_f32` takes x . w^T and is faster than the library's product."""
+    return linear_f32_supported(x, w) and bool(lib().mll_linear_f32_pays(x.shape[0], w.shape[0], w.shape[1]))
 
 
 def linear_f32(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor, epilogue: int = EPI_F32,

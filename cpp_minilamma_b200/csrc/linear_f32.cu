@@ -165,14 +165,15 @@ int launch_linear_f32(LinearF32Args a, int slices, cudaStream_t stream) {
   const int units = (a.N + F_ROWS - 1) / F_ROWS;
   if (slices <= 0) {
     // As many slices as still let all blocks be resident at once (o of the 1B shape, 4 rows: 8.7 us unsplit, 5.3 in four,
-    // 6.1 in eight).  A matrix that takes several waves anyway: slices of about 1,024 where two blocks share a
-    // multiprocessor (its 128,256-row head: 164 us unsplit, 156 in two, 168 in four), else none.
+    // 6.1 in eight; 256 x 192, 9 rows: 4.3 unsplit, 3.1 in four).  A matrix that takes several waves anyway: slices of 1,024, four
+    // at most, where two blocks share a multiprocessor (its 128,256-row head: 164 us unsplit, 156 in two, 168 in four; 131,072 x
+    // 512, one row: 39 unsplit, 62 in two), else none.
     const int resident = mll_sm_count() * OCC;
     slices = 1;
     if ((units + F_WARPS - 1) / F_WARPS <= resident) {
-      while (slices < F_WARPS && (units * slices * 2 + F_WARPS - 1) / F_WARPS <= resident && a.K / (slices * 2) >= 128) slices *= 2;
+      while (slices < F_WARPS && (units * slices * 2 + F_WARPS - 1) / F_WARPS <= resident && a.K / (slices * 2) >= 32) slices *= 2;
     } else if (OCC > 1) {
-      slices = a.K >= 4096 ? 4 : (a.K >= 256 ? 2 : 1);
+      while (slices < 4 && a.K / (slices * 2) >= 1024) slices *= 2;
     }
   }
   MLL_REQUIRE(slices == 1 || slices == 2 || slices == 4 || slices == 8, "linear_f32: %d slices", slices);
@@ -195,6 +196,16 @@ MLL_API int mll_linear_f32_supported(int M, int N, int K, int epilogue) {
   if (M < 1 || M > mll::F_MAX_M || N < 1 || K < 4 || K % 4 != 0 || (M > 8 && N > 16384)) return 0;
   if (epilogue == mll::FEPI_F32) return 1;
   return (epilogue == mll::FEPI_SWIGLU || epilogue == mll::FEPI_GEGLU) && N % 16 == 0;
+}
+
+// Whether it is the faster way for a product without an epilogue (us, the library / here): short rows of a tall matrix are not what
+// the kernel is laid out for (16,384 x 64, 8 rows 5.1 / 7.5; 6,144 x 256 6.9 / 4.3), from 9 rows on no short rows are (64 x 64,
+// 16 rows 2.6 / 3.3; 512 x 128 2.9 / 3.0; 1,024 x 128 4.9 / 3.2) and the tallest matrices need long ones (16,384 x 1,024, 16 rows
+// 36.8 / 39.8; x 2,048 70 / 66; 12,288 x 512 29 / 27).
+MLL_API int mll_linear_f32_pays(int M, int N, int K) {
+  if (M <= 4) return 1;
+  if (M <= 8) return K >= 256 || N <= 4096;
+  return K >= (N <= 4096 ? 128 : 256) && (N <= 12288 || K >= 2048);
 }
 
 // x: float32 [M, K]; w: float32 [N, K]; bias: optional float32 [N]; out: float32 [M, N] (epilogue 1), or [M, N / 2] =

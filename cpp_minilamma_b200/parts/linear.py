@@ -105,7 +105,7 @@ class Linear:
         return self._biased(out)
 
     def _product_f32(self, step, x: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
-        if x.shape[0] <= step.small_rows and out.is_contiguous() and K.linear_f32_supported(x, self.weight):
+        if x.shape[0] <= step.small_rows and out.is_contiguous() and K.linear_f32_pays(x, self.weight):
             K.linear_f32(x, self.weight, self.bias, out)
             return out
         torch.mm(x, self.weight.t(), out=out)

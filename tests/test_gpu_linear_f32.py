@@ -54,3 +54,23 @@ def test_refused_and_left_to_the_library():
     assert not K.linear_f32_supported(torch.zeros(2, 64, device=dev), torch.zeros(24, 64, device=dev), K.EPI_SWIGLU)
     with pytest.raises(K.KernelError):
         K.linear_f32(torch.zeros(2, 64, device=dev), w, None, torch.zeros(2, 31, device=dev))
+
+
+@pytest.mark.parametrize("m,n,k,own", [(4, 16384, 64, True), (5, 16384, 64, False), (8, 4096, 64, True), (8, 4100, 252, False), (8, 4100, 256, True),
+                                       (9, 64, 124, False), (9, 64, 128, True), (16, 4100, 252, False), (16, 12288, 256, True), (16, 12292, 256, False),
+                                       (16, 12292, 2048, True), (17, 64, 256, False)])
+def test_left_to_the_library_where_that_is_faster(m, n, k, own):
+    from types import SimpleNamespace
+    from cpp_minilamma_b200.csrc import kernels as K
+    from cpp_minilamma_b200.parts.linear import Linear
+    dev = torch.device("cuda:0")
+    gen = torch.Generator(device=dev).manual_seed(m + n + k)
+    x, w, bias = (torch.randn(s, generator=gen, device=dev) for s in ((m, k), (n, k), (n,)))
+    assert K.linear_f32_pays(x, w) == own
+    part, before = Linear(w, "w", bias=bias), K.calls.get("linear_f32", 0)
+    out = part._product_f32(SimpleNamespace(small_rows=64), x, torch.empty((m, n), device=dev))
+    assert K.calls.get("linear_f32", 0) - before == own
+    want = x.double() @ w.double().T + bias
+    # float32 sums of k terms, and the bias's addition
+    slack = (x.abs().double() @ w.abs().double().T) * k ** 0.5 * 2.0 ** -24 + 1e-7 * bias.abs() + want.abs() * 2.0 ** -23
+    assert ((out.double() - want).abs() <= slack).all()
