@@ -1960,23 +1960,38 @@ class MoePlan(NamedTuple):
     mma: bool
 
 
-MOE_TILE_ROWS_OVERRIDE: Optional[int] = None  # measurements only: 0, 1 or 2 picks the tensor-core tile at every size
+MOE_TILE_ROWS_OVERRIDE: Optional[int] = None  # measurements only: 0 to 3 picks the tensor-core tile at every size
 
 
-def moe_tile_rows(mma: bool, n_pairs: int = 1 << 30, n_experts: int = 1) -> int:
-    """Rows of a tile of the routed products: the plain kernels' size, or one of the tensor-core kernels' three - 16
-    rows while an expert gets 12 rows or fewer on average (single tokens), 32 rows up to 28 on average, else the 256 of
-    the tcgen05 kernel.  (Measured at 16 experts: at 10.7 rows an expert 16-row tiles are 5 to 18 % faster than 32-row
-    ones, at 16 rows an expert - where about half of the experts need a second 16-row tile - 32-row tiles are up to 20 %
-    faster.  Tiles of 32 rows against the tcgen05 kernel, both
-    products, 16 experts of 2,048 x 2,048: 24 rows an expert 105 / 136 us, 32 rows 151 / 125, 40 rows 184 / 125; of
-    4,096 x 3,584: 12.5 rows 325 / 306, 25 rows 328 / 317.)"""
+def moe_tile_rows(mma: bool, n_pairs: int = 1 << 30, n_experts: int = 1, width: int = 4096, inter: int = 4096) -> int:
+    """Rows of a tile of the routed products of experts of `inter` x `width`: the plain kernels' size, or one of the tensor-core
+    kernels' four.  Measured, both products, us (rows an expert on average):
+      * 16 rows up to 12 (at 10.7 rows 5 to 18 % faster than 32-row tiles, at 16 rows - where about half of the experts need a second
+        16-row tile - 32-row tiles are up to 20 % faster)
+      * the 256 of the tcgen05 kernel from 28 (16 experts of 2,048 x 2,048, 32-row tiles / tcgen05: 24 rows 102 / 131, 28 rows 133 /
+        120; 64 of 1,408 x 2,048 261 / 253, 286 / 255), beyond 8 M weights a matrix, which 32-row tiles read for little, at once
+        (16 of 3,584 x 4,096: 14 rows 327 / 301), and from 48 where down's tiles are fewer than the pairs of multiprocessors and long
+        (8 of 3,584 x 1,024: 40 rows 94 / 113, 48 rows 106 / 101).  Its launches cost 35 us however little they do, so the step has to
+        have the work: 0.85 G weights times rows (8 of 1,024 x 1,024: 64 rows 46 / 51, 128 rows 55 / 52), more for the smallest
+        experts, of which a tile of 256 x 256 is a large part (16 of 512 x 256, 800 rows: 128-row tiles 61, tcgen05 75)
+      * else 32 rows, or 128 from 160 (4 of 512 x 512: 100 rows 17 / 29, 300 rows 27 / 30, 600 rows 42 / 37; 16 of 512 x 256: 128 rows
+        24 / 29, 200 rows 30 / 29, 400 rows 53 / 40)"""
     if not mma:
         return int(lib().mll_moe_simt_rows())
-    if MOE_TILE_ROWS_OVERRIDE is not None:
-        return int(lib().mll_moe_mma_rows(ctypes.c_int(MOE_TILE_ROWS_OVERRIDE)))
-    small = 1 if n_pairs <= 12 * n_experts else (2 if n_pairs <= 28 * n_experts else 0)
-    return int(lib().mll_moe_mma_rows(ctypes.c_int(small)))
+    kind = moe_tile_kind(n_pairs, n_experts, width, inter) if MOE_TILE_ROWS_OVERRIDE is None else MOE_TILE_ROWS_OVERRIDE
+    return int(lib().mll_moe_mma_rows(ctypes.c_int(kind)))
+
+
+def moe_tile_kind(n_pairs: int, n_experts: int, width: int, inter: int, multiprocessors: int = 148) -> int:
+    """The rule of `moe_tile_rows`: 0 tcgen05, 1 tiles of 16 rows, 2 of 32, 3 of 128."""
+    if n_pairs <= 12 * n_experts:
+        return 1
+    weights = width * inter
+    few_long_tiles = n_experts * -(-width // 256) < multiprocessors // 2 and inter > width
+    rows_from = 0 if weights >= 8 << 20 else 48 if few_long_tiles else 28
+    if n_pairs >= rows_from * n_experts and n_pairs * weights >= max(850_000_000, 450_000_000_000_000 // weights):
+        return 0
+    return 3 if n_pairs >= 160 * n_experts else 2
 
 
 def moe_needs_rows(plan: MoePlan) -> bool:

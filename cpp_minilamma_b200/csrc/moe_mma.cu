@@ -1,15 +1,16 @@
-// The two products of the routed feed-forward (moe.cu) for steps with few rows per expert (single tokens), bfloat16:
-// mma.sync m16n8k16 with float32 accumulation on tiles of 16 rows of one expert - one MMA row tile - times 64 weight rows,
-// four warps side by side, operands through a cp.async ring (four stages of 64 columns of k, gate_up three of 128), three or four such blocks a
-// multiprocessor (256 weight rows, one block a multiprocessor: the same time; two warps on 128 weight rows: a quarter
-// slower).  Such a step streams every touched expert's weights once for a handful of rows: memory bounds it.
-// Between 12 and 32 rows per expert on average a second instance has tiles of 32 rows (two MMA row tiles a warp): with
-// 16-row tiles the experts that got 17 rows or more take a second tile each, and a few of those push the grid past the
-// blocks that are resident at once - a second, nearly empty wave.  Steps with more rows run in moe_tc5.cu.
-//   gate_up  the 64 weight rows are 32 gate rows and the 32 up rows of the same activation columns; a warp's
+// The two products of the routed feed-forward (moe.cu) for steps with few rows per expert (single tokens) and for small experts,
+// bfloat16: mma.sync m16n8k16 with float32 accumulation on tiles of 16 rows of one expert - one MMA row tile - times 64 weight
+// rows, four warps side by side, operands through a cp.async ring (four stages of 64 columns of k, gate_up three of 128),
+// three or four such blocks a multiprocessor (256 weight rows, one block a multiprocessor: the same time; two warps on 128 weight
+// rows: a quarter slower).  Such a step streams every touched expert's weights once for a handful of rows: memory bounds it.
+// A second instance has tiles of 32 rows (two MMA row tiles a warp): with 16-row tiles the experts that got 17 rows or more take a
+// second tile each, and a few of those push the grid past the blocks that are resident at once - a second, nearly empty wave.
+// A third, for many rows of experts that are too small for moe_tc5.cu, has tiles of 128 rows times 128 weight rows on eight warps.
+// Which steps take which, and which run in moe_tc5.cu: `moe_tile_rows` on the calling side.
+//   gate_up  half of the weight rows are gate rows, half the up rows of the same activation columns; a warp's
 //            8-column tiles are half of gate and the same half of up, so silu(gate) * up happens in the
 //            accumulator registers; rows are gathered from the step's tokens by (token, choice) pair.
-//   down     the 64 weight rows are output columns; a row's result is multiplied by its pair's routing weight
+//   down     the weight rows are output columns; a row's result is multiplied by its pair's routing weight
 //            and written as float32 to the pair's row (summed over a token's choices by the combine kernel).
 // Rows past a tile's end and columns past the matrices' edges are zero-filled in shared memory.
 #include "attention_decode.cuh"
@@ -31,7 +32,8 @@ struct MoeMmaShape {
 // 1,408 x 2,048, 32 tokens: 123.2 / 112.5).  down, with half the blocks, keeps four blocks a multiprocessor, which hold a
 // batch's tiles at once (24 tokens: 27.5 / 34.0; of 2,048 x 3,584: 86.2 / 91.6).
 using MoeMmaSmall = MoeMmaShape<1, 2, 1, 4, 64, 4>;
-using MoeMmaMedium = MoeMmaShape<2, 2, 1, 4, 64, 4>;  // 32 rows x 64 weight rows: single tokens, 12 to 32 rows an expert
+using MoeMmaMedium = MoeMmaShape<2, 2, 1, 4, 64, 4>;  // 32 rows x 64 weight rows
+using MoeMmaWide = MoeMmaShape<2, 8, 4, 2, 64, 3>;    // 128 rows x 128 weight rows
 
 // KIND 0: down; 1: gate_up (silu(gate) * up); 2: up alone with gelu (erf form) - the layout of `down`, rows gathered
 // by token, the activation in the accumulators, bfloat16 out by place.
@@ -192,16 +194,18 @@ int launch_moe_mma_rows(const MoeProductArgs& a, int max_tiles, int tile_rows, c
     else return launch_moe_mma<KIND, 1, 2, 1, 4, 64, 4>(a, max_tiles, stream);
   }
   if (tile_rows == MoeMmaMedium::BM) return launch_moe_mma<KIND, 2, 2, 1, 4, 64, 4>(a, max_tiles, stream);
-  mll_set_error("moe (mma): tiles of %d rows (known: %d, %d, %d)", tile_rows, MoeMmaSmall::BM, MoeMmaMedium::BM, mll_moe_tc5_rows());
+  if (tile_rows == MoeMmaWide::BM) return launch_moe_mma<KIND, 2, 8, 4, 2, 64, 3>(a, max_tiles, stream);
+  mll_set_error("moe (mma): tiles of %d rows (known: %d, %d, %d, %d)", tile_rows, MoeMmaSmall::BM, MoeMmaMedium::BM, MoeMmaWide::BM,
+                mll_moe_tc5_rows());
   return -1;
 }
 
 }  // namespace mll
 
-// Rows of a tile: those of moe_tc5.cu (small = 0) or one of the two here for steps with few rows per expert (1: 16 rows, 2: 32).
-MLL_API int mll_moe_mma_rows(int small) {
-  if (small == 0) return mll_moe_tc5_rows();
-  return small == 1 ? mll::MoeMmaSmall::BM : mll::MoeMmaMedium::BM;
+// Rows of a tile: those of moe_tc5.cu (kind 0) or of one of the three instances here (1: 16 rows, 2: 32, 3: 128).
+MLL_API int mll_moe_mma_rows(int kind) {
+  if (kind == 0) return mll_moe_tc5_rows();
+  return kind == 1 ? mll::MoeMmaSmall::BM : kind == 2 ? mll::MoeMmaMedium::BM : mll::MoeMmaWide::BM;
 }
 
 // bfloat16 only; rows of 16-byte words on both sides of both products.

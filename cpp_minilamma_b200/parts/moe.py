@@ -137,7 +137,7 @@ class RoutedFeedForward(FeedForward):
                 + (self.shared.parameter_bytes() if self.shared is not None else 0))
 
     def _plan(self, step, n_pairs: int, mma: bool) -> K.MoePlan:
-        rows = K.moe_tile_rows(mma, n_pairs, self.routed)
+        rows = K.moe_tile_rows(mma, n_pairs, self.routed, self.router.shape[1], self.inter)
         tiles = K.moe_max_tiles(n_pairs, self.routed, rows)
         ws = step.ws
         return K.MoePlan(ws.buffer("moe.order", (n_pairs,), torch.int32), ws.buffer("moe.offsets", (self.routed + 1,), torch.int32),
@@ -165,8 +165,8 @@ class RoutedFeedForward(FeedForward):
         shared_gate = ws.buffer("moe.shared_gate", (T,), torch.float32) if self.shared_gate_name else None
         K.moe_route(h, self.router, self.router_bias, chosen, weight, self.top, logits=logits, all_scores=self.all_scores,
                     scale=self.scale, gate_out=shared_gate, groups=self.groups)
-        # bfloat16: tiles of 64 rows on tensor cores at every size - with few rows per expert the products stream each
-        # touched expert's weights once, and a mostly empty tile costs nothing that memory does not hide
+        # bfloat16: tensor cores at every size, in tiles that fit the step (`moe_tile_rows`) - with few rows per expert the
+        # products stream each touched expert's weights once, and a mostly empty tile costs nothing that memory does not hide
         mma = K.USE_TENSOR_CORE_MOE and K.moe_mma_supported(act, D, self.inter)
         plan = self._plan(step, n_pairs, mma)
         K.moe_sort(chosen, plan, self.routed, n_real=self.experts)

@@ -67,3 +67,46 @@ def test_route(rows_, experts, width, tokens, given):
     assert clear.float().mean() > 0.9
     assert torch.equal(chosen[clear].long(), best.indices[clear][:, :top])
     assert (weight.double() - best.values[:, :top].softmax(1))[clear].abs().max() <= 1e-5
+
+
+@pytest.mark.parametrize("form", [0, 1])
+@pytest.mark.parametrize("per,experts,width,inter,top", [(0.25, 16, 512, 1024, 4), (0.6, 16, 512, 2048, 4), (3, 16, 520, 2048, 4), (1, 64, 256, 1408, 6), (4, 4, 64, 64, 2),
+                                                         (170, 4, 72, 136, 1), (300, 3, 512, 264, 2)])
+def test_small_and_wide_tiles(per, experts, width, inter, top, form):
+    """gate_up's 16-row tiles in long and in short stages and tiles of 128 rows, against float64 of the same bfloat16 values."""
+    from cpp_minilamma_b200.csrc import kernels as K
+    dev = torch.device("cuda:0")
+    gen = torch.Generator(device=dev).manual_seed(experts + width)
+    draw = lambda *shape: torch.randn(shape, generator=gen, device=dev)
+    T = max(1, round(per * experts / top))
+    chosen = torch.stack([torch.randperm(experts, generator=gen, device=dev)[:top] for _ in range(T)]).int().contiguous()
+    h = draw(T, width).to(torch.bfloat16)
+    first = (0.2 * draw(experts, inter * (1 if form else 2), width)).to(torch.bfloat16)
+    down, weight = (0.2 * draw(experts, width, inter)).to(torch.bfloat16), torch.rand((T, top), generator=gen, device=dev)
+    n = T * top
+    tile = K.moe_tile_rows(True, n, experts, width, inter)
+    assert tile == (16 if per < 100 else 128)
+    tiles = K.moe_max_tiles(n, experts, tile)
+    ints = lambda count: torch.full((count,), -7, dtype=torch.int32, device=dev)
+    plan = K.MoePlan(ints(n), ints(experts + 1), ints(tiles), ints(tiles), ints(1), tile, True)
+    K.moe_sort(chosen, plan, experts)
+    act = torch.full((n, inter), 7.0, dtype=torch.bfloat16, device=dev)
+    y = torch.full((n, width), 7.0, device=dev)
+    K.moe_gate_up(h, first, act, plan, top, form=form)
+    K.moe_down(act, down, y, weight, plan, top)
+    order = plan.order.long()
+    expert = chosen.view(-1)[order].long()
+    for e in expert.unique().tolist():
+        at = (expert == e).nonzero()[:, 0]
+        x, w = h[order[at] // top].double(), first[e].double()
+        z, slack = x @ w.T, (x.abs() @ w.abs().T) * width ** 0.5 * 2.0 ** -23  # float32 sums of `width` terms
+        if form:
+            want, slack = torch.nn.functional.gelu(z), 1.2 * slack
+        else:
+            gate, up = z[:, :inter], z[:, inter:]
+            want = torch.nn.functional.silu(gate) * up
+            slack = 1.2 * slack[:, :inter] * up.abs() + gate.abs() * slack[:, inter:]
+        assert ((act[at].double() - want).abs() <= want.abs() * 2.0 ** -8 + slack + 1e-6).all(), e
+        a, d = act[at].double(), down[e].double()
+        want = weight.view(-1)[order[at]].double()[:, None] * (a @ d.T)
+        assert ((y[order[at]].double() - want).abs() <= (a.abs() @ d.abs().T) * inter ** 0.5 * 2.0 ** -23 + 1e-6).all(), e

@@ -1,6 +1,7 @@
 """Rules by which a step picks a kernel, on either side of their lines, without a GPU."""
 import pytest
 
+from cpp_minilamma_b200.csrc.kernels import moe_tile_kind
 from cpp_minilamma_b200.parts.state_mixers import channel_runs_pay
 
 
@@ -11,3 +12,12 @@ from cpp_minilamma_b200.parts.state_mixers import channel_runs_pay
     ([128] * 16, 16, 128, 128, True), ([100] * 32, 2, 32, 32, True), ([100] * 32, 4, 64, 64, False)])
 def test_delta_rule_in_runs(lens, heads, d, dv, runs):
     assert channel_runs_pay(lens, heads, d, dv) == runs
+
+
+@pytest.mark.parametrize("rows,experts,width,inter,kind", [
+    (12, 16, 2048, 2048, 1), (13, 16, 2048, 2048, 2), (27, 16, 2048, 2048, 2), (28, 16, 2048, 2048, 0),  # rows an expert
+    (13, 16, 4096, 3584, 0), (12, 16, 4096, 3584, 1), (40, 8, 1024, 3584, 2), (48, 8, 1024, 3584, 0),
+    (64, 8, 1024, 1024, 2), (128, 8, 1024, 1024, 0), (159, 4, 512, 512, 2), (160, 4, 512, 512, 3), (800, 16, 256, 512, 3),
+    (4000, 16, 256, 512, 0), (16, 2, 4096, 4096, 2), (1 << 20, 1, 8, 8, 3)])
+def test_tiles_of_routed_products(rows, experts, width, inter, kind):
+    assert moe_tile_kind(rows * experts, experts, width, inter) == kind
