@@ -1,6 +1,6 @@
 // The two products of the routed feed-forward (moe.cu) for steps with few rows per expert (single tokens) and for small experts,
 // bfloat16: mma.sync m16n8k16 with float32 accumulation on tiles of 16 rows of one expert - one MMA row tile - times 64 weight
-// rows, four warps side by side, operands through a cp.async ring (four stages of 64 columns of k, gate_up three of 128),
+// rows, four warps side by side, operands through a cp.async ring (four stages of 64 columns of k, gate_up mostly three of 128),
 // three or four such blocks a multiprocessor (256 weight rows, one block a multiprocessor: the same time; two warps on 128 weight
 // rows: a quarter slower).  Such a step streams every touched expert's weights once for a handful of rows: memory bounds it.
 // A second instance has tiles of 32 rows (two MMA row tiles a warp): with 16-row tiles the experts that got 17 rows or more take a
@@ -13,6 +13,8 @@
 //   down     the weight rows are output columns; a row's result is multiplied by its pair's routing weight
 //            and written as float32 to the pair's row (summed over a token's choices by the combine kernel).
 // Rows past a tile's end and columns past the matrices' edges are zero-filled in shared memory.
+#include <cmath>
+
 #include "attention_decode.cuh"
 #include "common.cuh"
 #include "moe.cuh"
@@ -26,11 +28,10 @@ struct MoeMmaShape {
   static constexpr int BM = 16 * MT * WM, BN = 8 * NT * WN, LD = BK + 8, THREADS = 32 * WM * WN;
   static constexpr size_t SMEM = (size_t)STAGES * (BM + BN) * LD * sizeof(__nv_bfloat16);
 };
-// 16 rows x 64 weight rows: single tokens.  gate_up has three stages of 128 columns: whole 256-byte runs of a weight row a
-// stage and half the barriers, three blocks a multiprocessor (16 experts of 2,048 x 2,048, us, 4 stages of 64 / 3 of 128: one
-// token 25.7 / 19.8, 8 tokens 50.2 / 38.8, 24 tokens 52.2 / 52.9 (in a decode step 56 / 57); of 3,584 x 4,096, 24 tokens: 172.6 / 152.7; 64 experts of
-// 1,408 x 2,048, 32 tokens: 123.2 / 112.5).  down, with half the blocks, keeps four blocks a multiprocessor, which hold a
-// batch's tiles at once (24 tokens: 27.5 / 34.0; of 2,048 x 3,584: 86.2 / 91.6).
+// 16 rows x 64 weight rows: single tokens.  gate_up has three stages of 128 columns where `moe_long_stages` says so: whole 256-byte
+// runs of a weight row a stage and half the barriers, three blocks a multiprocessor.  down, with half the blocks, keeps four blocks
+// a multiprocessor, which hold a batch's tiles at once (24 tokens, 16 experts of 2,048 x 2,048: 27.5 us, in three stages 34.0; of
+// 2,048 x 3,584: 86.2 / 91.6).
 using MoeMmaSmall = MoeMmaShape<1, 2, 1, 4, 64, 4>;
 using MoeMmaMedium = MoeMmaShape<2, 2, 1, 4, 64, 4>;  // 32 rows x 64 weight rows
 using MoeMmaWide = MoeMmaShape<2, 8, 4, 2, 64, 3>;    // 128 rows x 128 weight rows
@@ -187,11 +188,24 @@ int launch_moe_mma(const MoeProductArgs& a, int max_tiles, cudaStream_t stream) 
   return 0;
 }
 
+// Whether gate_up's 16-row tiles run in three stages of 128 columns.  Their three blocks a multiprocessor are each the faster, but
+// where the blocks of the experts that a step is likely to touch fit the device in one wave fewer at four a multiprocessor, those
+// win (16 experts of 2,048 x 2,048, top 4, us, four stages of 64 / three of 128: one token 25.1 / 18.9, 3 tokens 29.5 / 35.6, 6
+// tokens 50.5 / 39.0, 24 tokens 52.1 / 53.8; of 3,584 x 4,096: one token 49.8 / 55.4, 2 tokens 95 / 72); beyond two waves of those
+// the waves no longer show (24 tokens 172 / 156), and k of less than two long stages leaves one half empty (64: 3.0 / 3.2).
+inline bool moe_long_stages(const MoeProductArgs& a, int n_pairs, int n_experts) {
+  const double touched = n_experts * (1.0 - pow(1.0 - (double)a.top / n_experts, (double)n_pairs / a.top));
+  const double blocks = rint(touched + n_pairs / 160.0) * ((a.n + 31) / 32);  // experts with more than 16 rows take a second tile
+  const double sm = mll_sm_count();
+  return a.k >= 256 && (blocks > 8 * sm || ceil(blocks / (3 * sm)) <= ceil(blocks / (4 * sm)));
+}
+
 template <int KIND>
-int launch_moe_mma_rows(const MoeProductArgs& a, int max_tiles, int tile_rows, cudaStream_t stream) {
+int launch_moe_mma_rows(const MoeProductArgs& a, int max_tiles, int tile_rows, int n_pairs, int n_experts, cudaStream_t stream) {
   if (tile_rows == MoeMmaSmall::BM) {
-    if constexpr (KIND == 1) return launch_moe_mma<KIND, 1, 2, 1, 4, 128, 3>(a, max_tiles, stream);
-    else return launch_moe_mma<KIND, 1, 2, 1, 4, 64, 4>(a, max_tiles, stream);
+    if (KIND == 1 && a.top <= n_experts && moe_long_stages(a, n_pairs, n_experts))
+      return launch_moe_mma<KIND, 1, 2, 1, 4, KIND == 1 ? 128 : 64, KIND == 1 ? 3 : 4>(a, max_tiles, stream);
+    return launch_moe_mma<KIND, 1, 2, 1, 4, 64, 4>(a, max_tiles, stream);
   }
   if (tile_rows == MoeMmaMedium::BM) return launch_moe_mma<KIND, 2, 2, 1, 4, 64, 4>(a, max_tiles, stream);
   if (tile_rows == MoeMmaWide::BM) return launch_moe_mma<KIND, 2, 8, 4, 2, 64, 3>(a, max_tiles, stream);
@@ -227,8 +241,8 @@ MLL_API int mll_moe_gate_up_mma(const void* h, const void* w, void* act, void* r
                 "moe gate_up (tc5): operands must be 16-byte aligned");
     return mll_moe_gate_up_tc5(h, rows, w, act, a.plan, max_tiles, n_pairs, n_experts, width, inter, top, form, stream);
   }
-  if (form == 1) return mll::launch_moe_mma_rows<2>(a, max_tiles, tile_rows, stream);
-  return mll::launch_moe_mma_rows<1>(a, max_tiles, tile_rows, stream);
+  if (form == 1) return mll::launch_moe_mma_rows<2>(a, max_tiles, tile_rows, n_pairs, n_experts, stream);
+  return mll::launch_moe_mma_rows<1>(a, max_tiles, tile_rows, n_pairs, n_experts, stream);
 }
 
 MLL_API int mll_moe_down_mma(const void* act, const void* w, float* y, const float* pair_weight, const int* order,
@@ -243,5 +257,5 @@ MLL_API int mll_moe_down_mma(const void* act, const void* w, float* y, const flo
     MLL_REQUIRE(((uintptr_t)act | (uintptr_t)w | (uintptr_t)y) % 16 == 0, "moe down (tc5): operands must be 16-byte aligned");
     return mll_moe_down_tc5(act, w, y, pair_weight, a.plan, max_tiles, n_pairs, n_experts, inter, width, top, stream);
   }
-  return mll::launch_moe_mma_rows<0>(a, max_tiles, tile_rows, stream);
+  return mll::launch_moe_mma_rows<0>(a, max_tiles, tile_rows, n_pairs, n_experts, stream);
 }
