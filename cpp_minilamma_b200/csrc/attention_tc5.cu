@@ -76,7 +76,11 @@ struct PrefillTc5Args {
   int keep_first;            // with a window: keys at positions below this stay visible
   float scale_over_cap;      // scale / cap, and cap / scale: a raw score s becomes (cap / scale) tanh(s scale / cap),
   float cap_over_scale;      // which the scale then turns into cap * tanh(..); both 0 without a cap
-  static constexpr bool GATED = false;
+  static constexpr bool GATED = false, MIXED = false;
+};
+// The same with every other pair of exponentials on the FMA pipe (see `mixed_pays`)
+struct PrefillTc5MixedArgs : PrefillTc5Args {
+  static constexpr bool MIXED = true;
 };
 // The same for heads with a gate each.  A type of its own: the kernel without gates then compiles to what it was (the two
 // more parameters alone moved its register allocation: 63 -> 67 us for 2,048 tokens of 32 heads of 128).
@@ -219,6 +223,28 @@ __device__ __forceinline__ float a_max3(float a, float b, float c) {
   asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
   return d;
 }
+// 2^x for both halves of x on the FMA pipe: x = n + f with n = round(x) (the magic-number add leaves n in the low mantissa bits of t),
+// 2^f on [-0.5, 0.5] by a quartic whose relative error is below 2.7e-6 (least maximum, fitted for this; P is rounded to 8 bits
+// of mantissa afterwards), and n added to the exponent bits.  x is clamped at -126 (a masked score is -infinity; 2^-126 is
+// nothing against a row's largest term, which is 1 or more).
+__device__ __forceinline__ void a_exp2_pair_fma(a_f32x2 x, float& p0, float& p1) {
+  float x0, x1;
+  a_unpack2(x, x0, x1);
+  x = a_pack2(fmaxf(x0, -126.f), fmaxf(x1, -126.f));
+  const a_f32x2 t = a_add2(x, a_pack2(12582912.f, 12582912.f));
+  const a_f32x2 n = a_add2(t, a_pack2(-12582912.f, -12582912.f));
+  const a_f32x2 f = a_fma2(n, a_pack2(-1.f, -1.f), x);
+  a_f32x2 p = a_fma2(f, a_pack2(0.00957010221f, 0.00957010221f), a_pack2(0.0559178628f, 0.0559178628f));
+  p = a_fma2(p, f, a_pack2(0.240247443f, 0.240247443f));
+  p = a_fma2(p, f, a_pack2(0.693121791f, 0.693121791f));
+  p = a_fma2(p, f, a_pack2(0.999999285f, 0.999999285f));
+  float t0, t1, q0, q1;
+  a_unpack2(t, t0, t1);
+  a_unpack2(p, q0, q1);
+  p0 = __int_as_float(__float_as_int(q0) + (__float_as_int(t0) << 23));
+  p1 = __int_as_float(__float_as_int(q1) + (__float_as_int(t1) << 23));
+}
+
 // 32 consecutive 32-bit columns of this thread's lane, written from registers
 __device__ __forceinline__ void a_tmem_st32(unsigned addr, const unsigned* r) {
   asm volatile(
@@ -511,20 +537,23 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_c
       if (moved && i == 0) l_run *= a_exp2(m_used - mx);  // nothing in O yet; the sink's share of the sum, if any
       if (moved) m_used = mx;
       const float shift = m_used > -INFINITY ? m_used : 0.f;  // a fully masked row stays at zero weight
-      // p = 2^(s * scale - shift), two columns per instruction, the exponentials on the special-function unit.  Every other
-      // pair's on the FMA pipe instead (a cubic, a dozen instructions a pair) was the slower form: two softmax warps a
-      // scheduler live by the length of their own instruction streams, with every pipe less than half busy.  8,192 tokens, 32
-      // heads: 567 us with half of the pairs on the FMA pipe, 534 with a quarter, 518 with none at head size 128; 482 and 472
-      // at 64; 2,048 tokens at 128 64.7 and 60.6.
+      // p = 2^(s * scale - shift), two columns per instruction, the exponentials on the special-function unit or (MIXED) those of
+      // every other pair on the FMA pipe
       const a_f32x2 scale2 = a_pack2(a.scale_log2, a.scale_log2), shift2 = a_pack2(-shift, -shift);
       a_f32x2 sum2[2] = {a_pack2(0.f, 0.f), a_pack2(0.f, 0.f)};
       unsigned packed[MLL_PAGE / 2];
 #pragma unroll
       for (int c = 0; c < MLL_PAGE; c += 2) {
         const a_f32x2 x = a_fma2(a_pack2(s[c], s[c + 1]), scale2, shift2);
-        float x0, x1;
-        a_unpack2(x, x0, x1);
-        const float p0 = a_exp2(x0), p1 = a_exp2(x1);
+        float p0, p1;
+        if (Args::MIXED && ((c >> 1) & 1)) {
+          a_exp2_pair_fma(x, p0, p1);
+        } else {
+          float x0, x1;
+          a_unpack2(x, x0, x1);
+          p0 = a_exp2(x0);
+          p1 = a_exp2(x1);
+        }
         sum2[(c >> 2) & 1] = a_add2(sum2[(c >> 2) & 1], a_pack2(p0, p1));
         __nv_bfloat162 pair = __floats2bfloat162_rn(p0, p1);
         packed[c >> 1] = *reinterpret_cast<unsigned*>(&pair);
@@ -612,11 +641,26 @@ int launch_prefill_tc5_as(const CUtensorMap& qmap, const CUtensorMap& kmap, cons
   return 0;
 }
 
+// Where every other pair of exponentials belongs on the FMA pipe.  Two softmax warps a scheduler live by the length of their own
+// instruction streams, with every pipe less than half busy, so all on the special-function unit is the shorter way as a rule
+// (8,192 tokens, 32 heads of 128: 567 us mixed, 518 not).  Capped scores put a tanh a score on the same unit, and there the two share
+// the work better (1,024 tokens, 64 heads of 64: 53.0 us mixed, 57.5 not; 2,048 tokens, 32 heads of 128 87.7 and 93.0).  So they do
+// at head size 64 while the blocks all run at once, four warps or eight a multiprocessor (2,048 tokens, 4 heads: 31.0 and 32.9; 32
+// heads, 512 blocks: 84 and 82).
+inline bool mixed_pays(const PrefillTc5Args& a, int d, int dv, int n_tiles) {
+  if (a.cap_over_scale > 0.f) return true;
+  return d == 64 && dv == 64 && (long long)n_tiles * a.n_heads <= 2 * mll_sm_count();
+}
+
 template <int D, int DV>
 int launch_prefill_tc5(const CUtensorMap& qmap, const CUtensorMap& kmap, const CUtensorMap& vmap,
                        const PrefillTc5GatedArgs& a, int n_tiles, cudaStream_t stream) {
-  return a.gate ? launch_prefill_tc5_as<D, DV, PrefillTc5GatedArgs>(qmap, kmap, vmap, a, n_tiles, stream)
-                : launch_prefill_tc5_as<D, DV, PrefillTc5Args>(qmap, kmap, vmap, a, n_tiles, stream);
+  if (a.gate) return launch_prefill_tc5_as<D, DV, PrefillTc5GatedArgs>(qmap, kmap, vmap, a, n_tiles, stream);
+  if (mixed_pays(a, D, DV, n_tiles)) {
+    const PrefillTc5MixedArgs mixed{static_cast<const PrefillTc5Args&>(a)};
+    return launch_prefill_tc5_as<D, DV, PrefillTc5MixedArgs>(qmap, kmap, vmap, mixed, n_tiles, stream);
+  }
+  return launch_prefill_tc5_as<D, DV, PrefillTc5Args>(qmap, kmap, vmap, a, n_tiles, stream);
 }
 
 }  // namespace mll
