@@ -1,6 +1,6 @@
-"""Prompt attention at head size 64, which walks two pages a step: walks of one, two and an odd number of pages, tiles that end
-inside them, and every mask the kernel knows, over contexts whose last page is full, nearly full and nearly empty.  The cache
-holds not-a-numbers wherever no sequence has a position.  Against float64 of the same bfloat16 values."""
+"""The tcgen05 prompt attention at its two head sizes: walks of one, two and an odd number of pages, tiles that end inside them,
+and every mask the kernel knows, over contexts whose last page is full, nearly full and nearly empty.  The cache holds
+not-a-numbers wherever no sequence has a position.  Against float64 of the same bfloat16 values."""
 import pytest
 import torch
 
@@ -12,9 +12,10 @@ DEV = torch.device("cuda:0")
                                    {"chunk": 128}, {"softcap": 3.0}, {"sink": True}, {"sink_values": True}, {"gate": True},
                                    {"window": 90, "softcap": 2.0, "sink": True}])
 @pytest.mark.parametrize("H,G", [(4, 2), (3, 1)])
-def test_two_pages_a_step(masks, H, G):
+@pytest.mark.parametrize("d", [64, 128])
+def test_masks_and_partial_pages(masks, H, G, d):
     from cpp_minilamma_b200.csrc import kernels as K
-    d, PAGE = 64, 64
+    PAGE = 64
     gen = torch.Generator(device=DEV).manual_seed(H + len(masks))
     draw = lambda *shape: torch.randn(shape, generator=gen, device=DEV)
     lens = [1, 63, 64, 65, 128, 129, 200, 3, 300, 1, 130]
