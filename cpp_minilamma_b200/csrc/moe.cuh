@@ -30,4 +30,4 @@ int mll_moe_tc5_rows();
 int mll_moe_gate_up_tc5(const void* h, void* rows, const void* w, void* act, const mll::MoePlan& plan, int max_tiles,
                         int n_pairs, int n_experts, int width, int inter, int top, int form, cudaStream_t stream);
 int mll_moe_down_tc5(const void* act, const void* w, float* y, const float* pair_weight, const mll::MoePlan& plan,
-                     int max_tiles, int n_pairs, int n_experts, int inter, int width, int top, cudaStream_t stream);
+                     int max_tiles, int n_pairs, int n_experts, int inter, int width, cudaStream_t stream);

@@ -255,7 +255,7 @@ MLL_API int mll_moe_down_mma(const void* act, const void* w, float* y, const flo
                                                              (int*)tile_row0, (int*)n_tiles}, inter, width, top};
   if (tile_rows == mll_moe_tc5_rows()) {
     MLL_REQUIRE(((uintptr_t)act | (uintptr_t)w | (uintptr_t)y) % 16 == 0, "moe down (tc5): operands must be 16-byte aligned");
-    return mll_moe_down_tc5(act, w, y, pair_weight, a.plan, max_tiles, n_pairs, n_experts, inter, width, top, stream);
+    return mll_moe_down_tc5(act, w, y, pair_weight, a.plan, max_tiles, n_pairs, n_experts, inter, width, stream);
   }
   return mll::launch_moe_mma_rows<0>(a, max_tiles, tile_rows, n_pairs, n_experts, stream);
 }

@@ -45,7 +45,7 @@ struct MoeTc5Args {
   void* out;
   const float* pair_weight;  // [pairs] (down)
   MoePlan plan;
-  int k, n, top;
+  int k, n;
   int* error;  // raised by a bounded wait that ran out: the flag of the tcgen05 products (device_error.h)
 };
 
@@ -339,13 +339,13 @@ int mll_moe_gate_up_tc5(const void* h, void* rows, const void* w, void* act, con
   MLL_LAUNCH((mll::moe_gather_kernel), (int)blocks, 256, 0, stream, (const uint4*)h, (uint4*)rows, (const int*)plan.order, top,
              width / 8, total);
   MLL_LAUNCH_CHECK();
-  mll::MoeTc5Args a{act, nullptr, plan, width, inter, top, nullptr};
+  mll::MoeTc5Args a{act, nullptr, plan, width, inter, nullptr};
   if (form == 1) return mll::launch_moe_tc5<2>(rows, n_pairs, w, (long long)n_experts * inter, a, max_tiles, stream);
   return mll::launch_moe_tc5<1>(rows, n_pairs, w, (long long)n_experts * 2 * inter, a, max_tiles, stream);
 }
 
 int mll_moe_down_tc5(const void* act, const void* w, float* y, const float* pair_weight, const mll::MoePlan& plan,
-                     int max_tiles, int n_pairs, int n_experts, int inter, int width, int top, cudaStream_t stream) {
-  mll::MoeTc5Args a{y, pair_weight, plan, inter, width, top, nullptr};
+                     int max_tiles, int n_pairs, int n_experts, int inter, int width, cudaStream_t stream) {
+  mll::MoeTc5Args a{y, pair_weight, plan, inter, width, nullptr};
   return mll::launch_moe_tc5<0>(act, n_pairs, w, (long long)n_experts * width, a, max_tiles, stream);
 }
