@@ -1546,8 +1546,9 @@ def state_chunks(q, k, v, state, out, scratch, run_seq, run_row0, seq_run0, seq_
                  token_decay: Optional[torch.Tensor] = None, beta: Optional[torch.Tensor] = None,
                  channel_decay: Optional[torch.Tensor] = None) -> None:
     """As `state_scan` for one decay per head (`head_decay` [H]) or per token and head (`token_decay` [T, H]; with `beta` the
-    delta rule), or the delta rule with a decay per key channel (`channel_decay` [T, H * d] and `beta`), a run of up to STATE_RUN tokens at a time: run_seq, run_row0 (int32 [runs]) list every
-    sequence's runs one after another, seq_run0 (int32 [sequences]) its first.  Decays lie in [0, 1]."""
+    delta rule), or the delta rule with a decay per key channel (`channel_decay` [T, H * d] and `beta`), a run of up to STATE_RUN
+    tokens at a time: run_seq, run_row0 (int32 [runs]) list every sequence's runs one after another, seq_run0 (int32 [sequences])
+    its first.  Decays lie in [0, 1]."""
     n = q.shape[0]
     for name, t, width in (("q", q, n_kv_heads * d), ("k", k, n_kv_heads * d), ("v", v, n_heads * dv),
                            ("out", out, n_heads * dv), ("token decay", token_decay, n_heads), ("beta", beta, n_heads),

@@ -199,9 +199,9 @@ MLL_API int mll_linear_f32_supported(int M, int N, int K, int epilogue) {
 }
 
 // Whether it is the faster way for a product without an epilogue (us, the library / here): short rows of a tall matrix are not what
-// the kernel is laid out for (16,384 x 64, 8 rows 5.1 / 7.5; 6,144 x 256 6.9 / 4.3), from 9 rows on no short rows are (64 x 64,
-// 16 rows 2.6 / 3.3; 512 x 128 2.9 / 3.0; 1,024 x 128 4.9 / 3.2) and the tallest matrices need long ones (16,384 x 1,024, 16 rows
-// 36.8 / 39.8; x 2,048 70 / 66; 12,288 x 512 29 / 27).
+// the kernel is laid out for (8 rows, 16,384 x 64 5.1 / 7.5; 6,144 x 256 9.3 / 5.4), from 9 rows on no short rows are (16 rows, 64 x
+// 64 2.6 / 3.3; 1,024 x 128 4.7 / 3.0) and the tallest matrices need long ones (16 rows, 12,288 x 512 19.6 / 17.8; 16,384 x 1,024
+// 36.8 / 39.8; x 2,048 70 / 66).
 MLL_API int mll_linear_f32_pays(int M, int N, int K) {
   if (M <= 4) return 1;
   if (M <= 8) return K >= 256 || N <= 4096;

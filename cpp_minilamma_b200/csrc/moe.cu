@@ -18,7 +18,7 @@
 // The products here are the plain form (a thread per output column, the tile's rows in shared memory, float32
 // accumulation in k order); every weight of an expert is read once per tile, which is what a decode step needs.
 // They serve float32 and sizes whose rows are no whole 16-byte words; bfloat16 steps take the tensor-core kernels of
-// moe_mma.cu for the two products.
+// moe_mma.cu and moe_tc5.cu for the two products.
 #include "common.cuh"
 #include "moe.cuh"
 

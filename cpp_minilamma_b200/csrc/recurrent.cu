@@ -764,9 +764,9 @@ int launch_scan(const ScanArgs& args, int n_seqs, cudaStream_t stream) {
 // for before anything else; a row of the tile is 256 consecutive bytes.  The sums over the rows go through shared memory,
 // once a token: with the delta rule both products are formed from the decayed state as it was, S' = diag(g) S, and
 //   u = beta (v - S'^T k),   o = S'^T q + u (k . q),   S <- S' + k u^T.
-// 16 sequences of 16 heads of 128 x 128, the delta rule (16.8 MB in and out, 5.1 us at the copy peak): 22.3 us on the general
-// scan, 10.1 here; 8 heads of 128 x 256, one decay per head: 19.0 and 8.4; 64 such sequences (20.6 us): 38.9 and 32.5, 36.4
-// and 24.9; one sequence 4.0 and 3.9.
+// 16 sequences of 16 heads of 128 x 128, the delta rule (16.8 MB in and as much out, 5.1 us at the copy peak): 23.2 us on the general
+// scan, 10.2 here; of 128 x 256, one decay per head: 20.9 and 14.8; 64 sequences of 32 heads (134 MB and 268 MB each way, 41 and 82
+// us): 74 and 54, 140 and 92; one sequence of 8 heads of 128 x 256, one decay per head: 5.4 and 3.3.
 constexpr int STEP_COLS = 64, STEP_GROUPS = 16;  // columns a block; groups of rows
 
 __device__ __forceinline__ float step_sum(const float (&x)[STEP_GROUPS / 2]) {

@@ -26,7 +26,7 @@
 //   * state_chunk_scan     the delta rule: a block per (16 columns of the state, head, sequence) walks the runs; the columns
 //                          of S in registers and in shared memory, the runs' matrices through cp.async, W and Q of the
 //                          next run on their way while this one is worked on
-// 2,047 tokens of 16 heads of 128 x 128 with a decay per key channel: 718 us token by token, 238 here (inputs 63, scan 175).
+// 2,047 tokens of 16 heads of 128 x 128 with a decay per key channel: 720 us token by token, 253 here.
 // All products are float32 FMAs: the recurrence stays exact to float32, which bfloat16 tensor-core products would not be,
 // and products cut into enough bfloat16 terms to be exact take as long on the tensor cores.
 #include "common.cuh"
