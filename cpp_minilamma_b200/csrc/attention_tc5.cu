@@ -644,19 +644,16 @@ int launch_prefill_tc5_as(const CUtensorMap& qmap, const CUtensorMap& kmap, cons
 // Where every other pair of exponentials belongs on the FMA pipe.  Two softmax warps a scheduler live by the length of their own
 // instruction streams, with every pipe less than half busy, so all on the special-function unit is the shorter way as a rule
 // (8,192 tokens, 32 heads of 128: 567 us mixed, 518 not).  Capped scores put a tanh a score on the same unit, and there the two share
-// the work better (1,024 tokens, 64 heads of 64: 53.0 us mixed, 57.5 not; 2,048 tokens, 32 heads of 128 87.7 and 93.0).  So they do
-// at head size 64 while the blocks all run at once, four warps or eight a multiprocessor (2,048 tokens, 4 heads: 31.0 and 32.9; 32
-// heads, 512 blocks: 84 and 82).
-inline bool mixed_pays(const PrefillTc5Args& a, int d, int dv, int n_tiles) {
-  if (a.cap_over_scale > 0.f) return true;
-  return d == 64 && dv == 64 && (long long)n_tiles * a.n_heads <= 2 * mll_sm_count();
-}
+// the work better (1,024 tokens, 64 heads of 64: 53.0 us mixed, 57.5 not; 2,048 tokens, 32 heads of 128 87.7 and 93.0).  (At head
+// size 64 so they do, by up to 6 %, while few blocks walk many pages - 2,048 tokens, 4 heads 31.0 and 32.9 - but not in short prompts,
+// whose grids look the same; the more exact form stays.)
+inline bool mixed_pays(const PrefillTc5Args& a) { return a.cap_over_scale > 0.f; }
 
 template <int D, int DV>
 int launch_prefill_tc5(const CUtensorMap& qmap, const CUtensorMap& kmap, const CUtensorMap& vmap,
                        const PrefillTc5GatedArgs& a, int n_tiles, cudaStream_t stream) {
   if (a.gate) return launch_prefill_tc5_as<D, DV, PrefillTc5GatedArgs>(qmap, kmap, vmap, a, n_tiles, stream);
-  if (mixed_pays(a, D, DV, n_tiles)) {
+  if (mixed_pays(a)) {
     const PrefillTc5MixedArgs mixed{static_cast<const PrefillTc5Args&>(a)};
     return launch_prefill_tc5_as<D, DV, PrefillTc5MixedArgs>(qmap, kmap, vmap, mixed, n_tiles, stream);
   }
