@@ -329,16 +329,19 @@ def linear_small(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor],
                                         _ptr(out_sumsq), ctypes.c_int(out_stride), _stream()), "linear_small")
 
 
+def _linear_f32_operands(x: torch.Tensor, w: torch.Tensor) -> bool:
+    return (SMALL_LINEAR != "none" and x.dtype == torch.float32 and w.dtype == torch.float32 and x.dim() == 2
+            and x.is_contiguous() and w.is_contiguous() and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+
+
 def linear_f32_supported(x: torch.Tensor, w: torch.Tensor, epilogue: int = EPI_F32) -> bool:
     """Whether `linear_f32` takes x . w^T: float32, the few rows of a decode step, rows on 16-byte boundaries."""
-    return (SMALL_LINEAR != "none" and x.dtype == torch.float32 and w.dtype == torch.float32 and x.dim() == 2
-            and x.is_contiguous() and w.is_contiguous() and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
-            and bool(lib().mll_linear_f32_supported(x.shape[0], w.shape[0], w.shape[1], epilogue)))
+    return _linear_f32_operands(x, w) and bool(lib().mll_linear_f32_supported(x.shape[0], w.shape[0], w.shape[1], epilogue))
 
 
 def linear_f32_pays(x: torch.Tensor, w: torch.Tensor) -> bool:
     """Whether `linear_f32` takes x . w^T and is faster than the library's product."""
-    return linear_f32_supported(x, w) and bool(lib().mll_linear_f32_pays(x.shape[0], w.shape[0], w.shape[1]))
+    return _linear_f32_operands(x, w) and bool(lib().mll_linear_f32_pays(x.shape[0], w.shape[0], w.shape[1]))
 
 
 def linear_f32(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor, epilogue: int = EPI_F32,

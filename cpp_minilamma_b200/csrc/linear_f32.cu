@@ -198,11 +198,12 @@ MLL_API int mll_linear_f32_supported(int M, int N, int K, int epilogue) {
   return (epilogue == mll::FEPI_SWIGLU || epilogue == mll::FEPI_GEGLU) && N % 16 == 0;
 }
 
-// Whether it is the faster way for a product without an epilogue (us, the library / here): short rows of a tall matrix are not what
+// Whether it takes this problem and is the faster way for a product without an epilogue (us, the library / here): short rows of a tall matrix are not what
 // the kernel is laid out for (8 rows, 16,384 x 64 5.1 / 7.5; 6,144 x 256 9.3 / 5.4), from 9 rows on no short rows are (16 rows, 64 x
 // 64 2.6 / 3.3; 1,024 x 128 4.7 / 3.0) and the tallest matrices need long ones (16 rows, 12,288 x 512 19.6 / 17.8; 16,384 x 1,024
 // 36.8 / 39.8; x 2,048 70 / 66).
 MLL_API int mll_linear_f32_pays(int M, int N, int K) {
+  if (!mll_linear_f32_supported(M, N, K, mll::FEPI_F32)) return 0;
   if (M <= 4) return 1;
   if (M <= 8) return K >= 256 || N <= 4096;
   return K >= (N <= 4096 ? 128 : 256) && (N <= 12288 || K >= 2048);

@@ -763,7 +763,8 @@ int launch_scan(const ScanArgs& args, int n_seqs, cudaStream_t stream) {
 // columns of one head's state, a thread four neighbouring columns (16 bytes) of ROWS neighbouring rows, all of which it asks
 // for before anything else; a row of the tile is 256 consecutive bytes.  The sums over the rows go through shared memory,
 // once a token: with the delta rule both products are formed from the decayed state as it was, S' = diag(g) S, and
-//   u = beta (v - S'^T k),   o = S'^T q + u (k . q),   S <- S' + k u^T.
+//   u = beta (v - S'^T k),   o = S'^T q + u (k . q),   S <- S' + k u^T
+// (one decay per head is left out of the sums and meets their results).
 // 16 sequences of 16 heads of 128 x 128, the delta rule (16.8 MB in and as much out, 5.1 us at the copy peak): 23.2 us on the general
 // scan, 10.2 here; of 128 x 256, one decay per head: 20.9 and 14.8; 64 sequences of 32 heads (134 MB and 268 MB each way, 41 and 82
 // us): 74 and 54, 140 and 92; one sequence of 8 heads of 128 x 256, one decay per head: 5.4 and 3.3.
@@ -805,7 +806,7 @@ __global__ void __launch_bounds__(256, step_blocks(ROWS, MODE)) state_step_kerne
     if (col < dv) v = *reinterpret_cast<const float4*>(a.v + ((size_t)t * H + h) * dv + col);
     const float beta = DELTA ? a.beta[(size_t)t * H + h] : 1.f;
     const float decay = MODE == 0 ? a.head_decay[h] : MODE == 3 ? a.beta[(size_t)t * H + h] : MODE == 4 ? a.g[(size_t)t * H + h] : 1.f;
-    // no chain of additions is longer than four: with more rows they are taken two by two
+    // chains of four additions (eight at 16 rows): from eight rows on they are taken two by two
     float kv[ROWS], o[4] = {0.f, 0.f, 0.f, 0.f}, c[4] = {0.f, 0.f, 0.f, 0.f}, kq = 0.f;
     float held[5];  // the first of two rows' products: with q, and k with q
     float held_k[4];
