@@ -22,8 +22,8 @@ from pathlib import Path
 
 CSRC = Path(__file__).resolve().parent
 SOURCES = ["elementwise.cu", "norm.cu", "rope_cache.cu", "attention.cu", "sampling.cu",
-           "linear_f32.cu", "linear_small.cu", "linear_tma.cu", "linear_tc5.cu", "attention_mma.cu", "attention_mma_odd.cu",
-           "attention_mma_prefill.cu", "attention_tc5.cu", "attention_decode_tma.cu", "device_error.cu",
+           "linear_f32.cu", "linear_f32_tc5.cu", "linear_small.cu", "linear_tma.cu", "linear_tc5.cu", "attention_mma.cu",
+           "attention_mma_odd.cu", "attention_mma_prefill.cu", "attention_tc5.cu", "attention_decode_tma.cu", "device_error.cu",
            "attention_local.cu", "attention_local_mma.cu", "recurrent.cu", "latent.cu", "moe.cu", "moe_mma.cu", "moe_tc5.cu",
            "attention_mix.cu", "attention_mix_mma.cu", "rglru.cu", "state_chunk.cu"]
 HEADERS = ["common.cuh", "no_alloc.h", "tensor_map.h", "attention_decode.cuh", "attention_mma.cuh", "device_error.h", "moe.cuh",

@@ -362,6 +362,43 @@ def linear_f32(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], o
                                 ctypes.c_int(epilogue), ctypes.c_int(slices), _stream()), "linear_f32")
 
 
+LINEAR_F32_TC5_ROWS = 2048  # rows of x split at a time
+
+
+def linear_f32_tc5_pieces(rows: int, in_features: int):
+    """Shape of the bfloat16 scratch that `linear_f32_tc5` needs for `rows` rows."""
+    return (3, min(rows, LINEAR_F32_TC5_ROWS), -(-in_features // 8) * 8)
+
+
+def linear_f32_tc5_supported(x: torch.Tensor, w: torch.Tensor, epilogue: int = EPI_F32) -> bool:
+    """Whether `linear_f32_tc5` takes x . w^T: float32, rows on 16-byte boundaries."""
+    return _linear_f32_operands(x, w) and bool(lib().mll_linear_f32_tc5_supported(x.shape[0], w.shape[0], w.shape[1], epilogue))
+
+
+def linear_f32_tc5(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], pieces: torch.Tensor, out: torch.Tensor,
+                   epilogue: int = EPI_F32, cols: int = 0, ranks: int = 0) -> None:
+    """out = x . w^T (+ bias) in true float32 for many rows, on the tensor cores; epilogues as in `linear_f32`.  `pieces`:
+    scratch of the shape that `linear_f32_tc5_pieces` gives; `cols`, `ranks`: rows of x a block takes (a multiple of 16,
+    at most 256) and blocks that share K (1, 2, 4 or 8); 0: chosen."""
+    for t, name in ((x, "x"), (w, "w"), (out, "out")):
+        _need(t, "linear_f32_tc5 " + name, torch.float32, 2)
+    _need(pieces, "linear_f32_tc5 pieces", torch.bfloat16, 3)
+    (rows, k), n = x.shape, w.shape[0]
+    if w.shape[1] != k or tuple(out.shape) != (rows, n if epilogue == EPI_F32 else n // 2):
+        raise KernelError(f"linear_f32_tc5: x {tuple(x.shape)}, w {tuple(w.shape)} and out {tuple(out.shape)} do not fit")
+    if tuple(pieces.shape) != linear_f32_tc5_pieces(rows, k):
+        raise KernelError(f"linear_f32_tc5: pieces {tuple(pieces.shape)}, expected {linear_f32_tc5_pieces(rows, k)}")
+    if bias is not None:
+        _need(bias, "linear_f32_tc5 bias", torch.float32, 1)
+        if bias.shape[0] != n:
+            raise KernelError("linear_f32_tc5: bias length differs from the output width")
+    for at in range(0, rows, LINEAR_F32_TC5_ROWS):
+        here, there = x[at:at + LINEAR_F32_TC5_ROWS], out[at:at + LINEAR_F32_TC5_ROWS]
+        _check(lib().mll_linear_f32_tc5(_ptr(here), _ptr(w), _ptr(bias), _ptr(pieces), _ptr(there), ctypes.c_int(here.shape[0]),
+                                        ctypes.c_int(n), ctypes.c_int(k), ctypes.c_int(epilogue), ctypes.c_int(cols),
+                                        ctypes.c_int(ranks), _stream()), "linear_f32_tc5")
+
+
 def linear_tma_supported(rows: int, out_features: int, in_features: int, epilogue: int = EPI_BF16) -> bool:
     return bool(lib().mll_linear_tma_supported(rows, out_features, in_features, epilogue))
 

@@ -1,0 +1,519 @@
+// y[M, N] = x[M, K] . W[N, K]^T in true float32 for the many rows of a prompt, on the 5th-generation tensor cores.
+//
+// A float32 number is the exact sum of three bfloat16 numbers (its significand cut into 8 + 8 + 8 bits, every cut towards zero, so
+// that no piece can overflow): x = x0 + x1 + x2, w = w0 + w1 + w2.  Of the nine products of pieces the six largest are formed
+// (w0 x2, w2 x0, w1 x1, w0 x1, w1 x0, w0 x0); the three left out are below 2^-22 of the product.  A product of two pieces is exact in
+// float32, and what remains is the sum's rounding: the tensor cores cut their running sum after every step instead of rounding it,
+// which over a long K would cost more than a chain of float32 additions does.  So 32 columns of k are summed up in tensor memory,
+// the small products first, and then added to float32 registers.
+// Bound: the tensor pipe, at a sixth of its bfloat16 rate.
+//
+// A block forms 128 weight rows (the M operand) times up to 256 rows of x (the N operand) over a slice of K, 32 columns a stage:
+//   warp 12    loads the three pieces of x, split by a kernel in front (x is small and every column of blocks reads it again): boxes of
+//              [rows x 32] with the 64-byte swizzle into a ring of their own.
+//   warp 14    loads W as it is: boxes of [128 x 32] floats.
+//   warps 8-11 split W: 32 rows a warp, from its ring into that of its pieces, where the swizzle puts them.  (Loading W into
+//              registers a stage or two ahead instead of through a ring was bound by those loads' latency: the fence in front of the
+//              tensor cores' reads waits for them too, 2,000 to 3,000 clocks a stage.)
+//   warps 13, 15  issue the products, one thread each: twelve a stage, the even stages' into one half of tensor memory, the odd
+//              ones' into the other.
+//   warps 0-7  add a stage's sums to their registers: a thread has half of a row's.
+// K is split over the blocks of a cluster where tiles alone would leave multiprocessors idle; the blocks then add their shares
+// in rank order through distributed shared memory, so a result does not depend on the run.
+// Infinities: a piece of an infinite number is infinite or zero, and their products with other pieces may be NaN where the product of the
+// numbers is not.  So a sum that is not finite is formed again, as a chain of float32 operations over the numbers themselves.
+// Every wait is bounded; a thread whose wait runs out raises an error flag (mll_take_device_error), and the block ends.  No load uses
+// cluster multicast.
+//
+// The reference calls cublasSgemm with rows = 1 for every linear (src/cuda_matmul.cc:181-186).
+#include <cooperative_groups.h>
+#include <cuda.h>
+
+#include "common.cuh"
+#include "device_error.h"
+#include "tensor_map.h"
+
+namespace cg = cooperative_groups;
+
+namespace mll {
+
+enum : int { XEPI_F32 = 1, XEPI_SWIGLU = 2, XEPI_GEGLU = 4 };  // numbered as the bfloat16 kernels' epilogues
+constexpr int X_SUMMERS = 8;              // warps that add up sums: two warpgroups
+constexpr int X_SPLITTERS = 4;            // warps that split W: one warpgroup
+constexpr int X_LOAD_X_WARP = 12, X_MMA_WARP = 13, X_LOAD_W_WARP = 14;  // and X_MMA_WARP + 2
+constexpr int X_THREADS = 512;            // four warpgroups: 168 + 168 + 88 + 40 registers a thread of the 128 each at the start
+constexpr int X_ROWS = 128;               // weight rows of a block
+constexpr int X_KB = 32;                  // columns of k a stage: 64 bytes of a piece, one swizzle span
+constexpr int X_W_PIECE = X_ROWS * X_KB * 2;
+constexpr int X_RAW = X_ROWS * X_KB * 4;  // bytes of W a stage
+constexpr int X_MAX_STAGES = 8;
+constexpr int X_RINGS = 230144;           // shared memory for the rings
+constexpr long long X_WAIT_CLOCKS = 2ll << 30;
+
+struct LinearX3Args {
+  const float* x;     // [M, K]
+  const float* w;     // [N, K]
+  const float* bias;  // optional [N]
+  float* out;         // [M, N] (gated epilogues: [M, N / 2])
+  int M, N, K, epilogue;
+  int cols;           // rows of x a block takes, a multiple of 16
+  int m_tiles, blocks_per_rank;
+  int x_stages, w_stages, raw_stages;
+  int* error;
+};
+
+__device__ __forceinline__ unsigned x_smem(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ bool x_try(unsigned bar, unsigned parity) {
+  unsigned done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+  return done != 0;
+}
+__device__ __forceinline__ bool x_wait(unsigned bar, unsigned parity, volatile int* gave_up, int* error) {
+  if (x_try(bar, parity)) return true;
+  const long long began = clock64();
+  while (clock64() - began < X_WAIT_CLOCKS) {
+    if (x_try(bar, parity)) return true;
+    if (*gave_up) return false;
+  }
+  *gave_up = 1;
+  if (error) atomicExch(error, 1);
+  return false;
+}
+__device__ __forceinline__ void x_init(unsigned bar, unsigned count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
+}
+__device__ __forceinline__ void x_box(unsigned dst, const CUtensorMap* map, int c, int r, unsigned bar) {
+  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+               ::"r"(dst), "l"(map), "r"(c), "r"(r), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void x_arrive(unsigned bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void x_expect(unsigned bar, unsigned bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void x_cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ bool x_elect() {
+  unsigned one;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
+  return one != 0;
+}
+// K-major tile with rows of 64 bytes and the 64-byte swizzle: groups of 8 rows are 512 bytes apart
+__device__ __forceinline__ unsigned long long x_desc(unsigned addr) {
+  return (unsigned long long)((addr >> 4) & 0x3FFFu) | (1ull << 16) | ((unsigned long long)(512 >> 4) << 32) | (1ull << 46) |
+         (4ull << 61);
+}
+__device__ __forceinline__ void x_mma(unsigned d, unsigned a, unsigned b, unsigned idesc, unsigned accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(d), "l"(x_desc(a)), "l"(x_desc(b)), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void x_commit(unsigned bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void x_tmem_ld32(unsigned (&v)[32], unsigned addr) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
+        "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
+        "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+      : "r"(addr));
+}
+
+// two neighbouring floats -> their three pieces, each as a word of two bfloat16
+__device__ __forceinline__ void x_split(float a, float b, unsigned& p0, unsigned& p1, unsigned& p2) {
+  const unsigned ua = __float_as_uint(a), ub = __float_as_uint(b);
+  p0 = __byte_perm(ua, ub, 0x7632);
+  const float ra = a - __uint_as_float(ua & 0xFFFF0000u), rb = b - __uint_as_float(ub & 0xFFFF0000u);  // exact
+  const unsigned va = __float_as_uint(ra), vb = __float_as_uint(rb);
+  p1 = __byte_perm(va, vb, 0x7632);
+  p2 = __byte_perm(__float_as_uint(ra - __uint_as_float(va & 0xFFFF0000u)), __float_as_uint(rb - __uint_as_float(vb & 0xFFFF0000u)),
+                   0x7632);
+}
+
+// pieces[i] = piece i of x: [3][M][stride], columns from K to the stride (a multiple of 8) zero.  Bound by memory (4 bytes in,
+// 6 out a value).
+__global__ void split_f32_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ pieces, int M, int K, int stride) {
+  const int words = stride / 8;
+  const long long total = (long long)M * words, plane = (long long)M * stride;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
+    const int row = (int)(i / words), c = (int)(i % words) * 8;
+    const float* src = x + (size_t)row * K + c;
+    const float4 a = *reinterpret_cast<const float4*>(src);  // K is a multiple of 4
+    const float4 b = c + 4 < K ? *reinterpret_cast<const float4*>(src + 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+    uint4 p[3];
+    x_split(a.x, a.y, p[0].x, p[1].x, p[2].x);
+    x_split(a.z, a.w, p[0].y, p[1].y, p[2].y);
+    x_split(b.x, b.y, p[0].z, p[1].z, p[2].z);
+    x_split(b.z, b.w, p[0].w, p[1].w, p[2].w);
+#pragma unroll
+    for (int j = 0; j < 3; ++j) *reinterpret_cast<uint4*>(pieces + j * plane + (size_t)row * stride + c) = p[j];
+  }
+}
+
+// The product of a row of x and a row of W in float32 operations, for sums that are not finite.
+__device__ __noinline__ float x_chain(const float* x, const float* w, int K) {
+  float s = 0.f;
+  for (int k = 0; k < K; ++k) s = fmaf(x[k], w[k], s);
+  return s;
+}
+
+// Row m of the result for a warp of weight rows (lane: row n), all lanes present
+__device__ __forceinline__ void x_write(const LinearX3Args& a, float v, int m, int n) {
+  const bool in = m < a.M && n < a.N;
+  if (in && !isfinite(v)) v = x_chain(a.x + (size_t)m * a.K, a.w + (size_t)n * a.K, a.K);
+  if (a.epilogue == XEPI_F32) {
+    if (in) a.out[(size_t)m * a.N + n] = a.bias ? v + a.bias[n] : v;
+  } else {  // gate rows 0-7, up rows 8-15 of every 16
+    const float up = __shfl_down_sync(0xffffffffu, v, 8);
+    if (in && (n & 8) == 0)
+      a.out[(size_t)m * (a.N >> 1) + (n >> 4) * 8 + (n & 7)] =
+          gate_act_mul<false>(a.epilogue == XEPI_GEGLU ? GATE_ACT_GELU_TANH : GATE_ACT_SILU, v, up);
+  }
+}
+
+// COLS: most columns (rows of x) of a block that one of the two groups of summing warps holds sums of
+template <int COLS, bool CLUSTER>
+__global__ void __launch_bounds__(X_THREADS, 1) linear_f32_tc5_kernel(const __grid_constant__ CUtensorMap x_map,
+                                                                      const __grid_constant__ CUtensorMap w_map, LinearX3Args a) {
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* base = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  __shared__ __align__(8) unsigned long long bars[6 * X_MAX_STAGES + 4];
+  __shared__ unsigned tmem_slot;
+  __shared__ int gave_up_word;
+  volatile int* gave_up = &gave_up_word;
+  const unsigned x_full = x_smem(bars), x_empty = x_full + 8 * X_MAX_STAGES, w_full = x_empty + 8 * X_MAX_STAGES,
+                 w_empty = w_full + 8 * X_MAX_STAGES, raw_full = w_empty + 8 * X_MAX_STAGES, raw_empty = raw_full + 8 * X_MAX_STAGES,
+                 sums_full = raw_empty + 8 * X_MAX_STAGES, sums_empty = sums_full + 16;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int x_piece = a.cols * X_KB * 2;
+  const int w_at = 3 * x_piece * a.x_stages, raw_at = w_at + 3 * X_W_PIECE * a.w_stages;  // places of the rings
+  int rank = 0, ranks = 1;
+  if (CLUSTER) {
+    rank = (int)cg::this_cluster().block_rank();
+    ranks = (int)cg::this_cluster().num_blocks();
+  }
+  const int tile = blockIdx.x / ranks;
+  const int m0 = (tile % a.m_tiles) * a.cols, n0 = (tile / a.m_tiles) * X_ROWS;
+  const int k_blocks = (a.K + X_KB - 1) / X_KB;
+  const int first = rank * a.blocks_per_rank, mine = max(0, min(k_blocks - first, a.blocks_per_rank));
+
+  if (tid == 0) {
+    for (int s = 0; s < X_MAX_STAGES; ++s) {
+      x_init(x_full + 8 * s, 1);
+      x_init(x_empty + 8 * s, 1);
+      x_init(w_full + 8 * s, X_SPLITTERS);
+      x_init(w_empty + 8 * s, 1);
+      x_init(raw_full + 8 * s, 1);
+      x_init(raw_empty + 8 * s, X_SPLITTERS);
+    }
+    for (int b = 0; b < 2; ++b) {
+      x_init(sums_full + 8 * b, 1);
+      x_init(sums_empty + 8 * b, X_SUMMERS);
+    }
+    gave_up_word = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == X_MMA_WARP) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(x_smem(&tmem_slot)), "r"(512u));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const unsigned tmem = tmem_slot;
+
+  if (warp < X_SUMMERS) {
+    // ---- sums out of tensor memory ------------------------------------------------------------------------------ //
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 168;");
+    const int group = warp >> 2;  // which half of the columns
+    const int half = a.cols >> 1;
+    float acc[COLS];
+#pragma unroll
+    for (int i = 0; i < COLS; ++i) acc[i] = 0.f;
+    const unsigned lanes = tmem + ((unsigned)((warp & 3) * 32) << 16) + (unsigned)(group * half);
+    for (int it = 0; it < mine; ++it) {
+      const int b = it & 1;
+      const bool ok = x_wait(sums_full + 8 * b, (it >> 1) & 1, gave_up, a.error);
+      if (!__all_sync(0xffffffffu, ok)) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+      for (int c = 0; c < COLS; c += 32) {
+        if (c < half) {  // columns beyond the half hold other sums, which are not written
+          unsigned t[32];
+          x_tmem_ld32(t, lanes + b * 256 + c);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int i = 0; i < 32; ++i) acc[c + i] += __uint_as_float(t[i]);
+        }
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) x_arrive(sums_empty + 8 * b);
+    }
+    const int r0 = (warp & 3) * 32 + lane;
+    const int wide = X_ROWS + 4;  // words of a column of the tile in shared memory
+    float* part = reinterpret_cast<float*>(base);
+    if (!*gave_up) {
+      if (CLUSTER) {
+        // the block's share into its rings (all copies into them have arrived: their products are through), column by column
+#pragma unroll
+        for (int c = 0; c < COLS; ++c)
+          if (c < half) part[(size_t)(group * half + c) * wide + r0] = acc[c];
+      } else {
+#pragma unroll
+        for (int c = 0; c < COLS; ++c)
+          if (c < half) x_write(a, acc[c], m0 + group * half + c, n0 + r0);
+      }
+    }
+    if (CLUSTER) {
+      x_cluster_sync();
+      const int per = (a.cols + ranks - 1) / ranks, from = rank * per, to = min(a.cols, from + per);
+      for (int i = from * 4 + warp; i < to * 4; i += X_SUMMERS) {
+        const int c = i >> 2, r = (i & 3) * 32 + lane;
+        float s = 0.f;
+        for (int j = 0; j < ranks; ++j) s += cg::this_cluster().map_shared_rank(part, j)[(size_t)c * wide + r];
+        x_write(a, s, m0 + c, n0 + r);
+      }
+      x_cluster_sync();
+    }
+  } else if (warp < X_SUMMERS + X_SPLITTERS) {
+    // ---- W's pieces --------------------------------------------------------------------------------------------- //
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
+    // a warp's 32 rows, four at a time: eight lanes a row of 128 bytes
+    const int chunk = lane & 7, row = (warp - X_SUMMERS) * 32 + (lane >> 3);
+    // byte offset in a piece: 16-byte chunks are exchanged by bits 1-2 of the row; of rows row + 4 i the first is bit 1 of
+    // `row`, the second the oddness of i
+    const int at = row * 64 + (chunk & 1) * 8, turn = (row >> 1) & 3;
+    const int even = at + (((chunk >> 1) ^ turn) << 4), odd = at + (((chunk >> 1) ^ turn ^ 2) << 4);
+    int s = 0, q = 0;
+    unsigned s_phase = 1, q_phase = 0;
+    for (int it = 0; it < mine; ++it) {
+      bool ok = x_wait(raw_full + 8 * q, q_phase, gave_up, a.error);
+      if (!__all_sync(0xffffffffu, ok)) break;
+      float4 v[8];
+      const float4* src = reinterpret_cast<const float4*>(base + raw_at + q * X_RAW) + row * 8 + chunk;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = src[i * 32];
+      ok = x_wait(w_empty + 8 * s, s_phase, gave_up, a.error);
+      if (!__all_sync(0xffffffffu, ok)) break;
+      unsigned char* dst = base + w_at + s * 3 * X_W_PIECE;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        uint2 p[3];
+        x_split(v[i].x, v[i].y, p[0].x, p[1].x, p[2].x);
+        x_split(v[i].z, v[i].w, p[0].y, p[1].y, p[2].y);
+#pragma unroll
+        for (int j = 0; j < 3; ++j) *reinterpret_cast<uint2*>(dst + j * X_W_PIECE + i * 256 + (i & 1 ? odd : even)) = p[j];
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // every lane's stores, before the lane that arrives
+      __syncwarp();
+      if (lane == 0) {
+        x_arrive(raw_empty + 8 * q);
+        x_arrive(w_full + 8 * s);
+      }
+      if (++s == a.w_stages) { s = 0; s_phase ^= 1; }
+      if (++q == a.raw_stages) { q = 0; q_phase ^= 1; }
+    }
+    if (CLUSTER) {
+      x_cluster_sync();
+      x_cluster_sync();
+    }
+  } else {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+    if (warp == X_LOAD_X_WARP && lane == 0) {
+      // ---- the pieces of x -------------------------------------------------------------------------------------- //
+      int s = 0;
+      unsigned phase = 1;
+      for (int it = 0; it < mine; ++it) {
+        if (!x_wait(x_empty + 8 * s, phase, gave_up, a.error)) break;
+        const unsigned bar = x_full + 8 * s, dst = x_smem(base) + s * 3 * x_piece;
+        x_expect(bar, 3u * x_piece);
+#pragma unroll
+        for (int p = 0; p < 3; ++p) x_box(dst + p * x_piece, &x_map, (first + it) * X_KB, p * a.M + m0, bar);
+        if (++s == a.x_stages) { s = 0; phase ^= 1; }
+      }
+    } else if (warp == X_LOAD_W_WARP && lane == 0) {
+      // ---- W ---------------------------------------------------------------------------------------------------- //
+      int s = 0;
+      unsigned phase = 1;
+      for (int it = 0; it < mine; ++it) {
+        if (!x_wait(raw_empty + 8 * s, phase, gave_up, a.error)) break;
+        x_expect(raw_full + 8 * s, (unsigned)X_RAW);
+        x_box(x_smem(base) + raw_at + s * X_RAW, &w_map, (first + it) * X_KB, n0, raw_full + 8 * s);
+        if (++s == a.raw_stages) { s = 0; phase ^= 1; }
+      }
+    } else if (warp == X_MMA_WARP || warp == X_MMA_WARP + 2) {
+      // ---- products: a warp each for the even and the odd stages, which sum in halves of tensor memory of their own ---- //
+      // (the loop is the whole warp's, so that descriptors stay in uniform registers; one lane issues)
+      // float32 accumulator, bfloat16 operands, both K-major, N = cols, M = 128
+      const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(a.cols >> 3) << 17) | ((128u >> 4) << 24);
+      const int b = warp == X_MMA_WARP ? 0 : 1;
+      const unsigned d = tmem + b * 256;
+      for (int it = b; it < mine; it += 2) {
+        const int s = it % a.x_stages, q = it % a.w_stages;
+        bool ok = x_wait(sums_empty + 8 * b, ((it >> 1) & 1) ^ 1, gave_up, a.error);
+        ok = ok && x_wait(x_full + 8 * s, (it / a.x_stages) & 1, gave_up, a.error);
+        ok = ok && x_wait(w_full + 8 * q, (it / a.w_stages) & 1, gave_up, a.error);
+        if (!__all_sync(0xffffffffu, ok)) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const unsigned xs = x_smem(base) + s * 3 * x_piece, ws = x_smem(base) + w_at + q * 3 * X_W_PIECE;
+        if (x_elect()) {
+          // smallest first: what is cut off a sum that is still small is small
+#pragma unroll
+          for (int o = 0; o < X_KB * 2; o += 32) x_mma(d, ws + o, xs + 2 * x_piece + o, idesc, o ? 1u : 0u);
+#pragma unroll
+          for (int o = 0; o < X_KB * 2; o += 32) x_mma(d, ws + 2 * X_W_PIECE + o, xs + o, idesc, 1u);
+#pragma unroll
+          for (int o = 0; o < X_KB * 2; o += 32) x_mma(d, ws + X_W_PIECE + o, xs + x_piece + o, idesc, 1u);
+#pragma unroll
+          for (int o = 0; o < X_KB * 2; o += 32) x_mma(d, ws + o, xs + x_piece + o, idesc, 1u);
+#pragma unroll
+          for (int o = 0; o < X_KB * 2; o += 32) x_mma(d, ws + X_W_PIECE + o, xs + o, idesc, 1u);
+#pragma unroll
+          for (int o = 0; o < X_KB * 2; o += 32) x_mma(d, ws + o, xs + o, idesc, 1u);
+          x_commit(w_empty + 8 * q);
+          x_commit(x_empty + 8 * s);
+          x_commit(sums_full + 8 * b);
+        }
+        __syncwarp();
+      }
+    }
+    __syncwarp();
+    if (CLUSTER) {
+      x_cluster_sync();
+      x_cluster_sync();
+    }
+  }
+
+  // (the code that all warps share is kept to what the fewest registers hold)
+  if (*gave_up) {  // copies may still be on their way into this block's shared memory
+    for (int i = 0; i < 2000; ++i) __nanosleep(1000);
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  if (warp == X_MMA_WARP) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u));
+}
+
+template <int COLS, bool CLUSTER>
+int launch_linear_f32_tc5(const CUtensorMap& x_map, const CUtensorMap& w_map, const LinearX3Args& a, int ranks, cudaStream_t stream) {
+  auto kernel = linear_f32_tc5_kernel<COLS, CLUSTER>;
+  const size_t ring = (size_t)3 * (a.cols * X_KB * 2 * a.x_stages + X_W_PIECE * a.w_stages) + (size_t)X_RAW * a.raw_stages,
+               sums = CLUSTER ? (size_t)a.cols * (X_ROWS + 4) * 4 : 0;
+  const size_t smem = 1024 + (ring > sums ? ring : sums);
+  cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 1024 + X_RINGS);
+  if (err != cudaSuccess) {
+    mll_set_error("linear_f32_tc5: cannot reserve %d bytes of shared memory: %s", 1024 + X_RINGS, cudaGetErrorString(err));
+    return (int)err;
+  }
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3((unsigned)(a.m_tiles * ((a.N + X_ROWS - 1) / X_ROWS) * ranks));
+  config.blockDim = dim3(X_THREADS);
+  config.dynamicSmemBytes = smem;
+  config.stream = stream;
+  cudaLaunchAttribute attr[1];
+  if (CLUSTER) {
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)ranks;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    config.attrs = attr;
+    config.numAttrs = 1;
+  }
+  err = cudaLaunchKernelEx(&config, kernel, x_map, w_map, a);
+  if (err == cudaSuccess) err = cudaGetLastError();
+  if (err != cudaSuccess) {
+    mll_set_error("linear_f32_tc5: launch failed: %s", cudaGetErrorString(err));
+    return (int)err;
+  }
+  return 0;
+}
+
+// How M rows and K are cut up: the fewest rounds of blocks over the device, weighed by a block's time - per 32 columns of k six
+// products of `cols` columns, or the splitting of W if that is longer, and the start and end of a block.
+struct X3Plan {
+  int cols, ranks;
+};
+X3Plan x3_plan(int M, int N, int K) {
+  const int n_tiles = (N + X_ROWS - 1) / X_ROWS, k_blocks = (K + X_KB - 1) / X_KB, sms = mll_sm_count();
+  X3Plan best{0, 1};
+  double least = 0.0;
+  const int fewest = (M + 255) / 256;
+  for (int m_tiles = fewest; m_tiles <= fewest + 4; ++m_tiles) {
+    const int cols = ((M + m_tiles - 1) / m_tiles + 15) / 16 * 16;
+    const int tiles = (M + cols - 1) / cols;
+    for (int ranks = 1; ranks <= 8; ranks *= 2) {
+      if (ranks > 1 && k_blocks / ranks < 8) break;
+      const long long blocks = (long long)tiles * n_tiles * ranks;
+      const int resident = sms / ranks * ranks;  // clusters are resident as a whole
+      const double rounds = (double)((blocks + resident - 1) / resident);
+      const double stage = cols * 6.0 > 600.0 ? cols * 6.0 : 600.0;
+      const double time = rounds * ((double)((k_blocks + ranks - 1) / ranks) * stage + 8000.0 + (ranks > 1 ? 3000.0 : 0.0));
+      if (best.cols == 0 || time < least) {
+        least = time;
+        best = X3Plan{cols, ranks};
+      }
+    }
+  }
+  return best;
+}
+
+}  // namespace mll
+
+MLL_API int mll_linear_f32_tc5_supported(int M, int N, int K, int epilogue) {
+  if (M < 1 || N < 1 || K < 4 || K % 4 != 0) return 0;
+  if (M > (1 << 24) || N > (1 << 28)) return 0;  // row numbers of the tensor map and block numbers
+  if (epilogue == mll::XEPI_F32) return 1;
+  return (epilogue == mll::XEPI_SWIGLU || epilogue == mll::XEPI_GEGLU) && N % 16 == 0;
+}
+
+// x: float32 [M, K]; w: float32 [N, K]; bias: optional float32 [N]; pieces: room for [3, M, K rounded up to 8] bfloat16; out and
+// epilogue as in mll_linear_f32.  cols (a multiple of 16, at most 256) and ranks (1, 2, 4 or 8): how the work is cut up, 0 = choose.
+MLL_API int mll_linear_f32_tc5(const float* x, const float* w, const float* bias, void* pieces, float* out, int M, int N, int K,
+                               int epilogue, int cols, int ranks, cudaStream_t stream) {
+  MLL_REQUIRE(mll_linear_f32_tc5_supported(M, N, K, epilogue), "linear_f32_tc5: unsupported sizes M=%d N=%d K=%d epilogue %d", M, N, K,
+              epilogue);
+  MLL_REQUIRE(((uintptr_t)x | (uintptr_t)w | (uintptr_t)pieces) % 16 == 0, "linear_f32_tc5: operands must be 16-byte aligned");
+  MLL_REQUIRE(epilogue == mll::XEPI_F32 || bias == nullptr, "linear_f32_tc5: the gated epilogues take no bias");
+  const mll::X3Plan plan = mll::x3_plan(M, N, K);
+  if (cols == 0) cols = plan.cols;
+  if (ranks == 0) ranks = plan.ranks;
+  MLL_REQUIRE(cols >= 16 && cols <= 256 && cols % 16 == 0 && (ranks == 1 || ranks == 2 || ranks == 4 || ranks == 8),
+              "linear_f32_tc5: tiles of %d columns in clusters of %d", cols, ranks);
+  const int stride = (K + 7) / 8 * 8, k_blocks = (K + mll::X_KB - 1) / mll::X_KB;
+  const long long words = (long long)M * (stride / 8);
+  long long blocks = (words + 255) / 256;
+  if (blocks > mll_sm_count() * 8) blocks = mll_sm_count() * 8;
+  MLL_LAUNCH((mll::split_f32_kernel), (int)blocks, 256, 0, stream, x, (__nv_bfloat16*)pieces, M, K, stride);
+  MLL_LAUNCH_CHECK();
+  CUtensorMap x_map, w_map;
+  if (mll::tensor_map_bf16_span64(pieces, 3ll * M, stride, cols, &x_map) != 0) return -1;
+  if (mll::tensor_map_f32_span128(w, N, K, mll::X_ROWS, &w_map) != 0) return -1;
+  MllDeviceErrorWords errors;
+  mll_device_error_words(&errors);  // all null if they cannot be had: a wait that ran out is then not reported
+  // three stages of both operands' pieces, two of W's where the rows of x leave no room for a third; what is left is W's on its way
+  const int x_stage = 3 * cols * mll::X_KB * 2, w_stage = 3 * mll::X_W_PIECE;
+  const int w_stages = 3 * (x_stage + w_stage) + 2 * mll::X_RAW <= mll::X_RINGS ? 3 : 2;
+  int raw_stages = (mll::X_RINGS - 3 * x_stage - w_stages * w_stage) / mll::X_RAW;
+  if (raw_stages > mll::X_MAX_STAGES) raw_stages = mll::X_MAX_STAGES;
+  mll::LinearX3Args a{x, w, bias, out, M, N, K, epilogue, cols, (M + cols - 1) / cols, (k_blocks + ranks - 1) / ranks, 3, w_stages, raw_stages,
+                      errors.word[1]};
+  const bool wide = cols > 128;
+  if (ranks == 1)
+    return wide ? mll::launch_linear_f32_tc5<128, false>(x_map, w_map, a, 1, stream)
+                : mll::launch_linear_f32_tc5<64, false>(x_map, w_map, a, 1, stream);
+  return wide ? mll::launch_linear_f32_tc5<128, true>(x_map, w_map, a, ranks, stream)
+              : mll::launch_linear_f32_tc5<64, true>(x_map, w_map, a, ranks, stream);
+}
