@@ -149,6 +149,12 @@ __device__ __forceinline__ void a_umma(unsigned tmem_d, unsigned long long desc_
 __device__ __forceinline__ void a_commit(unsigned bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
+// true in one lane of a converged warp
+__device__ __forceinline__ bool a_elect() {
+  unsigned one;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
+  return one != 0;
+}
 __device__ __forceinline__ void a_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void a_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 // generic-proxy writes to shared memory become visible to the tensor cores and TMA
@@ -412,28 +418,22 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_c
       }
     }
   } else if (warp == MMA_WARP) {
-    // ---- S = Q K^T, one thread.  S_i goes into buffer i % SB, which held P_{i-SB}: it waits for that page's P V.
-    if (lane == 0) {
-      constexpr unsigned idesc_s = a_idesc(A_ROWS, MLL_PAGE, false);
-      // The descriptors are built once; a step inside a tile only adds to the address field (16-byte units, 14
-      // bits: the tiles lie in the first 256 KB of shared memory, so the sum cannot carry out of it).  Built
-      // anew for every instruction they cost this thread some twenty dependent instructions per MMA.
-      const unsigned long long q_desc = a_desc(q_s, 16);
-      unsigned long long k_desc[KS];
-#pragma unroll
-      for (int s = 0; s < KS; ++s) k_desc[s] = a_desc(k_s + s * L::K_BYTES, 16);
-      wait(bar(L::AB_Q, 0), 0);
-      for (int i = 0; i < n_pages && !*abort_flag; ++i) {
-        const int sb = i % SB, st = i % KS;
-        unsigned long long kd = k_desc[0];
-#pragma unroll
-        for (int s = 1; s < KS; ++s)
-          if (st == s) kd = k_desc[s];
-        wait(bar(L::AB_K_FULL, st), (i / KS) & 1);
-        if (i >= SB) wait(bar(L::AB_PV_DONE, sb), ((i - SB) / SB) & 1);  // the buffer's P, of page i - SB, has been read
-        a_fence_after();
-        if (*abort_flag) break;
-        const unsigned d = tmem_base + sb * MLL_PAGE;
+    // ---- S = Q K^T.  S_i goes into buffer i % SB, which held P_{i-SB}: it waits for that page's P V.  The loop is the
+    // whole warp's and one elected lane issues: inside a branch of one lane the descriptors go through ordinary registers and
+    // every MMA costs its thread some hundred clocks, in a loop that all lanes walk they stay in uniform ones.
+    constexpr unsigned idesc_s = a_idesc(A_ROWS, MLL_PAGE, false);
+    wait(bar(L::AB_Q, 0), 0);
+    for (int i = 0; i < n_pages; ++i) {
+      const int sb = i % SB, st = i % KS;
+      wait(bar(L::AB_K_FULL, st), (i / KS) & 1);
+      if (i >= SB) wait(bar(L::AB_PV_DONE, sb), ((i - SB) / SB) & 1);  // the buffer's P, of page i - SB, has been read
+      a_fence_after();
+      if (__any_sync(0xffffffffu, *abort_flag)) break;
+      // a step inside a tile only adds to the address field (16-byte units, 14 bits: the tiles lie in the first 256 KB of
+      // shared memory, so the sum cannot carry out of it)
+      const unsigned long long q_desc = a_desc(q_s, 16), kd = a_desc(k_s + st * L::K_BYTES, 16);
+      const unsigned d = tmem_base + sb * MLL_PAGE;
+      if (a_elect()) {
 #pragma unroll
         for (int b = 0; b < DB; ++b)
 #pragma unroll
@@ -443,26 +443,20 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_c
         a_commit(bar(L::AB_S_FULL, sb));
         a_commit(bar(L::AB_K_EMPTY, st));
       }
+      __syncwarp();
     }
   } else if (warp == PV_WARP) {
-    // ---- O += P V, a thread of its own: with one thread for both products a page's MMAs went out one behind
-    // the other (75 clocks apiece for S, 135 for P V, and a hundred for every wait, even one that is over),
-    // 2,400 to 3,000 clocks a page of which the tensor cores worked 640, and the softmax warps waited
-    if (lane == 0) {
-      constexpr unsigned idesc_o = a_idesc(A_ROWS, DV, true);
-      unsigned long long v_desc[KS];
-#pragma unroll
-      for (int s = 0; s < KS; ++s) v_desc[s] = a_desc(v_s + s * L::V_BYTES, MLL_PAGE * 128);
-      for (int i = 0; i < n_pages && !*abort_flag; ++i) {
-        const int sb = i % SB, st = i % KS;
-        unsigned long long vd = v_desc[0];
-#pragma unroll
-        for (int s = 1; s < KS; ++s)
-          if (st == s) vd = v_desc[s];
-        wait(bar(L::AB_V_FULL, st), (i / KS) & 1);
-        wait(bar(L::AB_P_READY, sb), (i / SB) & 1);
-        a_fence_after();
-        if (*abort_flag) break;
+    // ---- O += P V, a warp of its own: with one thread for both products a page's MMAs went out one behind
+    // the other with their waits in between, and the softmax warps waited
+    constexpr unsigned idesc_o = a_idesc(A_ROWS, DV, true);
+    for (int i = 0; i < n_pages; ++i) {
+      const int sb = i % SB, st = i % KS;
+      wait(bar(L::AB_V_FULL, st), (i / KS) & 1);
+      wait(bar(L::AB_P_READY, sb), (i / SB) & 1);
+      a_fence_after();
+      if (__any_sync(0xffffffffu, *abort_flag)) break;
+      const unsigned long long vd = a_desc(v_s + st * L::V_BYTES, MLL_PAGE * 128);
+      if (a_elect()) {
 #pragma unroll
         for (int k = 0; k < 4; ++k)  // P: 16 keys = 8 packed columns per step
           a_umma_ts(tmem_base + L::O_COL, tmem_base + sb * MLL_PAGE + k * 8, vd + (unsigned long long)((k * (16 * 128)) >> 4),
@@ -470,6 +464,7 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_c
         a_commit(bar(L::AB_PV_DONE, sb));
         a_commit(bar(L::AB_V_EMPTY, st));
       }
+      __syncwarp();
     }
   } else if (warp < 4) {
     // ---- softmax: thread r owns query row r = lane r of tensor memory ------------------------- //

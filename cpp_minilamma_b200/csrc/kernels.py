@@ -367,12 +367,17 @@ LINEAR_F32_TC5_ROWS = 2048  # rows of x split at a time
 
 def linear_f32_tc5_pieces(rows: int, in_features: int):
     """Shape of the bfloat16 scratch that `linear_f32_tc5` needs for `rows` rows."""
-    return (3, min(rows, LINEAR_F32_TC5_ROWS), -(-in_features // 8) * 8)
+    return (-(-in_features // 32), 3, min(rows, LINEAR_F32_TC5_ROWS) + 256, 32)
 
 
 def linear_f32_tc5_supported(x: torch.Tensor, w: torch.Tensor, epilogue: int = EPI_F32) -> bool:
     """Whether `linear_f32_tc5` takes x . w^T: float32, rows on 16-byte boundaries."""
     return _linear_f32_operands(x, w) and bool(lib().mll_linear_f32_tc5_supported(x.shape[0], w.shape[0], w.shape[1], epilogue))
+
+
+def linear_f32_tc5_pays(x: torch.Tensor, w: torch.Tensor, epilogue: int = EPI_F32) -> bool:
+    """Whether `linear_f32_tc5` takes x . w^T and is faster than the library's product."""
+    return _linear_f32_operands(x, w) and bool(lib().mll_linear_f32_tc5_pays(x.shape[0], w.shape[0], w.shape[1], epilogue))
 
 
 def linear_f32_tc5(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], pieces: torch.Tensor, out: torch.Tensor,
@@ -382,7 +387,7 @@ def linear_f32_tc5(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor
     at most 256) and blocks that share K (1, 2, 4 or 8); 0: chosen."""
     for t, name in ((x, "x"), (w, "w"), (out, "out")):
         _need(t, "linear_f32_tc5 " + name, torch.float32, 2)
-    _need(pieces, "linear_f32_tc5 pieces", torch.bfloat16, 3)
+    _need(pieces, "linear_f32_tc5 pieces", torch.bfloat16, 4)
     (rows, k), n = x.shape, w.shape[0]
     if w.shape[1] != k or tuple(out.shape) != (rows, n if epilogue == EPI_F32 else n // 2):
         raise KernelError(f"linear_f32_tc5: x {tuple(x.shape)}, w {tuple(w.shape)} and out {tuple(out.shape)} do not fit")

@@ -9,14 +9,14 @@
 // Bound: the tensor pipe, at a sixth of its bfloat16 rate.
 //
 // A block forms 128 weight rows (the M operand) times up to 256 rows of x (the N operand) over a slice of K, 32 columns a stage:
-//   warp 12    loads the three pieces of x, split by a kernel in front (x is small and every column of blocks reads it again): boxes of
-//              [rows x 32] with the 64-byte swizzle into a ring of their own.
+//   warp 12    loads the three pieces of x, split by a kernel in front (x is small and every column of blocks reads it again) that
+//              leaves them in the order in which they lie in shared memory: a copy a piece and stage, all in one run of bytes.
+//              (As boxes of a matrix, 64 bytes a row, these loads set the pace.)
 //   warp 14    loads W as it is: boxes of [128 x 32] floats.
 //   warps 8-11 split W: 32 rows a warp, from its ring into that of its pieces, where the swizzle puts them.  (Loading W into
 //              registers a stage or two ahead instead of through a ring was bound by those loads' latency: the fence in front of the
 //              tensor cores' reads waits for them too, 2,000 to 3,000 clocks a stage.)
-//   warps 13, 15  issue the products, one thread each: twelve a stage, the even stages' into one half of tensor memory, the odd
-//              ones' into the other.
+//   warp 13    issues the products: twelve a stage, into one of two halves of tensor memory.
 //   warps 0-7  add a stage's sums to their registers: a thread has half of a row's.
 // K is split over the blocks of a cluster where tiles alone would leave multiprocessors idle; the blocks then add their shares
 // in rank order through distributed shared memory, so a result does not depend on the run.
@@ -40,7 +40,7 @@ namespace mll {
 enum : int { XEPI_F32 = 1, XEPI_SWIGLU = 2, XEPI_GEGLU = 4 };  // numbered as the bfloat16 kernels' epilogues
 constexpr int X_SUMMERS = 8;              // warps that add up sums: two warpgroups
 constexpr int X_SPLITTERS = 4;            // warps that split W: one warpgroup
-constexpr int X_LOAD_X_WARP = 12, X_MMA_WARP = 13, X_LOAD_W_WARP = 14;  // and X_MMA_WARP + 2
+constexpr int X_LOAD_X_WARP = 12, X_MMA_WARP = 13, X_LOAD_W_WARP = 14;
 constexpr int X_THREADS = 512;            // four warpgroups: 168 + 168 + 88 + 40 registers a thread of the 128 each at the start
 constexpr int X_ROWS = 128;               // weight rows of a block
 constexpr int X_KB = 32;                  // columns of k a stage: 64 bytes of a piece, one swizzle span
@@ -54,10 +54,11 @@ struct LinearX3Args {
   const float* x;     // [M, K]
   const float* w;     // [N, K]
   const float* bias;  // optional [N]
+  const unsigned char* pieces;  // of x: [k blocks][3][height] rows of 64 bytes
   float* out;         // [M, N] (gated epilogues: [M, N / 2])
   int M, N, K, epilogue;
   int cols;           // rows of x a block takes, a multiple of 16
-  int m_tiles, blocks_per_rank;
+  int m_tiles, blocks_per_rank, height;
   int x_stages, w_stages, raw_stages;
   int* error;
 };
@@ -89,6 +90,10 @@ __device__ __forceinline__ void x_init(unsigned bar, unsigned count) {
 __device__ __forceinline__ void x_box(unsigned dst, const CUtensorMap* map, int c, int r, unsigned bar) {
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                ::"r"(dst), "l"(map), "r"(c), "r"(r), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void x_copy(unsigned dst, const void* src, unsigned bytes, unsigned bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
 __device__ __forceinline__ void x_arrive(unsigned bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
@@ -143,23 +148,25 @@ __device__ __forceinline__ void x_split(float a, float b, unsigned& p0, unsigned
                    0x7632);
 }
 
-// pieces[i] = piece i of x: [3][M][stride], columns from K to the stride (a multiple of 8) zero.  Bound by memory (4 bytes in,
-// 6 out a value).
-__global__ void split_f32_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ pieces, int M, int K, int stride) {
-  const int words = stride / 8;
-  const long long total = (long long)M * words, plane = (long long)M * stride;
+// pieces[kb][i][row] = 32 columns of piece i of x's row, 64 bytes, whose 16-byte chunks are exchanged by bits 1-2 of the row (the
+// 64-byte swizzle).  Columns from K on are zero; rows from M to the padded height are left as they are: their sums are not
+// written.  Bound by memory (4 bytes in, 6 out a value).
+__global__ void split_f32_kernel(const float* __restrict__ x, unsigned char* __restrict__ pieces, int M, int K, int height) {
+  const long long total = (long long)M * ((K + X_KB - 1) / X_KB * 4);
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const int row = (int)(i / words), c = (int)(i % words) * 8;
-    const float* src = x + (size_t)row * K + c;
-    const float4 a = *reinterpret_cast<const float4*>(src);  // K is a multiple of 4
-    const float4 b = c + 4 < K ? *reinterpret_cast<const float4*>(src + 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const int chunk = (int)(i & 3), kb = (int)((i >> 2) / M), row = (int)((i >> 2) % M), c = kb * X_KB + chunk * 8;
+    const float* src = x + (size_t)row * K + c;  // K is a multiple of 4
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 a = c < K ? *reinterpret_cast<const float4*>(src) : zero;
+    const float4 b = c + 4 < K ? *reinterpret_cast<const float4*>(src + 4) : zero;
     uint4 p[3];
     x_split(a.x, a.y, p[0].x, p[1].x, p[2].x);
     x_split(a.z, a.w, p[0].y, p[1].y, p[2].y);
     x_split(b.x, b.y, p[0].z, p[1].z, p[2].z);
     x_split(b.z, b.w, p[0].w, p[1].w, p[2].w);
+    unsigned char* dst = pieces + ((size_t)kb * 3 * height + row) * 64 + ((chunk ^ ((row >> 1) & 3)) << 4);
 #pragma unroll
-    for (int j = 0; j < 3; ++j) *reinterpret_cast<uint4*>(pieces + j * plane + (size_t)row * stride + c) = p[j];
+    for (int j = 0; j < 3; ++j) *reinterpret_cast<uint4*>(dst + (size_t)j * height * 64) = p[j];
   }
 }
 
@@ -186,8 +193,7 @@ __device__ __forceinline__ void x_write(const LinearX3Args& a, float v, int m, i
 
 // COLS: most columns (rows of x) of a block that one of the two groups of summing warps holds sums of
 template <int COLS, bool CLUSTER>
-__global__ void __launch_bounds__(X_THREADS, 1) linear_f32_tc5_kernel(const __grid_constant__ CUtensorMap x_map,
-                                                                      const __grid_constant__ CUtensorMap w_map, LinearX3Args a) {
+__global__ void __launch_bounds__(X_THREADS, 1) linear_f32_tc5_kernel(const __grid_constant__ CUtensorMap w_map, LinearX3Args a) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* base = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   __shared__ __align__(8) unsigned long long bars[6 * X_MAX_STAGES + 4];
@@ -266,29 +272,27 @@ __global__ void __launch_bounds__(X_THREADS, 1) linear_f32_tc5_kernel(const __gr
     const int r0 = (warp & 3) * 32 + lane;
     const int wide = X_ROWS + 4;  // words of a column of the tile in shared memory
     float* part = reinterpret_cast<float*>(base);
+    // The block's share into its rings (all copies into them have arrived: their products are through), column by column, and from
+    // there to the result.  (Straight from the registers, a column's code once for each of them, the writing waited for its own
+    // instructions: 30 to 67 us where the sums took 75.)
     if (!*gave_up) {
-      if (CLUSTER) {
-        // the block's share into its rings (all copies into them have arrived: their products are through), column by column
 #pragma unroll
-        for (int c = 0; c < COLS; ++c)
-          if (c < half) part[(size_t)(group * half + c) * wide + r0] = acc[c];
-      } else {
-#pragma unroll
-        for (int c = 0; c < COLS; ++c)
-          if (c < half) x_write(a, acc[c], m0 + group * half + c, n0 + r0);
-      }
+      for (int c = 0; c < COLS; ++c)
+        if (c < half) part[(size_t)(group * half + c) * wide + r0] = acc[c];
     }
-    if (CLUSTER) {
-      x_cluster_sync();
-      const int per = (a.cols + ranks - 1) / ranks, from = rank * per, to = min(a.cols, from + per);
-      for (int i = from * 4 + warp; i < to * 4; i += X_SUMMERS) {
-        const int c = i >> 2, r = (i & 3) * 32 + lane;
-        float s = 0.f;
+    if (CLUSTER) x_cluster_sync();
+    else asm volatile("bar.sync 1, 256;" ::: "memory");
+    const int per = (a.cols + ranks - 1) / ranks, from = rank * per, to = min(a.cols, from + per);
+#pragma unroll 1
+    for (int i = from * 4 + warp; i < to * 4; i += X_SUMMERS) {
+      const int c = i >> 2, r = (i & 3) * 32 + lane;
+      float s = 0.f;
+      if (CLUSTER)
         for (int j = 0; j < ranks; ++j) s += cg::this_cluster().map_shared_rank(part, j)[(size_t)c * wide + r];
-        x_write(a, s, m0 + c, n0 + r);
-      }
-      x_cluster_sync();
+      else s = part[(size_t)c * wide + r];
+      x_write(a, s, m0 + c, n0 + r);
     }
+    if (CLUSTER) x_cluster_sync();
   } else if (warp < X_SUMMERS + X_SPLITTERS) {
     // ---- W's pieces --------------------------------------------------------------------------------------------- //
     asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
@@ -342,7 +346,8 @@ __global__ void __launch_bounds__(X_THREADS, 1) linear_f32_tc5_kernel(const __gr
         const unsigned bar = x_full + 8 * s, dst = x_smem(base) + s * 3 * x_piece;
         x_expect(bar, 3u * x_piece);
 #pragma unroll
-        for (int p = 0; p < 3; ++p) x_box(dst + p * x_piece, &x_map, (first + it) * X_KB, p * a.M + m0, bar);
+        for (int p = 0; p < 3; ++p)
+          x_copy(dst + p * x_piece, a.pieces + ((size_t)((first + it) * 3 + p) * a.height + m0) * 64, (unsigned)x_piece, bar);
         if (++s == a.x_stages) { s = 0; phase ^= 1; }
       }
     } else if (warp == X_LOAD_W_WARP && lane == 0) {
@@ -355,21 +360,20 @@ __global__ void __launch_bounds__(X_THREADS, 1) linear_f32_tc5_kernel(const __gr
         x_box(x_smem(base) + raw_at + s * X_RAW, &w_map, (first + it) * X_KB, n0, raw_full + 8 * s);
         if (++s == a.raw_stages) { s = 0; phase ^= 1; }
       }
-    } else if (warp == X_MMA_WARP || warp == X_MMA_WARP + 2) {
-      // ---- products: a warp each for the even and the odd stages, which sum in halves of tensor memory of their own ---- //
-      // (the loop is the whole warp's, so that descriptors stay in uniform registers; one lane issues)
+    } else if (warp == X_MMA_WARP) {
+      // ---- products (the loop is the whole warp's, so that descriptors stay in uniform registers; one lane issues) ---- //
       // float32 accumulator, bfloat16 operands, both K-major, N = cols, M = 128
       const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(a.cols >> 3) << 17) | ((128u >> 4) << 24);
-      const int b = warp == X_MMA_WARP ? 0 : 1;
-      const unsigned d = tmem + b * 256;
-      for (int it = b; it < mine; it += 2) {
-        const int s = it % a.x_stages, q = it % a.w_stages;
+      int s = 0, q = 0;
+      unsigned s_phase = 0, q_phase = 0;
+      for (int it = 0; it < mine; ++it) {
+        const int b = it & 1;
         bool ok = x_wait(sums_empty + 8 * b, ((it >> 1) & 1) ^ 1, gave_up, a.error);
-        ok = ok && x_wait(x_full + 8 * s, (it / a.x_stages) & 1, gave_up, a.error);
-        ok = ok && x_wait(w_full + 8 * q, (it / a.w_stages) & 1, gave_up, a.error);
+        ok = ok && x_wait(x_full + 8 * s, s_phase, gave_up, a.error);
+        ok = ok && x_wait(w_full + 8 * q, q_phase, gave_up, a.error);
         if (!__all_sync(0xffffffffu, ok)) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const unsigned xs = x_smem(base) + s * 3 * x_piece, ws = x_smem(base) + w_at + q * 3 * X_W_PIECE;
+        const unsigned xs = x_smem(base) + s * 3 * x_piece, ws = x_smem(base) + w_at + q * 3 * X_W_PIECE, d = tmem + b * 256;
         if (x_elect()) {
           // smallest first: what is cut off a sum that is still small is small
 #pragma unroll
@@ -389,6 +393,8 @@ __global__ void __launch_bounds__(X_THREADS, 1) linear_f32_tc5_kernel(const __gr
           x_commit(sums_full + 8 * b);
         }
         __syncwarp();
+        if (++s == a.x_stages) { s = 0; s_phase ^= 1; }
+        if (++q == a.w_stages) { q = 0; q_phase ^= 1; }
       }
     }
     __syncwarp();
@@ -409,10 +415,10 @@ __global__ void __launch_bounds__(X_THREADS, 1) linear_f32_tc5_kernel(const __gr
 }
 
 template <int COLS, bool CLUSTER>
-int launch_linear_f32_tc5(const CUtensorMap& x_map, const CUtensorMap& w_map, const LinearX3Args& a, int ranks, cudaStream_t stream) {
+int launch_linear_f32_tc5(const CUtensorMap& w_map, const LinearX3Args& a, int ranks, cudaStream_t stream) {
   auto kernel = linear_f32_tc5_kernel<COLS, CLUSTER>;
   const size_t ring = (size_t)3 * (a.cols * X_KB * 2 * a.x_stages + X_W_PIECE * a.w_stages) + (size_t)X_RAW * a.raw_stages,
-               sums = CLUSTER ? (size_t)a.cols * (X_ROWS + 4) * 4 : 0;
+               sums = (size_t)a.cols * (X_ROWS + 4) * 4;
   const size_t smem = 1024 + (ring > sums ? ring : sums);
   cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 1024 + X_RINGS);
   if (err != cudaSuccess) {
@@ -432,7 +438,7 @@ int launch_linear_f32_tc5(const CUtensorMap& x_map, const CUtensorMap& w_map, co
     config.attrs = attr;
     config.numAttrs = 1;
   }
-  err = cudaLaunchKernelEx(&config, kernel, x_map, w_map, a);
+  err = cudaLaunchKernelEx(&config, kernel, w_map, a);
   if (err == cudaSuccess) err = cudaGetLastError();
   if (err != cudaSuccess) {
     mll_set_error("linear_f32_tc5: launch failed: %s", cudaGetErrorString(err));
@@ -479,8 +485,14 @@ MLL_API int mll_linear_f32_tc5_supported(int M, int N, int K, int epilogue) {
   return (epilogue == mll::XEPI_SWIGLU || epilogue == mll::XEPI_GEGLU) && N % 16 == 0;
 }
 
-// x: float32 [M, K]; w: float32 [N, K]; bias: optional float32 [N]; pieces: room for [3, M, K rounded up to 8] bfloat16; out and
-// epilogue as in mll_linear_f32.  cols (a multiple of 16, at most 256) and ranks (1, 2, 4 or 8): how the work is cut up, 0 = choose.
+// Whether it takes this problem and is the faster way (us, the library / here).
+MLL_API int mll_linear_f32_tc5_pays(int M, int N, int K, int epilogue) {
+  if (!mll_linear_f32_tc5_supported(M, N, K, epilogue) || M <= 16) return 0;
+  return (double)M * N * K >= 1.0e9;
+}
+
+// x: float32 [M, K]; w: float32 [N, K]; bias: optional float32 [N]; pieces: room for [K / 32 rounded up, 3, M + 256, 32] bfloat16; out
+// and epilogue as in mll_linear_f32.  cols (a multiple of 16, at most 256) and ranks (1, 2, 4 or 8): how the work is cut up, 0 = choose.
 MLL_API int mll_linear_f32_tc5(const float* x, const float* w, const float* bias, void* pieces, float* out, int M, int N, int K,
                                int epilogue, int cols, int ranks, cudaStream_t stream) {
   MLL_REQUIRE(mll_linear_f32_tc5_supported(M, N, K, epilogue), "linear_f32_tc5: unsupported sizes M=%d N=%d K=%d epilogue %d", M, N, K,
@@ -492,14 +504,13 @@ MLL_API int mll_linear_f32_tc5(const float* x, const float* w, const float* bias
   if (ranks == 0) ranks = plan.ranks;
   MLL_REQUIRE(cols >= 16 && cols <= 256 && cols % 16 == 0 && (ranks == 1 || ranks == 2 || ranks == 4 || ranks == 8),
               "linear_f32_tc5: tiles of %d columns in clusters of %d", cols, ranks);
-  const int stride = (K + 7) / 8 * 8, k_blocks = (K + mll::X_KB - 1) / mll::X_KB;
-  const long long words = (long long)M * (stride / 8);
+  const int k_blocks = (K + mll::X_KB - 1) / mll::X_KB, m_tiles = (M + cols - 1) / cols, height = m_tiles * cols;  // below M + 256
+  const long long words = (long long)M * k_blocks * 4;
   long long blocks = (words + 255) / 256;
   if (blocks > mll_sm_count() * 8) blocks = mll_sm_count() * 8;
-  MLL_LAUNCH((mll::split_f32_kernel), (int)blocks, 256, 0, stream, x, (__nv_bfloat16*)pieces, M, K, stride);
+  MLL_LAUNCH((mll::split_f32_kernel), (int)blocks, 256, 0, stream, x, (unsigned char*)pieces, M, K, height);
   MLL_LAUNCH_CHECK();
-  CUtensorMap x_map, w_map;
-  if (mll::tensor_map_bf16_span64(pieces, 3ll * M, stride, cols, &x_map) != 0) return -1;
+  CUtensorMap w_map;
   if (mll::tensor_map_f32_span128(w, N, K, mll::X_ROWS, &w_map) != 0) return -1;
   MllDeviceErrorWords errors;
   mll_device_error_words(&errors);  // all null if they cannot be had: a wait that ran out is then not reported
@@ -508,12 +519,12 @@ MLL_API int mll_linear_f32_tc5(const float* x, const float* w, const float* bias
   const int w_stages = 3 * (x_stage + w_stage) + 2 * mll::X_RAW <= mll::X_RINGS ? 3 : 2;
   int raw_stages = (mll::X_RINGS - 3 * x_stage - w_stages * w_stage) / mll::X_RAW;
   if (raw_stages > mll::X_MAX_STAGES) raw_stages = mll::X_MAX_STAGES;
-  mll::LinearX3Args a{x, w, bias, out, M, N, K, epilogue, cols, (M + cols - 1) / cols, (k_blocks + ranks - 1) / ranks, 3, w_stages, raw_stages,
+  mll::LinearX3Args a{x, w, bias, (const unsigned char*)pieces, out, M, N, K, epilogue, cols, m_tiles, (k_blocks + ranks - 1) / ranks, height, 3, w_stages, raw_stages,
                       errors.word[1]};
   const bool wide = cols > 128;
   if (ranks == 1)
-    return wide ? mll::launch_linear_f32_tc5<128, false>(x_map, w_map, a, 1, stream)
-                : mll::launch_linear_f32_tc5<64, false>(x_map, w_map, a, 1, stream);
-  return wide ? mll::launch_linear_f32_tc5<128, true>(x_map, w_map, a, ranks, stream)
-              : mll::launch_linear_f32_tc5<64, true>(x_map, w_map, a, ranks, stream);
+    return wide ? mll::launch_linear_f32_tc5<128, false>(w_map, a, 1, stream)
+                : mll::launch_linear_f32_tc5<64, false>(w_map, a, 1, stream);
+  return wide ? mll::launch_linear_f32_tc5<128, true>(w_map, a, ranks, stream)
+              : mll::launch_linear_f32_tc5<64, true>(w_map, a, ranks, stream);
 }

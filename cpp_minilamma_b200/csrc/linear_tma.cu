@@ -302,11 +302,11 @@ struct MapKey {
 struct MapKeyHash {
   size_t operator()(const MapKey& k) const {
     return std::hash<const void*>()(k.ptr) ^ (std::hash<long long>()(k.rows * 1315423911LL + k.cols) << 1) ^
-           (k.box_rows * 4 + k.kind);
+           (k.box_rows * 2 + k.kind);
   }
 };
 
-enum : int { MAP_BF16_128 = 0, MAP_BF16_64 = 1, MAP_F32_128 = 2 };  // boxes of 64 or 32 bfloat16 columns with their swizzle, 32 floats
+enum : int { MAP_BF16 = 0, MAP_F32 = 1 };  // boxes of 64 bfloat16 columns with the 128-byte swizzle, of 32 floats without one
 static int tensor_map_of(const void* ptr, long long rows, long long cols, int box_rows, int kind, CUtensorMap* out) {
   static std::unordered_map<MapKey, CUtensorMap, MapKeyHash> cache;
   static std::mutex lock;
@@ -323,16 +323,14 @@ static int tensor_map_of(const void* ptr, long long rows, long long cols, int bo
     return -1;
   }
   const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-  const cuuint64_t strides[1] = {(cuuint64_t)cols * (kind == MAP_F32_128 ? 4 : 2)};
-  const cuuint32_t box[2] = {(cuuint32_t)(kind == MAP_BF16_128 ? T_KB : 32), (cuuint32_t)box_rows};
+  const cuuint64_t strides[1] = {(cuuint64_t)cols * (kind == MAP_F32 ? 4 : 2)};
+  const cuuint32_t box[2] = {(cuuint32_t)(kind == MAP_F32 ? 32 : T_KB), (cuuint32_t)box_rows};
   const cuuint32_t elem[2] = {1, 1};
   CUtensorMap map;
-  const CUresult rc = encode(&map, kind == MAP_F32_128 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
+  const CUresult rc = encode(&map, kind == MAP_F32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
                              const_cast<void*>(ptr), dims, strides, box, elem,
                              CU_TENSOR_MAP_INTERLEAVE_NONE,
-                             kind == MAP_F32_128   ? CU_TENSOR_MAP_SWIZZLE_NONE
-                             : kind == MAP_BF16_64 ? CU_TENSOR_MAP_SWIZZLE_64B
-                                                   : CU_TENSOR_MAP_SWIZZLE_128B,
+                             kind == MAP_F32 ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B,
                              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (rc != CUDA_SUCCESS) {
     mll_set_error("linear_tma: cuTensorMapEncodeTiled failed with code %d for a [%lld, %lld] matrix", (int)rc, rows, cols);
@@ -345,13 +343,10 @@ static int tensor_map_of(const void* ptr, long long rows, long long cols, int bo
 }
 
 int tensor_map_bf16(const void* ptr, long long rows, long long cols, int box_rows, CUtensorMap* out) {
-  return tensor_map_of(ptr, rows, cols, box_rows, MAP_BF16_128, out);
-}
-int tensor_map_bf16_span64(const void* ptr, long long rows, long long cols, int box_rows, CUtensorMap* out) {
-  return tensor_map_of(ptr, rows, cols, box_rows, MAP_BF16_64, out);
+  return tensor_map_of(ptr, rows, cols, box_rows, MAP_BF16, out);
 }
 int tensor_map_f32_span128(const void* ptr, long long rows, long long cols, int box_rows, CUtensorMap* out) {
-  return tensor_map_of(ptr, rows, cols, box_rows, MAP_F32_128, out);
+  return tensor_map_of(ptr, rows, cols, box_rows, MAP_F32, out);
 }
 
 template <int NT>

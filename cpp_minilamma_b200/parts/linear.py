@@ -4,7 +4,8 @@ W is row-major [out, in] as in the reference (src/cuda_matmul.cc:181-186, one
 `cublasSgemm` per call there).  The product runs in the dtype of the weight:
   * bfloat16 weight, bfloat16 x: tensor-core product with float32 accumulation;
   * float32 weight: a true float32 product (TF32 must be off; it is refused otherwise), for the few rows of a decode
-    step on a weight-streaming kernel of this package; bfloat16 activations are widened first and the result narrowed
+    step on a weight-streaming kernel of this package, for the many of a prompt on one that splits float32 numbers over
+    the bfloat16 tensor cores without losing bits; bfloat16 activations are widened first and the result narrowed
     afterwards.
 A bias (float32 [N], not in the reference) is added in float32 by the weight-streaming kernels' epilogues, or by a
 kernel behind the library product.
@@ -75,9 +76,9 @@ class Linear:
                 x = wide
             if out_dtype == torch.float32:
                 out = given if given is not None else ws.buffer(out_name, (rows, self.out_features), torch.float32)
-                return self._product_f32(step, x, out)
+                return self._product_f32(step, x, out_name, out)
             wide_out = ws.buffer(out_name + ".y32", (rows, self.out_features), torch.float32)
-            self._product_f32(step, x, wide_out)
+            self._product_f32(step, x, out_name, wide_out)
             out = given if given is not None else ws.buffer(out_name, (rows, self.out_features), out_dtype)
             K.cast(wide_out, out)
             return out
@@ -104,9 +105,12 @@ class Linear:
             _mm_bf16_to_f32(x, w, out)
         return self._biased(out)
 
-    def _product_f32(self, step, x: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
+    def _product_f32(self, step, x: torch.Tensor, out_name: str, out: torch.Tensor) -> torch.Tensor:
         if x.shape[0] <= step.small_rows and out.is_contiguous() and K.linear_f32_pays(x, self.weight):
             K.linear_f32(x, self.weight, self.bias, out)
+            return out
+        if out.is_contiguous() and K.linear_f32_tc5_pays(x, self.weight):
+            K.linear_f32_tc5(x, self.weight, self.bias, f32_pieces(step, x, out_name), out)
             return out
         torch.mm(x, self.weight.t(), out=out)
         return self._biased(out)
@@ -128,6 +132,13 @@ class Linear:
         if not K.small_linear(x, self.weight, self.bias, values, K.EPI_RESID, row_norm, K.ResidualOut(into.x, weight, sumsq)):
             return None
         return PreNormed(values, sumsq, partials, eps, into.norm)
+
+
+def f32_pieces(step, x: torch.Tensor, out_name: str) -> torch.Tensor:
+    """Scratch for a float32 product of many rows: one buffer for the products of a prompt step, which run one behind the
+    other, and one each for those of a step of single tokens, which may run side by side."""
+    name = out_name + ".pieces" if step.all_decode else "linear.pieces"
+    return step.ws.buffer(name, K.linear_f32_tc5_pieces(*x.shape), torch.bfloat16)
 
 
 _MM_OUT_DTYPE_WITH_OUT = None

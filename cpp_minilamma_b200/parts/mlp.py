@@ -18,7 +18,7 @@ import torch
 
 from ..csrc import kernels as K
 from .base import BuildContext, FeedForward, PreNormed, WeightSpec, register_part
-from .linear import Linear
+from .linear import Linear, f32_pieces
 
 INTERLEAVE = 8
 
@@ -111,6 +111,10 @@ class SwiGLUFeedForward(FeedForward):
               and K.linear_f32_supported(values, w, self.epilogue) and not torch.backends.cuda.matmul.allow_tf32):
             act = step.ws.buffer("act", (rows, self.inter), torch.float32)
             K.linear_f32(values, w, None, act, self.epilogue)
+        elif (self.block == INTERLEAVE and K.linear_f32_tc5_pays(values, w, self.epilogue)
+              and not torch.backends.cuda.matmul.allow_tf32):
+            act = step.ws.buffer("act", (rows, self.inter), torch.float32)
+            K.linear_f32_tc5(values, w, None, f32_pieces(step, values, "gu"), act, self.epilogue)
         elif (row_norm is not None and w.dtype == torch.bfloat16 and self.inter % 8 == 0
               and not K.small_linear_kind(rows, 2 * self.inter, w.shape[1], K.EPI_BF16)):
             # the library product cannot finish the norm in front of it: it runs on the rows as they are and

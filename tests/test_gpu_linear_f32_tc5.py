@@ -1,0 +1,109 @@
+"""float32 products of many rows on the tensor cores, against float64.
+
+A float32 operand is split without loss, so what is left are the sums: 32 columns at a time in tensor memory, cut twice per
+sum of the large products, and one rounding a stage in registers.  An element's error is bounded by (K / 32 + 8) * 2^-23 times
+the sum of its products' magnitudes; the tests hold it to a quarter of that and the norm of all to 1e-6."""
+import numpy as np
+import pytest
+import torch
+
+import cpp_minilamma_b200 as ml
+from cpp_minilamma_b200 import api
+from cpp_minilamma_b200.csrc import kernels as K
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(M, N, k, seed=0):
+    g = torch.Generator(device="cuda").manual_seed(seed + M * 7 + N * 3 + k)
+    x = torch.randn((M, k), generator=g, device="cuda") * torch.exp(torch.randn((M, 1), generator=g, device="cuda"))
+    w = torch.randn((N, k), generator=g, device="cuda") * 0.05
+    return x, w
+
+
+def _run(x, w, bias=None, epilogue=K.EPI_F32, cols=0, ranks=0):
+    M, N = x.shape[0], w.shape[0]
+    out = torch.full((M, N if epilogue == K.EPI_F32 else N // 2), float("nan"), device="cuda")
+    pieces = torch.full(K.linear_f32_tc5_pieces(M, x.shape[1]), float("nan"), dtype=torch.bfloat16, device="cuda")
+    K.linear_f32_tc5(x, w, bias, pieces, out, epilogue, cols, ranks)
+    assert K.take_device_error() == 0
+    return out
+
+
+def _check(y, x, w, bias=None):
+    want = x.double() @ w.double().t()
+    bound = (x.shape[1] / 32 + 8) * 2.0 ** -23 / 4 * (x.double().abs() @ w.double().abs().t())
+    if bias is not None:
+        want = want + bias.double()
+        bound = bound + 2.0 ** -23 * want.abs()
+    assert ((y.double() - want).abs() <= bound + 1e-30).all()
+    assert ((y.double() - want).norm() / want.norm()).item() < 1e-6
+
+
+@pytest.mark.parametrize("M,N,k,cols,ranks", [
+    (1, 1, 4, 0, 0), (16, 128, 32, 16, 1), (17, 129, 36, 32, 1), (33, 136, 100, 0, 0), (255, 127, 260, 256, 1), (257, 256, 512, 0, 0),
+    (100, 384, 2048, 112, 2), (240, 130, 1028, 240, 4), (475, 256, 2048, 240, 8), (130, 512, 288, 128, 8), (300, 64, 96, 48, 1),
+    (2049, 128, 64, 0, 0)])
+def test_against_float64(M, N, k, cols, ranks):
+    x, w = _case(M, N, k)
+    bias = torch.randn(N, device="cuda") if N % 2 == 0 else None
+    y = _run(x, w, bias, cols=cols, ranks=ranks)
+    _check(y, x, w, bias)
+    assert torch.equal(y, _run(x, w, bias, cols=cols, ranks=ranks))  # the same on every run
+
+
+@pytest.mark.parametrize("epilogue", [K.EPI_SWIGLU, K.EPI_GEGLU])
+@pytest.mark.parametrize("M,N,k,ranks", [(20, 16, 64, 1), (130, 272, 512, 2), (70, 400, 100, 1)])
+def test_gated(epilogue, M, N, k, ranks):
+    x, w = _case(M, N, k)
+    y = _run(x, w, epilogue=epilogue, ranks=ranks)
+    both = (x.double() @ w.double().t()).view(M, N // 16, 2, 8)
+    form = torch.nn.functional.silu if epilogue == K.EPI_SWIGLU else (lambda t: torch.nn.functional.gelu(t, approximate="tanh"))
+    want = (form(both[:, :, 0]) * both[:, :, 1]).reshape(M, N // 2)
+    assert ((y.double() - want).norm() / want.norm()).item() < 2e-6
+
+
+@pytest.mark.parametrize("ranks", [1, 4])
+def test_numbers_at_the_edges(ranks):
+    """Infinities, NaN, the largest and the smallest numbers give what a chain of float32 operations gives."""
+    x, w = _case(40, 128, 1024)
+    x[3, 5] = float("inf")
+    x[4, 6], w[:, 6] = float("-inf"), w[:, 6].abs() + 1.0  # exact in bfloat16 or not: the product is -infinity
+    w[7, 6] = 2.0
+    x[5, 7] = float("nan")
+    x[6] = 0.0
+    x[6, 9], w[:, 9] = torch.finfo(torch.float32).max, 0.5
+    x[8] = 0.0
+    x[8, 11], w[:, 11] = 1e-38, 1.0
+    w[20] = 0.0
+    y = _run(x, w, ranks=ranks)
+    want = x.double() @ w.double().t()
+    assert torch.equal(torch.isnan(y), torch.isnan(want)) and torch.equal(torch.isinf(y), torch.isinf(want))
+    inf = torch.isinf(want)
+    assert torch.equal(y[inf].sign(), want[inf].sign().float())
+    assert (y[6] == want[6].float()).all()
+    assert ((y[8].double() - want[8]).abs() <= 1e-40).all()
+    rows = [0, 1, 2, 7] + list(range(9, 40))
+    _check(y[rows], x[rows], w)
+
+
+def test_a_prompt_in_a_float32_model_takes_it(monkeypatch):
+    taken = []
+    real = K.linear_f32_tc5
+    monkeypatch.setattr(K, "linear_f32_tc5", lambda *a, **k: (taken.append(1), real(*a, **k))[1])
+    config = ml.config_from_dict({"architectures": ["LlamaForCausalLM"], "vocab_size": 257, "hidden_size": 512, "intermediate_size": 1024,
+                                  "num_hidden_layers": 2, "num_attention_heads": 8, "num_key_value_heads": 4, "head_dim": 64,
+                                  "max_position_embeddings": 1024, "rope_theta": 10000.0, "rms_norm_eps": 1e-5, "torch_dtype": "float32"})
+    logits = []
+    for pays in (True, False):
+        if not pays:
+            monkeypatch.setattr(K, "linear_f32_tc5_pays", lambda *a, **k: False)
+        model = ml.build_model(config, "float32", torch.device("cuda:0"), 1024)
+        g = torch.Generator(device="cuda").manual_seed(5)
+        model.bind({s.name: torch.randn(tuple(s.shape), generator=g, device="cuda") * 0.05 for s in model.weight_specs()})
+        llm = api.LLM(config, model, max_tokens=1024, max_seqs=1)
+        slot = llm.engine.acquire(1)[0]
+        prompt = [int(t) for t in np.random.RandomState(1).randint(0, 200, 700)]
+        logits.append(llm.step([ml.StepEntry(slot, prompt, [0, 350, 699])]).cpu().numpy().copy())
+    assert taken
+    np.testing.assert_allclose(logits[0], logits[1], rtol=0, atol=2e-5 * np.abs(logits[1]).max())
