@@ -6,7 +6,11 @@
 // float32, and what remains is the sum's rounding: the tensor cores cut their running sum after every step instead of rounding it,
 // which over a long K would cost more than a chain of float32 additions does.  So 32 columns of k are summed up in tensor memory,
 // the small products first, and then added to float32 registers.
-// Bound: the tensor pipe, at a sixth of its bfloat16 rate.
+// Bound: shared memory's bandwidth (the products' operands, 98 bytes a clock, beside the copies and the splitting, 50) at many rows, a
+// stage's fixed work of some 1,100 clocks at few.  In a CUDA graph, us, this kernel (the splitting of x with it) / the library's SGEMM on the
+// multiprocessors' FMA units, 475 rows of the 1B shape: o 39 / 85, q/k/v 55 / 142, gate/up 185 / 575, down 96 / 328 (164
+// TFLOP/s of float32 products); 17 rows, gate/up 51 / 69, down 54 / 89; 2,048 rows, 665 / 2,130 and 349 / 1,244.  Its error against 64 bits
+// there is 1.3e-7 to 3e-7 of the result, the library's 5e-7 to 1.6e-6.
 //
 // A block forms 128 weight rows (the M operand) times up to 256 rows of x (the N operand) over a slice of K, 32 columns a stage:
 //   warp 12    loads the three pieces of x, split by a kernel in front (x is small and every column of blocks reads it again) that
@@ -178,11 +182,11 @@ __device__ __noinline__ float x_chain(const float* x, const float* w, int K) {
 }
 
 // Row m of the result for a warp of weight rows (lane: row n), all lanes present
-__device__ __forceinline__ void x_write(const LinearX3Args& a, float v, int m, int n) {
+__device__ __forceinline__ void x_write(const LinearX3Args& a, float v, float bias, int m, int n) {
   const bool in = m < a.M && n < a.N;
   if (in && !isfinite(v)) v = x_chain(a.x + (size_t)m * a.K, a.w + (size_t)n * a.K, a.K);
   if (a.epilogue == XEPI_F32) {
-    if (in) a.out[(size_t)m * a.N + n] = a.bias ? v + a.bias[n] : v;
+    if (in) a.out[(size_t)m * a.N + n] = v + bias;
   } else {  // gate rows 0-7, up rows 8-15 of every 16
     const float up = __shfl_down_sync(0xffffffffu, v, 8);
     if (in && (n & 8) == 0)
@@ -283,14 +287,22 @@ __global__ void __launch_bounds__(X_THREADS, 1) linear_f32_tc5_kernel(const __gr
     if (CLUSTER) x_cluster_sync();
     else asm volatile("bar.sync 1, 256;" ::: "memory");
     const int per = (a.cols + ranks - 1) / ranks, from = rank * per, to = min(a.cols, from + per);
+    const int n = n0 + r0;
+    const float bias = a.bias != nullptr && n < a.N ? a.bias[n] : 0.f;
+    // a warp has its 32 weight rows of every other column, four columns at a time: their reads from the other blocks are in flight
+    // together
 #pragma unroll 1
-    for (int i = from * 4 + warp; i < to * 4; i += X_SUMMERS) {
-      const int c = i >> 2, r = (i & 3) * 32 + lane;
-      float s = 0.f;
-      if (CLUSTER)
-        for (int j = 0; j < ranks; ++j) s += cg::this_cluster().map_shared_rank(part, j)[(size_t)c * wide + r];
-      else s = part[(size_t)c * wide + r];
-      x_write(a, s, m0 + c, n0 + r);
+    for (int c = from + group; c < to; c += 8) {
+      float s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 2
+      for (int j = 0; j < ranks; ++j) {
+        const float* there = (CLUSTER ? cg::this_cluster().map_shared_rank(part, j) : part) + r0;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) s[u] += there[min(c + 2 * u, to - 1) * wide];
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (c + 2 * u < to) x_write(a, s[u], bias, m0 + c + 2 * u, n);
     }
     if (CLUSTER) x_cluster_sync();
   } else if (warp < X_SUMMERS + X_SPLITTERS) {
@@ -447,8 +459,8 @@ int launch_linear_f32_tc5(const CUtensorMap& w_map, const LinearX3Args& a, int r
   return 0;
 }
 
-// How M rows and K are cut up: the fewest rounds of blocks over the device, weighed by a block's time - per 32 columns of k six
-// products of `cols` columns, or the splitting of W if that is longer, and the start and end of a block.
+// How M rows and K are cut up: the fewest rounds of blocks over the device, weighed by a block's time in clocks as measured - 1,270 a
+// stage at 32 columns, 1,550 at 128, 1,980 at 240 - and its start and end.
 struct X3Plan {
   int cols, ranks;
 };
@@ -465,8 +477,8 @@ X3Plan x3_plan(int M, int N, int K) {
       const long long blocks = (long long)tiles * n_tiles * ranks;
       const int resident = sms / ranks * ranks;  // clusters are resident as a whole
       const double rounds = (double)((blocks + resident - 1) / resident);
-      const double stage = cols * 6.0 > 600.0 ? cols * 6.0 : 600.0;
-      const double time = rounds * ((double)((k_blocks + ranks - 1) / ranks) * stage + 8000.0 + (ranks > 1 ? 3000.0 : 0.0));
+      const double stage = 1100.0 + 3.6 * cols;
+      const double time = rounds * ((double)((k_blocks + ranks - 1) / ranks) * stage + 8000.0 + 24.0 * cols + (ranks > 1 ? 2000.0 * ranks : 0.0));
       if (best.cols == 0 || time < least) {
         least = time;
         best = X3Plan{cols, ranks};
@@ -485,10 +497,18 @@ MLL_API int mll_linear_f32_tc5_supported(int M, int N, int K, int epilogue) {
   return (epilogue == mll::XEPI_SWIGLU || epilogue == mll::XEPI_GEGLU) && N % 16 == 0;
 }
 
-// Whether it takes this problem and is the faster way (us, the library / here).
+// Whether it takes this problem and is the faster way (us, the library / here).  The library's time is a chain over K where few
+// blocks run, this kernel's a fixed 8 to 12 at least.  Long rows: always (17 rows, 256 x 1,024 13.6 / 13.1; 475 rows, 2,048 x 2,048
+// 85 / 39), but not for a handful of weight rows, which a tile of 128 is mostly empty for (4,000 rows, 16 x 2,048 36 / 54; 2,048
+// rows, 64 x 4,096 66 / 40).  Shorter rows: where results are many (512: 256 rows of 2,048 16.6 / 17.9, of 8,192 45 / 26; 256:
+// 1,024 rows of 512 9.9 / 18.4, of 2,048 25.5 / 19.0), the shortest not at all (1,024 rows, 2,048 x 128 15.6 / 15.5; 2,048 rows, 1,024
+// x 192 20.7 / 25.4).  Few rows are the weight-streaming kernel's (linear_f32.cu) but for tall matrices from 9 rows on (16 rows, 16,384
+// x 2,048, that kernel / here 65 / 50).
 MLL_API int mll_linear_f32_tc5_pays(int M, int N, int K, int epilogue) {
-  if (!mll_linear_f32_tc5_supported(M, N, K, epilogue) || M <= 16) return 0;
-  return (double)M * N * K >= 1.0e9;
+  if (!mll_linear_f32_tc5_supported(M, N, K, epilogue) || M < 9 || N < 64 || K < 256) return 0;
+  if (M <= 16) return N >= 16384 && K >= 1024;
+  if (K >= 1024) return 1;
+  return (long long)M * N >= (K >= 512 ? 1000000 : 1500000);
 }
 
 // x: float32 [M, K]; w: float32 [N, K]; bias: optional float32 [N]; pieces: room for [K / 32 rounded up, 3, M + 256, 32] bfloat16; out

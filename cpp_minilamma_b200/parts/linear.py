@@ -76,9 +76,9 @@ class Linear:
                 x = wide
             if out_dtype == torch.float32:
                 out = given if given is not None else ws.buffer(out_name, (rows, self.out_features), torch.float32)
-                return self._product_f32(step, x, out_name, out)
+                return self._product_f32(step, x, out, out_name)
             wide_out = ws.buffer(out_name + ".y32", (rows, self.out_features), torch.float32)
-            self._product_f32(step, x, out_name, wide_out)
+            self._product_f32(step, x, wide_out, out_name)
             out = given if given is not None else ws.buffer(out_name, (rows, self.out_features), out_dtype)
             K.cast(wide_out, out)
             return out
@@ -105,12 +105,12 @@ class Linear:
             _mm_bf16_to_f32(x, w, out)
         return self._biased(out)
 
-    def _product_f32(self, step, x: torch.Tensor, out_name: str, out: torch.Tensor) -> torch.Tensor:
-        if x.shape[0] <= step.small_rows and out.is_contiguous() and K.linear_f32_pays(x, self.weight):
-            K.linear_f32(x, self.weight, self.bias, out)
-            return out
+    def _product_f32(self, step, x: torch.Tensor, out: torch.Tensor, out_name: str = "linear") -> torch.Tensor:
         if out.is_contiguous() and K.linear_f32_tc5_pays(x, self.weight):
             K.linear_f32_tc5(x, self.weight, self.bias, f32_pieces(step, x, out_name), out)
+            return out
+        if x.shape[0] <= step.small_rows and out.is_contiguous() and K.linear_f32_pays(x, self.weight):
+            K.linear_f32(x, self.weight, self.bias, out)
             return out
         torch.mm(x, self.weight.t(), out=out)
         return self._biased(out)

@@ -107,14 +107,14 @@ class SwiGLUFeedForward(FeedForward):
             # few rows: one weight-streaming kernel whose epilogue applies the activation
             act = step.ws.buffer("act", (rows, self.inter), torch.bfloat16)
             K.small_linear(values, w, None, act, self.epilogue, row_norm)
+        elif (self.block == INTERLEAVE and not torch.backends.cuda.matmul.allow_tf32
+              and K.linear_f32_tc5_pays(values, w, self.epilogue)):
+            act = step.ws.buffer("act", (rows, self.inter), torch.float32)
+            K.linear_f32_tc5(values, w, None, f32_pieces(step, values, "gu"), act, self.epilogue)
         elif (rows <= step.small_rows and self.block == INTERLEAVE
               and K.linear_f32_supported(values, w, self.epilogue) and not torch.backends.cuda.matmul.allow_tf32):
             act = step.ws.buffer("act", (rows, self.inter), torch.float32)
             K.linear_f32(values, w, None, act, self.epilogue)
-        elif (self.block == INTERLEAVE and K.linear_f32_tc5_pays(values, w, self.epilogue)
-              and not torch.backends.cuda.matmul.allow_tf32):
-            act = step.ws.buffer("act", (rows, self.inter), torch.float32)
-            K.linear_f32_tc5(values, w, None, f32_pieces(step, values, "gu"), act, self.epilogue)
         elif (row_norm is not None and w.dtype == torch.bfloat16 and self.inter % 8 == 0
               and not K.small_linear_kind(rows, 2 * self.inter, w.shape[1], K.EPI_BF16)):
             # the library product cannot finish the norm in front of it: it runs on the rows as they are and

@@ -91,8 +91,8 @@ def test_a_prompt_in_a_float32_model_takes_it(monkeypatch):
     taken = []
     real = K.linear_f32_tc5
     monkeypatch.setattr(K, "linear_f32_tc5", lambda *a, **k: (taken.append(1), real(*a, **k))[1])
-    config = ml.config_from_dict({"architectures": ["LlamaForCausalLM"], "vocab_size": 257, "hidden_size": 512, "intermediate_size": 1024,
-                                  "num_hidden_layers": 2, "num_attention_heads": 8, "num_key_value_heads": 4, "head_dim": 64,
+    config = ml.config_from_dict({"architectures": ["LlamaForCausalLM"], "vocab_size": 257, "hidden_size": 1024, "intermediate_size": 1024,
+                                  "num_hidden_layers": 2, "num_attention_heads": 16, "num_key_value_heads": 4, "head_dim": 64,
                                   "max_position_embeddings": 1024, "rope_theta": 10000.0, "rms_norm_eps": 1e-5, "torch_dtype": "float32"})
     logits = []
     for pays in (True, False):
