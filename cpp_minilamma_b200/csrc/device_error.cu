@@ -7,6 +7,8 @@
 // kernel that gave up without any copy or wait of its own.  mll_raise_device_error() sets flags from
 // the host, for tests of the host's reaction: no kernel has to fail for them.
 // The reference has no counterpart: its kernels have no waits that could run out.
+#include <mutex>
+
 #include "common.cuh"
 #include "device_error.h"
 
@@ -40,21 +42,30 @@ bool mll_device_error_words(MllDeviceErrorWords* words) {
   return true;
 }
 
-// The flags as a bit mask (see device_error.h), cleared; -1 if they cannot be read.  Synchronises.
+// one warp: the flags as a bit mask, cleared
+__global__ void take_device_error_kernel(MllDeviceErrorWords words, volatile int* mask) {
+  const int flag = threadIdx.x < 4 ? atomicExch(words.word[threadIdx.x], 0) : 0;
+  const unsigned set = __ballot_sync(0xffffffffu, flag != 0);
+  if (threadIdx.x == 0) *mask = (int)set;
+}
+
+// The flags as a bit mask (see device_error.h), cleared; -1 if they cannot be read.  Synchronises.  Bound: the wait that ends a step;
+// one kernel that writes to the host's memory in place of a copy a flag, each with a wait of its own (four of 3 us on the device and
+// some 8 on the host).
 MLL_API int mll_take_device_error() {
   MllDeviceErrorWords words;
   if (!mll_device_error_words(&words)) return -1;
-  int mask = 0;
-  const int zero = 0;
-  for (int i = 0; i < 4; ++i) {
-    int flag = 0;
-    if (cudaMemcpy(&flag, words.word[i], sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) return -1;
-    if (flag) {
-      if (cudaMemcpy(words.word[i], &zero, sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess) return -1;
-      mask |= 1 << i;
-    }
+  static std::mutex lock;
+  static int* mask = nullptr;  // pinned, for all devices; the lock keeps calls apart
+  std::lock_guard<std::mutex> guard(lock);
+  if (mask == nullptr && cudaHostAlloc((void**)&mask, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+    cudaGetLastError();
+    mask = nullptr;
+    return -1;
   }
-  return mask;
+  take_device_error_kernel<<<1, 32, 0, cudaStreamLegacy>>>(words, mask);
+  if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess) return -1;
+  return *(volatile int*)mask;
 }
 
 // Sets the flags named in `mask` as a kernel that gave up would (for tests of the host side).
