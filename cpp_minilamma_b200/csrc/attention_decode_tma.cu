@@ -322,7 +322,7 @@ __device__ __forceinline__ void dt_page_step(const DecodeMmaArgs& a, unsigned ch
 template <int D, int DV, bool FUSED, bool CLUSTER>
 __global__ void __launch_bounds__(DT_THREADS, 2)
 attn_decode_tma_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap,
-                       DecodeMmaArgs a) {
+                       DecodeMmaArgs a, int early) {
   using L = DecodeTmaSmem<D, DV>;
   constexpr int KSTEPS = D / 16;  // k-steps of the score product
   constexpr int NT = DV / 8;      // output n-tiles (8 columns) per warp: every warp holds all columns
@@ -339,6 +339,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_co
   const int chunks = (group + 15) / 16;
   // sequences are the slower grid index, so blocks start in the order of `seq_order` (longest contexts first);
   // with a work list the slower index runs over its (sequence, split) pairs instead
+  if (early) grid_wait();
   const int entry = !CLUSTER && a.work != nullptr ? a.work[blockIdx.y] : 0;
   if (entry < 0) return;  // an unused place of the list (the same for the whole block)
   const bool listed = !CLUSTER && a.work != nullptr;
@@ -455,6 +456,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_co
       }
     }
 
+    if (early) grid_let_next_start();
     // ---- the four warps' partial results, merged through the drained ring --------------------- //
     __syncthreads();  // every page has been consumed: the ring is free
     if (warp < 4) {
@@ -556,16 +558,22 @@ int launch_decode_tma_as(const CUtensorMap& kmap, const CUtensorMap& vmap, const
   config.blockDim = dim3(DT_THREADS);
   config.dynamicSmemBytes = smem;
   config.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
+  config.attrs = attr;
   if (CLUSTER) {
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 1;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = a.n_splits;
-    config.attrs = attr;
     config.numAttrs = 1;
   }
-  err = cudaLaunchKernelEx(&config, kernel, kmap, vmap, a);
+  // (fused: the kernel before is the q/k/v product)
+  const int early = FUSED && a.work == nullptr ? mll_starts_early(n_seqs, a.n_heads * D) : 0;
+  if (early) {
+    attr[config.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[config.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  err = cudaLaunchKernelEx(&config, kernel, kmap, vmap, a, early);
   if (err != cudaSuccess) {
     mll_set_error("attention decode (tma): launch failed: %s", cudaGetErrorString(err));
     return (int)err;

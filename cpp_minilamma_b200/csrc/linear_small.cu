@@ -17,6 +17,8 @@
 //   * epilogue EPI_RESID adds the result to the float32 residual stream, and writes the new row times the
 //     next norm's weight, in bfloat16, with the tile's share of the row's sum of squares.
 //
+// In narrow models' steps of up to four rows the chain of short kernels overlaps at its seams (mll_starts_early, common.cuh).
+//
 // The reference calls cublasSgemm with rows = 1 for every linear (src/cuda_matmul.cc:181-186).
 #include <cooperative_groups.h>
 
@@ -39,6 +41,7 @@ struct LinearArgs {
   const float* next_w;     // EPI_RESID: weight [N] of the norm that follows
   float* out_sumsq;        // EPI_RESID: [M, out_stride], entry [m][tile] = sum over the tile's columns of resid^2
   int out_stride;
+  int early;               // launched while the kernel before may still run: wait for it, and let the next one start early in turn
 };
 
 __device__ __forceinline__ uint4 ldg_stream(const void* p) {
@@ -104,6 +107,7 @@ linear_small_kernel(LinearArgs a) {
   for (int n = 0; n < NT; ++n)
 #pragma unroll
     for (int i = 0; i < 4; ++i) acc[n][i] = 0.f;
+  if (a.early) grid_wait();
 
   // At most 16 rows and 8 warps: warp m works out the norm factors of rows m and m + 8 now, before its loop.  The partial sums lie
   // in the L2 cache, so this is one cache latency (0.5 us); the warp first asks the L2 cache for the weights of its
@@ -180,6 +184,8 @@ linear_small_kernel(LinearArgs a) {
       mma_bf16(acc[n], ta.z, tb.z, ta.w, tb.w, fx.z, fx.w);
     }
   }
+
+  if (a.early) grid_let_next_start();
 
   // this warp's 16 x (8 NT) partial tile: rows g and g + 8, batch columns n * 8 + 2 t + {0, 1}
 #pragma unroll
@@ -298,6 +304,11 @@ int launch_linear_small(const LinearArgs& a, int tiles, int ranks, cudaStream_t 
   cudaError_t err;
   config.attrs = attr;
   config.numAttrs = 0;
+  if (a.early) {
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    config.numAttrs = 1;
+  }
   if (ranks > 1) {
     attr[config.numAttrs].id = cudaLaunchAttributeClusterDimension;
     attr[config.numAttrs].val.clusterDim.x = ranks;
@@ -371,7 +382,7 @@ MLL_API int mll_linear_small_fused(const void* x, const void* w, const float* bi
   }
   MLL_REQUIRE(ranks == 1 || ranks == 2 || ranks == 4 || ranks == 8, "linear_small: cluster size %d", ranks);
   mll::LinearArgs a{(const __nv_bfloat16*)x, (const __nv_bfloat16*)w, bias, out, M, N, K, epilogue, 0,
-                    mll::RowNormIn{in_sumsq, in_partials, in_stride, in_eps}, resid, next_w, out_sumsq, out_stride};
+                    mll::RowNormIn{in_sumsq, in_partials, in_stride, in_eps}, resid, next_w, out_sumsq, out_stride, mll_starts_early(M, N < K ? N : K)};
   const int splits = warps * ranks;
   a.chunks_per_warp = (chunks + splits - 1) / splits;
   if (M <= 8) {
