@@ -76,11 +76,17 @@ struct PrefillTc5Args {
   int keep_first;            // with a window: keys at positions below this stay visible
   float scale_over_cap;      // scale / cap, and cap / scale: a raw score s becomes (cap / scale) tanh(s scale / cap),
   float cap_over_scale;      // which the scale then turns into cap * tanh(..); both 0 without a cap
-  static constexpr bool GATED = false, MIXED = false;
+  static constexpr bool GATED = false, MIXED = false, LATENT = false;
 };
 // The same with every other pair of exponentials on the FMA pipe (see `mixed_pays`)
 struct PrefillTc5MixedArgs : PrefillTc5Args {
   static constexpr bool MIXED = true;
+};
+// The same for attention over a latent: one kv head whose values are the leading columns of its keys, sizes of their own.  The
+// kernel's D and DV are then the most they may be.
+struct PrefillTc5LatentArgs : PrefillTc5Args {
+  static constexpr bool LATENT = true;
+  int boxes, dv;  // 64-column boxes of a query or key row; value columns, a multiple of 8
 };
 // The same for heads with a gate each.  A type of its own: the kernel without gates then compiles to what it was (the two
 // more parameters alone moved its register allocation: 63 -> 67 us for 2,048 tokens of 32 heads of 128).
@@ -299,15 +305,15 @@ __device__ __forceinline__ void a_mbar_arrive(unsigned bar) {
 constexpr int A_SOFTMAX_REGS = 168, A_OTHER_REGS = 40;
 constexpr float A_RESCALE_STEP = 8.f;  // the output is rescaled only when a row's maximum grows by more than 2^8
 
-template <int D, int DV>
+template <int D, int DV, bool LATENT = false>
 struct PrefillTc5Smem {
   static constexpr int THREADS = 256;
-  static constexpr int KV_STAGES = D == 64 && DV == 64 ? 3 : 2;  // at most 80 KB a block
+  static constexpr int KV_STAGES = LATENT ? 4 : D == 64 && DV == 64 ? 3 : 2;  // at most 80 KB a block
   static constexpr int Q_BYTES = A_ROWS * D * 2;       // D / 64 boxes of [128 rows x 128 bytes]
   static constexpr int K_BYTES = MLL_PAGE * D * 2;     // D / 64 boxes of [64 rows x 128 bytes]
   static constexpr int V_BYTES = MLL_PAGE * DV * 2;    // DV / 64 boxes
-  static constexpr int Q_OFF = 0, K_OFF = Q_BYTES, V_OFF = K_OFF + KV_STAGES * K_BYTES;
-  static constexpr int BAR_OFF = V_OFF + KV_STAGES * V_BYTES;
+  static constexpr int Q_OFF = 0, K_OFF = Q_BYTES, V_OFF = LATENT ? K_OFF : K_OFF + KV_STAGES * K_BYTES;
+  static constexpr int BAR_OFF = V_OFF + KV_STAGES * (LATENT ? K_BYTES : V_BYTES);
   // Two blocks per multiprocessor (their tensor memory: 2 x 256 columns); never three: the request
   // is padded above a third of the shared memory.  The kernel checks that its dynamic shared
   // memory starts on a 1024-byte boundary (the swizzle's period) and refuses otherwise.
@@ -317,7 +323,7 @@ struct PrefillTc5Smem {
   // for two S buffers, value size 64 for three: the chain softmax -> P V -> S -> softmax that bounds a block's pace
   // then runs over three pages instead of two.
   static constexpr int S_BUFS = DV == 64 ? 3 : 2;
-  static constexpr int TMEM_COLS = 256;
+  static constexpr int TMEM_COLS = LATENT ? 512 : 256;  // (a latent's block has a multiprocessor to itself)
   static constexpr int O_COL = S_BUFS * MLL_PAGE;
   static_assert(O_COL + DV <= TMEM_COLS, "S buffers and O must fit the block's columns");
   // barrier slots: the queries; keys and values full / empty per ring stage; per S buffer: S full, P ready,
@@ -330,10 +336,10 @@ struct PrefillTc5Smem {
 };
 
 template <int D, int DV, typename Args>
-__global__ void __launch_bounds__(PrefillTc5Smem<D, DV>::THREADS, 2)
+__global__ void __launch_bounds__(PrefillTc5Smem<D, DV, Args::LATENT>::THREADS, 2)
 attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap kmap,
                         const __grid_constant__ CUtensorMap vmap, Args a) {
-  using L = PrefillTc5Smem<D, DV>;
+  using L = PrefillTc5Smem<D, DV, Args::LATENT>;
   constexpr int DB = D / 64, VB = DV / 64;  // 64-column boxes per row of Q and K, and of V
   constexpr int KS = L::KV_STAGES, SB = L::S_BUFS;
   constexpr int LOAD_WARP = 4, MMA_WARP = 5, PV_WARP = 6;
@@ -360,6 +366,11 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_c
   };
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  int boxes = DB, dv = DV;  // constants but for a latent
+  if constexpr (Args::LATENT) {
+    boxes = a.boxes;
+    dv = a.dv;
+  }
   const int seq = a.tile_seq[tile];
   const int h = blockIdx.x % a.n_heads;
   const int kvh = h / (a.n_heads / a.n_kv_heads);
@@ -398,21 +409,22 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_c
   if (warp == LOAD_WARP) {
     // ---- loads: the query tile once, then key and value pages into the ring ----------------- //
     if (lane == 0) {
-      a_mbar_expect_tx(bar(L::AB_Q, 0), L::Q_BYTES);
+      a_mbar_expect_tx(bar(L::AB_Q, 0), boxes * (A_ROWS * 128));
 #pragma unroll
       for (int b = 0; b < DB; ++b)
-        a_tma_load_2d(q_s + b * (A_ROWS * 128), &qmap, h * D + b * 64, qstart + row0, bar(L::AB_Q, 0));
+        if (b < boxes) a_tma_load_2d(q_s + b * (A_ROWS * 128), &qmap, (h * boxes + b) * 64, qstart + row0, bar(L::AB_Q, 0));
       int page = table[page_at(0)];
       for (int i = 0; i < n_pages && !*abort_flag; ++i) {
         const int st = i % KS;
         const unsigned parity = ((i / KS) & 1) ^ 1;  // the stage's previous use (none in the first round)
         const int row = (page * a.n_kv_heads + kvh) * MLL_PAGE;
         if (i + 1 < n_pages) page = table[page_at(i + 1)];  // looked up while this page's loads fly
-        wait(bar(L::AB_K_EMPTY, st), parity);
-        a_mbar_expect_tx(bar(L::AB_K_FULL, st), L::K_BYTES);
+        wait(bar(Args::LATENT ? L::AB_V_EMPTY : L::AB_K_EMPTY, st), parity);  // a latent's page is free once its P V is done
+        a_mbar_expect_tx(bar(L::AB_K_FULL, st), boxes * (MLL_PAGE * 128));
 #pragma unroll
         for (int b = 0; b < DB; ++b)
-          a_tma_load_2d(k_s + st * L::K_BYTES + b * (MLL_PAGE * 128), &kmap, b * 64, row, bar(L::AB_K_FULL, st));
+          if (b < boxes) a_tma_load_2d(k_s + st * L::K_BYTES + b * (MLL_PAGE * 128), &kmap, b * 64, row, bar(L::AB_K_FULL, st));
+        if constexpr (Args::LATENT) continue;
         wait(bar(L::AB_V_EMPTY, st), parity);
         a_mbar_expect_tx(bar(L::AB_V_FULL, st), L::V_BYTES);
 #pragma unroll
@@ -442,24 +454,24 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_c
         for (int b = 0; b < DB; ++b)
 #pragma unroll
           for (int k = 0; k < 4; ++k)
-            a_umma(d, q_desc + (unsigned long long)((b * (A_ROWS * 128) + k * 32) >> 4),
+            if (b < boxes) a_umma(d, q_desc + (unsigned long long)((b * (A_ROWS * 128) + k * 32) >> 4),
                    kd + (unsigned long long)((b * (MLL_PAGE * 128) + k * 32) >> 4), idesc_s, (b > 0 || k > 0) ? 1u : 0u);
         a_commit(bar(L::AB_S_FULL, sb));
-        a_commit(bar(L::AB_K_EMPTY, st));
+        if (!Args::LATENT) a_commit(bar(L::AB_K_EMPTY, st));
       }
       __syncwarp();
     }
   } else if (warp == PV_WARP) {
     // ---- O += P V, a warp of its own: with one thread for both products a page's MMAs went out one behind
     // the other with their waits in between, and the softmax warps waited
-    constexpr unsigned idesc_o = a_idesc(A_ROWS, DV, true);
+    const unsigned idesc_o = a_idesc(A_ROWS, (dv + 15) / 16 * 16, true);
     for (int i = 0; i < n_pages; ++i) {
       const int sb = i % SB, st = i % KS;
-      wait(bar(L::AB_V_FULL, st), (i / KS) & 1);
+      if (!Args::LATENT) wait(bar(L::AB_V_FULL, st), (i / KS) & 1);
       wait(bar(L::AB_P_READY, sb), (i / SB) & 1);
       a_fence_after();
       if (__any_sync(0xffffffffu, *abort_flag)) break;
-      const unsigned long long vd = a_desc(v_s + st * L::V_BYTES, MLL_PAGE * 128);
+      const unsigned long long vd = a_desc(v_s + st * (Args::LATENT ? L::K_BYTES : L::V_BYTES), MLL_PAGE * 128);
       if (a_elect()) {
 #pragma unroll
         for (int k = 0; k < 4; ++k)  // P: 16 keys = 8 packed columns per step
@@ -525,6 +537,7 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_c
         a_fence_after();
 #pragma unroll
         for (int c = 0; c < DV; c += 32) {
+          if (c >= dv) break;
           float o[32];
           a_tmem_ld32(tmem_row + L::O_COL + c, o);
 #pragma unroll
@@ -566,10 +579,10 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_c
       a_tmem_st32(tmem_row + sb * MLL_PAGE, packed);  // P over the first half of S
       const int valid = ctx - k0;  // positions of this page that the sequence has
       if (valid < MLL_PAGE) {      // only the sequence's last page: the rest of it may hold anything
-        wait(bar(L::AB_V_FULL, st), (i / KS) & 1);
-        unsigned char* vt = base + L::V_OFF + st * L::V_BYTES;
+        if (!Args::LATENT) wait(bar(L::AB_V_FULL, st), (i / KS) & 1);  // (a latent's scores are there: its page is, and is read no more)
+        unsigned char* vt = base + L::V_OFF + st * (Args::LATENT ? L::K_BYTES : L::V_BYTES);
         const int n_chunks = (MLL_PAGE - valid) * 8;  // 16-byte chunks per box
-        for (int b = 0; b < VB; ++b)
+        for (int b = 0; b < (Args::LATENT ? boxes : VB); ++b)
           for (int c = r; c < n_chunks; c += A_ROWS)
             *reinterpret_cast<uint4*>(vt + b * (MLL_PAGE * 128) + valid * 128 + c * 16) = make_uint4(0, 0, 0, 0);
         a_fence_async_smem();
@@ -592,14 +605,16 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_c
       const bool store = !*abort_flag && r < rows;
       const float inv_l = l_run > 0.f ? 1.f / l_run : 0.f;
       const float inv = Args::GATED ? inv_l / (1.f + expf(-gate_z)) : inv_l;
-      __nv_bfloat16* dst = a.out + ((size_t)qstart + row0 + (store ? r : 0)) * a.n_heads * DV + (size_t)h * DV;
+      __nv_bfloat16* dst = a.out + ((size_t)qstart + row0 + (store ? r : 0)) * a.n_heads * dv + (size_t)h * dv;
 #pragma unroll
       for (int c = 0; c < DV; c += 32) {
+        if (c >= dv) break;
         float o[32];
         a_tmem_ld32(tmem_row + L::O_COL + c, o);
         if (store) {
 #pragma unroll
           for (int j = 0; j < 32; j += 8) {
+            if (c + j >= dv) break;
             uint4 w;
             __nv_bfloat162* hp = reinterpret_cast<__nv_bfloat162*>(&w);
 #pragma unroll
@@ -626,7 +641,7 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_c
 template <int D, int DV, typename Args>
 int launch_prefill_tc5_as(const CUtensorMap& qmap, const CUtensorMap& kmap, const CUtensorMap& vmap,
                           const Args& a, int n_tiles, cudaStream_t stream) {
-  using L = PrefillTc5Smem<D, DV>;
+  using L = PrefillTc5Smem<D, DV, Args::LATENT>;
   const size_t smem = L::BYTES;
   auto kernel = attn_prefill_tc5_kernel<D, DV, Args>;
   cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -712,4 +727,35 @@ MLL_API int mll_attn_prefill_tc5(const void* q, const void* k_cache, const void*
   if (head_dim == 64) return mll::launch_prefill_tc5<64, 128>(qmap, kmap, vmap, a, n_tiles, stream);
   if (v_head_dim == 64) return mll::launch_prefill_tc5<128, 64>(qmap, kmap, vmap, a, n_tiles, stream);
   return mll::launch_prefill_tc5<128, 128>(qmap, kmap, vmap, a, n_tiles, stream);
+}
+
+// Whether mll_attn_prefill_latent_tc5 takes rows of `row` columns whose first `value` are their values.
+MLL_API int mll_attn_prefill_latent_tc5_supported(int row, int value) {
+  return row > 128 && row <= 256 && row % 64 == 0 && value >= 8 && value <= row && value % 8 == 0;
+}
+
+// Prompt attention over a latent, bfloat16: q [n_tokens, n_heads * row], one cache row of `row` columns a position (cache: pages of 64
+// rows), whose first `value` columns are also its value; out [n_tokens, n_heads * value].  The other arguments as in
+// mll_attn_prefill_tc5.  A block's tensor memory holds two S buffers and up to 256 columns of O, its shared memory the query tile
+// and four pages, so it has a multiprocessor to itself; pages are loaded once for both products.  A request of three
+// prompts (3,970 tokens, 16 heads, rows of 256) 5,440 -> 4,942 us; the kernel before, mma.sync (attention_local_mma.cu), took 364 of them a layer.
+MLL_API int mll_attn_prefill_latent_tc5(const void* q, const void* cache, const int* seq_slot, const int* seq_ctx,
+                                        const int* seq_qstart, const int* seq_qlen, const int* tile_seq, const int* tile_row0,
+                                        const int* block_table, void* out, int n_tokens, long long n_pages, int n_tiles,
+                                        int n_heads, int row, int value, int max_blocks, int window, float scale, int sink,
+                                        const float* sink_values, cudaStream_t stream) {
+  MLL_REQUIRE(mll_attn_prefill_latent_tc5_supported(row, value), "latent attention (tcgen05): rows of %d, values of %d", row, value);
+  MLL_REQUIRE(n_heads > 0 && n_tiles >= 0 && n_tokens >= 0 && (long long)n_tiles * n_heads < (1ll << 31) && window >= 0,
+              "latent attention (tcgen05): bad counts or window");
+  MLL_REQUIRE(n_pages > 0 && n_pages * MLL_PAGE < (1ll << 31), "latent attention (tcgen05): %lld pages are more than the row coordinate holds",
+              n_pages);
+  MLL_REQUIRE(((uintptr_t)q | (uintptr_t)cache | (uintptr_t)out) % 16 == 0, "latent attention (tcgen05): operands must be 16-byte aligned");
+  if (n_tiles == 0 || n_tokens == 0) return 0;
+  CUtensorMap qmap, kmap;
+  if (mll::tensor_map_bf16(q, n_tokens, (long long)n_heads * row, mll::A_ROWS, &qmap) != 0) return -1;
+  if (mll::tensor_map_bf16(cache, n_pages * MLL_PAGE, row, MLL_PAGE, &kmap) != 0) return -1;
+  const mll::PrefillTc5LatentArgs a{{seq_slot, seq_ctx, seq_qstart, seq_qlen, tile_seq, tile_row0, block_table, (__nv_bfloat16*)out,
+                                     n_heads, 1, max_blocks, window, 0, scale * 1.4426950408889634f, (sink || sink_values) ? 1 : 0,
+                                     sink_values, 0, 0.f, 0.f}, row / 64, value};
+  return mll::launch_prefill_tc5_as<256, 256, mll::PrefillTc5LatentArgs>(qmap, kmap, kmap, a, n_tiles, stream);
 }

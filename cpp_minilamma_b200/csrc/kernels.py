@@ -1390,6 +1390,40 @@ def local_attention_tiles(q, k_cache, v_cache, seq_slot, seq_ctx, seq_qstart, se
         "local_attention_mma (window)" if keep_first or softcap else "local_attention_mma")
 
 
+def latent_attention_tc5_supported(dtype: torch.dtype, row: int, value: int) -> bool:
+    """Whether `latent_attention_tiles` takes cache rows of `row` columns whose first `value` are their values."""
+    return (USE_TENSOR_CORE_PREFILL and USE_TCGEN05_PREFILL and dtype == torch.bfloat16
+            and bool(lib().mll_attn_prefill_latent_tc5_supported(row, value)))
+
+
+def latent_attention_tiles(q, cache, seq_slot, seq_ctx, seq_qstart, seq_qlen, tile_seq, tile_row0, block_table, out, n_heads: int,
+                           row: int, value: int, window: int, scale: float, sink: bool = False,
+                           sink_values: Optional[torch.Tensor] = None) -> None:
+    """Prompt attention over a latent on the 5th-generation tensor cores: q [T, n_heads * row], one cache row a position
+    (cache [pages, 1, 64, row]) whose first `value` columns are its value, out [T, n_heads * value]; tiles of 128 query rows as
+    (sequence, first row), walked from the back.  `sink`, `sink_values` as in `attention_prefill`."""
+    _need(q, "latent attention q", torch.bfloat16, 2)
+    _need(out, "latent attention out", torch.bfloat16, 2)
+    _need(cache, "latent attention cache", torch.bfloat16, 4)
+    n = q.shape[0]
+    if tuple(q.shape) != (n, n_heads * row) or tuple(out.shape) != (n, n_heads * value) or tuple(cache.shape[1:]) != (1, 64, row):
+        raise KernelError(f"latent attention: q {tuple(q.shape)} / out {tuple(out.shape)} / cache {tuple(cache.shape)} for {n_heads} "
+                          f"heads of {row} / {value}")
+    for name, t in (("seq_slot", seq_slot), ("seq_ctx", seq_ctx), ("seq_qstart", seq_qstart), ("seq_qlen", seq_qlen),
+                    ("tile_seq", tile_seq), ("tile_row0", tile_row0)):
+        _need(t, f"latent attention {name}", torch.int32, 1)
+    _need(block_table, "latent attention block_table", torch.int32, 2)
+    if tile_seq.shape != tile_row0.shape:
+        raise KernelError("latent attention: the tile lists differ in length")
+    _check_sink_values(sink_values, n_heads)
+    _check(lib().mll_attn_prefill_latent_tc5(
+        _ptr(q), _ptr(cache), _ptr(seq_slot), _ptr(seq_ctx), _ptr(seq_qstart), _ptr(seq_qlen), _ptr(tile_seq), _ptr(tile_row0),
+        _ptr(block_table), _ptr(out), ctypes.c_int(n), ctypes.c_longlong(cache.shape[0]), ctypes.c_int(tile_seq.shape[0]),
+        ctypes.c_int(n_heads), ctypes.c_int(row), ctypes.c_int(value), ctypes.c_int(block_table.shape[1]), ctypes.c_int(window),
+        ctypes.c_float(scale), ctypes.c_int(int(sink or sink_values is not None)), _ptr(sink_values), _stream()),
+        "latent_attention (tcgen05)")
+
+
 def local_attention_heads(q, k_cache, v_cache, seq_slot, seq_ctx, seq_qstart, seq_qlen, block_table, out, n_seqs: int,
                           n_heads: int, n_kv_heads: int, d: int, dv: int, chunk: int, window: int, scale: float,
                           sink: bool = False, v_in_k: bool = False, n_splits: int = 1,

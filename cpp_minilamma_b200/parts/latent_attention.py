@@ -172,6 +172,10 @@ class LatentAttention(Mixer):
             K.local_attention_heads(q, cache.k, cache.v, step.seq_slot, step.seq_ctx, step.seq_qstart, step.seq_qlen,
                                     cache.block_table, latent, T, H, 1, self.row, self.rank, 0, self.window, self.scale,
                                     v_in_k=True, n_splits=splits, scratch=scratch, **sink)
+        elif tiles and K.latent_attention_tc5_supported(act, self.row, self.rank):
+            K.latent_attention_tiles(q, cache.k, step.seq_slot, step.seq_ctx, step.seq_qstart, step.seq_qlen, tiles["wide_seq"],
+                                     tiles["wide_row0"], cache.block_table, latent, H, self.row, self.rank, self.window,
+                                     self.scale, **sink)
         elif tiles and K.local_attention_mma_supported(act, self.row, self.rank):
             K.local_attention_tiles(q, cache.k, cache.v, step.seq_slot, step.seq_ctx, step.seq_qstart, step.seq_qlen,
                                     tiles["tile_seq"], tiles["tile_row0"], cache.block_table, latent, H, 1, self.row,
