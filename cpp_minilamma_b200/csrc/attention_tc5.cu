@@ -737,8 +737,9 @@ MLL_API int mll_attn_prefill_latent_tc5_supported(int row, int value) {
 // Prompt attention over a latent, bfloat16: q [n_tokens, n_heads * row], one cache row of `row` columns a position (cache: pages of 64
 // rows), whose first `value` columns are also its value; out [n_tokens, n_heads * value].  The other arguments as in
 // mll_attn_prefill_tc5.  A block's tensor memory holds two S buffers and up to 256 columns of O, its shared memory the query tile
-// and four pages, so it has a multiprocessor to itself; pages are loaded once for both products.  A request of three
-// prompts (3,970 tokens, 16 heads, rows of 256) 5,440 -> 4,942 us; the kernel before, mma.sync (attention_local_mma.cu), took 364 of them a layer.
+// and four pages, so it has a multiprocessor to itself; pages are loaded once for both products.  Bound by a page's
+// chain, scores - softmax - values, of which two are in flight: us, mma.sync (attention_local_mma.cu) / here, rows of 256 with values
+// of 192, 16 heads: 3 prompts of 600 to 2,047 353 / 97, one of 4,095 812 / 186 (0.65 PFLOP/s).
 MLL_API int mll_attn_prefill_latent_tc5(const void* q, const void* cache, const int* seq_slot, const int* seq_ctx,
                                         const int* seq_qstart, const int* seq_qlen, const int* tile_seq, const int* tile_row0,
                                         const int* block_table, void* out, int n_tokens, long long n_pages, int n_tiles,

@@ -139,6 +139,11 @@ class LatentAttention(Mixer):
     def prepare_step(self, shape):
         return prompt_tiles(shape)
 
+    # Rows a tile of 128 must hold on average for the tcgen05 kernel: its tiles have a multiprocessor each, the mma.sync kernel's of 64 rows
+    # a third (us, that / tcgen05, rows of 256, 16 heads: 30 sequences of 40 tokens 22.1 / 33.4, one of 300 in three tiles 29.7 / 20.1, three of
+    # 600 to 2,047 353 / 97, one of 4,095 812 / 186; up to 64 tokens they are alike).
+    TILE_ROWS = 80
+
     def forward(self, step, h, cache):
         T, H = h.shape[0], self.n_heads
         act = self.ctx.act_dtype
@@ -172,7 +177,7 @@ class LatentAttention(Mixer):
             K.local_attention_heads(q, cache.k, cache.v, step.seq_slot, step.seq_ctx, step.seq_qstart, step.seq_qlen,
                                     cache.block_table, latent, T, H, 1, self.row, self.rank, 0, self.window, self.scale,
                                     v_in_k=True, n_splits=splits, scratch=scratch, **sink)
-        elif tiles and K.latent_attention_tc5_supported(act, self.row, self.rank):
+        elif tiles and T >= self.TILE_ROWS * tiles["wide_seq"].shape[0] and K.latent_attention_tc5_supported(act, self.row, self.rank):
             K.latent_attention_tiles(q, cache.k, step.seq_slot, step.seq_ctx, step.seq_qstart, step.seq_qlen, tiles["wide_seq"],
                                      tiles["wide_row0"], cache.block_table, latent, H, self.row, self.rank, self.window,
                                      self.scale, **sink)
